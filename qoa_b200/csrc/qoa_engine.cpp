@@ -52,9 +52,11 @@ cudaError_t launch_collapse(double2* a, uint64_t len, uint32_t q, uint32_t outco
 cudaError_t launch_materialize(double2* a, uint64_t len, double* norm2, double* partials, uint32_t* status, cudaStream_t st);
 cudaError_t launch_set_scalar(double* p, double v, cudaStream_t st);
 cudaError_t launch_probs(const double2* a, uint64_t off, uint64_t cnt, const double* norm2, double* out, cudaStream_t st);
-cudaError_t launch_tree(const void* a, bool f32, uint32_t n, const double* norm2, double* tree, cudaStream_t st);
-cudaError_t launch_sample(const void* a, bool f32, uint32_t n, const double* norm2, const double* tree,
-                          const double* u, uint64_t shots, int mode, unsigned long long* out, cudaStream_t st);
+SampleLevels sample_levels(uint32_t n);
+cudaError_t launch_sample_tree(const void* a, bool f32, uint32_t n, const double* norm2, const SampleLevels& L, double* tree,
+                               cudaStream_t st);
+cudaError_t launch_shots(const void* a, bool f32, uint32_t n, const double* norm2, const double* tree, const SampleLevels& L,
+                         const double* u, uint64_t shots, int mode, unsigned long long* out, cudaStream_t st);
 cudaError_t launch_f32_pass(float2* amps, const F32PassParams& P, const float* mats, const F32PhaseOp* pops,
                             const F32Angle* angles, const F32Phase* phases, const float2* tables,
                             const double* norm2_in, double* partials, uint32_t* status, cudaStream_t st);
@@ -309,6 +311,8 @@ struct qoa_state_s {
     uint32_t* status = nullptr;   // device status words
     double* partials = nullptr;
     size_t partials_cap = 0;
+    double* ws = nullptr;         // scratch kept between calls (workspace)
+    size_t ws_cap = 0;
     double* host_scal = nullptr;  // pinned mirror of scal
     uint64_t seed = 0;
     uint64_t noise_stream = 0;
@@ -432,6 +436,31 @@ int alloc_state(qoa_state_t s, uint32_t n) {
     CK(device_alloc((void**)&s->amps, (s->precision == QOA_PREC_F32 ? sizeof(float2) : sizeof(double2)) << n));
     s->partials_cap = partials_needed(n);
     CK(device_alloc((void**)&s->partials, s->partials_cap * sizeof(double)));
+    return QOA_OK;
+}
+
+// Scratch of a synchronous call (sampling, probabilities) on the handle's
+// stream, kept by the handle up to kWorkspaceKept bytes: a buffer allocated
+// per call is mapped and unmapped each time (0.9 to 3 ms per GB). Larger
+// ones are freed by workspace_done.
+constexpr size_t kWorkspaceKept = size_t(256) << 20;
+int workspace(qoa_state_t s, size_t bytes, double** out) {
+    if (bytes > s->ws_cap) {
+        if (s->ws) cudaFree(s->ws);
+        s->ws = nullptr;
+        s->ws_cap = 0;
+        CK(device_alloc((void**)&s->ws, bytes));
+        s->ws_cap = bytes;
+    }
+    *out = s->ws;
+    return QOA_OK;
+}
+int workspace_done(qoa_state_t s) {
+    if (s->ws_cap > kWorkspaceKept) {
+        cudaFree(s->ws);
+        s->ws = nullptr;
+        s->ws_cap = 0;
+    }
     return QOA_OK;
 }
 
@@ -3045,6 +3074,7 @@ int qoa_destroy(qoa_state_t s) {
     if (s->f32_mats) cudaFree(s->f32_mats);
     if (s->f32_phases) cudaFree(s->f32_phases);
     if (s->partials) cudaFree(s->partials);
+    if (s->ws) cudaFree(s->ws);
     if (s->scal) cudaFree(s->scal);
     if (s->status) cudaFree(s->status);
     if (s->host_scal) cudaFreeHost(s->host_scal);
@@ -3106,24 +3136,22 @@ int qoa_sample(qoa_state_t s, const double* u, size_t shots, int mode, uint64_t*
     if (shots == 0) return QOA_OK;
     const uint32_t n = s->n;
     const size_t nu = mode == 0 ? shots * n : shots;
-    double* d_tree = nullptr;
-    double* d_u = nullptr;
-    unsigned long long* d_out = nullptr;
-    const size_t tree_len = (n >= 2) ? ((1ull << n) - 2) : 1;
-    CK(cudaMallocAsync(&d_tree, tree_len * sizeof(double), s->stream));
-    CK(cudaMallocAsync(&d_u, nu * sizeof(double), s->stream));
-    CK(cudaMallocAsync(&d_out, shots * sizeof(unsigned long long), s->stream));
+    const SampleLevels L = sample_levels(n);
+    // uniforms, then the outcomes, then the tree levels: one workspace
+    double* ws = nullptr;
+    rc = workspace(s, (nu + shots + (size_t)L.total) * sizeof(double), &ws);
+    if (rc) return rc;
+    double* d_u = ws;
+    unsigned long long* d_out = reinterpret_cast<unsigned long long*>(ws + nu);
+    double* d_tree = ws + nu + shots;
     CK(cudaMemcpyAsync(d_u, u, nu * sizeof(double), cudaMemcpyHostToDevice, s->stream));
     const bool f32 = s->precision == QOA_PREC_F32;
-    CK(launch_tree(s->amps, f32, n, s->scal, d_tree, s->stream));
-    CK(launch_sample(s->amps, f32, n, s->scal, d_tree, d_u, shots, mode, d_out, s->stream));
-    s->launches += (n >= 2 ? (n - 1) : 0) + 1;
+    CK(launch_sample_tree(s->amps, f32, n, s->scal, L, d_tree, s->stream));
+    CK(launch_shots(s->amps, f32, n, s->scal, d_tree, L, d_u, shots, mode, d_out, s->stream));
+    s->launches += L.count + 1;
     CK(cudaMemcpyAsync(out, d_out, shots * sizeof(uint64_t), cudaMemcpyDeviceToHost, s->stream));
-    CK(cudaFreeAsync(d_tree, s->stream));
-    CK(cudaFreeAsync(d_u, s->stream));
-    CK(cudaFreeAsync(d_out, s->stream));
     CK(cudaStreamSynchronize(s->stream));
-    return QOA_OK;
+    return workspace_done(s);
 }
 
 int qoa_probabilities(qoa_state_t s, double* out) {
@@ -3133,7 +3161,8 @@ int qoa_probabilities(qoa_state_t s, double* out) {
     const uint64_t len = state_len(s);
     const uint64_t chunk = std::min<uint64_t>(len, 1ull << 24);
     double* d = nullptr;
-    CK(cudaMallocAsync(&d, chunk * sizeof(double), s->stream));
+    rc = workspace(s, chunk * sizeof(double), &d);
+    if (rc) return rc;
     for (uint64_t off = 0; off < len; off += chunk) {
         const uint64_t cnt = std::min(chunk, len - off);
         if (s->precision == QOA_PREC_F32)
@@ -3143,9 +3172,8 @@ int qoa_probabilities(qoa_state_t s, double* out) {
         s->launches++;
         CK(cudaMemcpyAsync(out + off, d, cnt * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
     }
-    CK(cudaFreeAsync(d, s->stream));
     CK(cudaStreamSynchronize(s->stream));
-    return QOA_OK;
+    return workspace_done(s);
 }
 
 int qoa_expect_z(qoa_state_t s, const uint64_t* masks, size_t k, double* out) {

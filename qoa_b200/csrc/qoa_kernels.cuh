@@ -248,6 +248,15 @@ struct SampleJob {
     uint64_t out_start;
 };
 
+// Stored levels of a state's marginal tree (qoa_sample.cu): level k holds
+// 2^bits[k] sums at tree + off[k]; bits descend.
+struct SampleLevels {
+    uint32_t count;
+    uint32_t bits[8];
+    uint64_t off[8];
+    uint64_t total;  // doubles of all levels
+};
+
 // ---------------------------------------------------------------------------
 // Per-gate kernels over global memory (fallback / per-gate mode / shims).
 // ---------------------------------------------------------------------------
