@@ -149,97 +149,6 @@ cudaError_t launch_small_batch(bool f32, const SmallCircuit* circs, uint32_t cou
 }
 
 // --------------------------------------------------------------------------
-// <Z_mask> of the arena circuits: kernel 1 sums chunks of EXPZ_CHUNK
-// amplitudes of every circuit (one CTA per chunk, every mask of the circuit
-// plus the squared norm); kernel 2 (one CTA per circuit) adds each slot's
-// chunk sums in chunk order and divides by the norm, so results do not depend
-// on the launch shape.
-template <typename T>
-__device__ __forceinline__ double amp_abs2(const T* a, uint64_t i) {
-    const T x = a[i];
-    return (double)x.x * x.x + (double)x.y * x.y;
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) k_arena_expz_partials(const ExpzJob* __restrict__ jobs, uint32_t njobs,
-                                                             const uint64_t* __restrict__ masks,
-                                                             double* __restrict__ partials) {
-    __shared__ double red[9][8];
-    const uint32_t b = blockIdx.x;
-    uint32_t lo = 0, hi = njobs - 1;
-    while (lo < hi) {
-        const uint32_t mid = (lo + hi + 1) >> 1;
-        if (jobs[mid].chunk_start <= b) lo = mid;
-        else hi = mid - 1;
-    }
-    const ExpzJob J = jobs[lo];
-    const T* a = reinterpret_cast<const T*>(J.amps);
-    const uint64_t c = b - J.chunk_start;
-    const uint64_t len = 1ull << J.n;
-    const uint64_t begin = c * EXPZ_CHUNK;
-    const uint64_t end = begin + EXPZ_CHUNK < len ? begin + EXPZ_CHUNK : len;
-    const uint32_t slots = J.mask_count + 1;
-    double* out = partials + J.part_start + c * slots;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (uint32_t m0 = 0; m0 == 0 || m0 < J.mask_count; m0 += 8) {
-        double v[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-        uint64_t mk[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) mk[q] = (m0 + q < J.mask_count) ? masks[J.mask_start + m0 + q] : 0;
-        for (uint64_t i = begin + threadIdx.x; i < end; i += blockDim.x) {
-            const double p = amp_abs2<T>(a, i);
-            v[8] += p;
-#pragma unroll
-            for (int q = 0; q < 8; ++q) v[q] += (__popcll(i & mk[q]) & 1) ? -p : p;
-        }
-#pragma unroll
-        for (int q = 0; q < 9; ++q) {
-            double x = v[q];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-            if (lane == 0) red[q][w] = x;
-        }
-        __syncthreads();
-        if (threadIdx.x < 9) {
-            double t = 0.0;
-            for (int k = 0; k < (int)(blockDim.x >> 5); ++k) t += red[threadIdx.x][k];
-            const uint32_t slot = threadIdx.x < 8 ? m0 + threadIdx.x : J.mask_count;
-            if (slot < J.mask_count || (threadIdx.x == 8 && m0 == 0)) out[slot] = t;
-        }
-        __syncthreads();
-    }
-}
-
-__global__ void __launch_bounds__(256) k_arena_expz_final(const ExpzJob* __restrict__ jobs,
-                                                          const double* __restrict__ partials,
-                                                          double* __restrict__ out) {
-    __shared__ double sums[EXPZ_MAX_MASKS + 1];
-    const ExpzJob J = jobs[blockIdx.x];
-    const uint32_t slots = J.mask_count + 1;
-    const uint64_t len = 1ull << J.n;
-    const uint32_t chunks = (uint32_t)((len + EXPZ_CHUNK - 1) / EXPZ_CHUNK);
-    for (uint32_t s = threadIdx.x; s < slots; s += blockDim.x) {
-        double t = 0.0;
-        for (uint32_t c = 0; c < chunks; ++c) t += partials[J.part_start + (uint64_t)c * slots + s];
-        sums[s] = t;
-    }
-    __syncthreads();
-    for (uint32_t s = threadIdx.x; s < J.mask_count; s += blockDim.x)
-        out[J.out_start + s] = sums[s] / sums[J.mask_count];
-}
-
-cudaError_t launch_arena_expz(bool f32, const ExpzJob* jobs, uint32_t njobs, uint32_t chunks, const uint64_t* masks,
-                              double* partials, double* out, cudaStream_t st) {
-    if (!njobs) return cudaSuccess;
-    if (f32) k_arena_expz_partials<float2><<<chunks, 256, 0, st>>>(jobs, njobs, masks, partials);
-    else k_arena_expz_partials<double2><<<chunks, 256, 0, st>>>(jobs, njobs, masks, partials);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    k_arena_expz_final<<<njobs, 256, 0, st>>>(jobs, partials, out);
-    return cudaGetLastError();
-}
-
-// --------------------------------------------------------------------------
 // Shots of sampled batch circuits: one CTA per circuit builds the marginal
 // tree of its final state in global scratch (level k, 1 <= k < n, holds the
 // 2^k sums over qubits k..n-1 at tree + 2^k - 2, as k_tree_leaf / k_tree_up

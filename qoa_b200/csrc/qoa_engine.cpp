@@ -44,8 +44,9 @@ int reduce_blocks(uint64_t len);
 cudaError_t launch_norm(const double2* a, uint64_t len, double* partials, double* out, uint32_t* status, cudaStream_t st);
 cudaError_t launch_p01(const double2* a, uint64_t len, uint32_t q, double* partials, double* out2, const double* norm2,
                        cudaStream_t st);
-cudaError_t launch_expz(const double2* a, uint64_t len, const uint64_t* masks, uint32_t k, double* partials, double* out,
-                        const double* norm2, cudaStream_t st);
+uint32_t expz_blocks(uint64_t len);
+cudaError_t launch_expz(const void* a, bool f32, uint64_t len, const ExpzMasks& M, uint32_t k, const double* norm2,
+                        double* partials, unsigned int* ticket, double* out, cudaStream_t st);
 cudaError_t launch_reduce_partials(const double* partials, uint32_t count, double* out, uint32_t* status, cudaStream_t st);
 cudaError_t launch_collapse(double2* a, uint64_t len, uint32_t q, uint32_t outcome, double f, double* partials,
                             double* norm2_out, uint32_t* status, cudaStream_t st);
@@ -68,8 +69,6 @@ cudaError_t launch_f32_materialize(float2* a, uint64_t len, double* norm2, doubl
 cudaError_t launch_f32_probs(const float2* a, uint64_t off, uint64_t cnt, const double* norm2, double* out,
                              cudaStream_t st);
 cudaError_t launch_random_state(void* a, bool f32, uint64_t len, uint64_t seed, cudaStream_t st);
-cudaError_t launch_f32_expz(const float2* a, uint64_t len, const uint64_t* masks, uint32_t k, double* partials,
-                            double* out, const double* norm2, cudaStream_t st);
 cudaError_t launch_pass_p32(float2* amps, const PassParams& P, const double* norm2_in, double* partials,
                             cudaStream_t st);
 cudaError_t launch_pass_p32_arena(const ArenaJob* jobs, uint32_t njobs, const uint32_t* tile_start, uint32_t tiles,
@@ -80,8 +79,8 @@ cudaError_t launch_pass_arena(const ArenaJob* jobs, uint32_t njobs, const uint32
 cudaError_t launch_f32_pass_arena(const ArenaJob* jobs, uint32_t njobs, const uint32_t* tile_start, uint32_t tiles,
                                   const float* mats, const F32PhaseOp* pops, const F32Angle* angles,
                                   const F32Phase* phases, const float2* tables, uint32_t* status, cudaStream_t st);
-cudaError_t launch_arena_expz(bool f32, const ExpzJob* jobs, uint32_t njobs, uint32_t chunks, const uint64_t* masks,
-                              double* partials, double* out, cudaStream_t st);
+cudaError_t launch_arena_expz(bool f32, const ExpzJob* jobs, uint32_t njobs, uint32_t chunks, uint32_t max_masks,
+                              const uint64_t* masks, double* partials, double* out, cudaStream_t st);
 cudaError_t launch_sample_jobs(bool f32, const SampleJob* jobs, uint32_t njobs, const double* u,
                                unsigned long long* out, cudaStream_t st);
 cudaError_t launch_small_batch(bool f32, const SmallCircuit* circs, uint32_t count, const SmallOp* ops,
@@ -307,13 +306,13 @@ struct qoa_state_s {
     int device = 0;
     cudaStream_t stream = nullptr;
     double2* amps = nullptr;
-    double* scal = nullptr;       // [0] norm2, [1] P0, [2] P1, [3..] scratch
+    double* scal = nullptr;       // SCAL_DOUBLES: [0] norm2, [1] P0, [2] P1, [3..] scratch, ticket word
     uint32_t* status = nullptr;   // device status words
     double* partials = nullptr;
     size_t partials_cap = 0;
     double* ws = nullptr;         // scratch kept between calls (workspace)
     size_t ws_cap = 0;
-    double* host_scal = nullptr;  // pinned mirror of scal
+    double* host_scal = nullptr;  // pinned: mirror of scal, then EXPZ_MASKS results
     uint64_t seed = 0;
     uint64_t noise_stream = 0;
     uint64_t noise_event = 0;
@@ -369,6 +368,7 @@ int set_err(qoa_state_t s, int code, const char* fmt, ...) {
     } while (0)
 
 uint64_t state_len(const qoa_state_t s) { return 1ull << s->n; }
+unsigned int* ticket(const qoa_state_t s) { return reinterpret_cast<unsigned int*>(s->scal + SCAL_TICKET); }
 
 size_t partials_needed(uint32_t n) {
     size_t a = (n >= (uint32_t)TILE_BITS) ? (size_t)1 << (n - TILE_BITS) : 1;
@@ -2272,7 +2272,7 @@ struct qoa_batch_s {
     uint32_t narena = 0;
     // expectation values of arena and view circuits
     ExpzJob* d_ejobs = nullptr;
-    uint32_t n_ejobs = 0, e_chunks = 0;
+    uint32_t n_ejobs = 0, e_chunks = 0, e_max_masks = 0;
     double* d_epart = nullptr;
     // sampled circuits (qoa_batch_add_trajectory)
     double* d_shot_u = nullptr;
@@ -2653,7 +2653,7 @@ int batch_prepare(qoa_batch_t b) {
         if (c.route != R_VIEW) continue;
         view_off.push_back(total);
         total = al(total + partials_needed(c.n) * sizeof(double));
-        total = al(total + 16 * sizeof(double));
+        total = al(total + SCAL_DOUBLES * sizeof(double));
         total = al(total + 4 * sizeof(uint32_t));
     }
     // sampled circuits: marginal-tree scratch (2^n - 2 doubles each)
@@ -2818,7 +2818,7 @@ int batch_prepare(qoa_batch_t b) {
 
     // expectation values of every arena and view circuit
     std::vector<ExpzJob> ej;
-    uint32_t chunks = 0;
+    uint32_t chunks = 0, max_masks = 0;
     uint64_t parts = 0;
     for (size_t i = 0; i < b->circs.size(); ++i) {
         const auto& c = b->circs[i];
@@ -2836,10 +2836,12 @@ int batch_prepare(qoa_batch_t b) {
         const uint32_t nch = (uint32_t)(((1ull << c.n) + EXPZ_CHUNK - 1) / EXPZ_CHUNK);
         chunks += nch;
         parts += (uint64_t)nch * (J.mask_count + 1);
+        max_masks = std::max(max_masks, J.mask_count);
         ej.push_back(J);
     }
     b->n_ejobs = (uint32_t)ej.size();
     b->e_chunks = chunks;
+    b->e_max_masks = max_masks;
     if (!ej.empty()) {
         if ((rc = upload(b, b->d_ejobs, ej))) return rc;
         BCK(dalloc(b, b->d_epart, parts * sizeof(double)));
@@ -2880,7 +2882,8 @@ int batch_prepare(qoa_batch_t b) {
         v->partials_cap = partials_needed(c.n);
         o = al(o + v->partials_cap * sizeof(double));
         v->scal = (double*)(base + o);
-        o = al(o + 16 * sizeof(double));
+        BCK(cudaMemsetAsync(v->scal, 0, SCAL_DOUBLES * sizeof(double), b->streams[0]));
+        o = al(o + SCAL_DOUBLES * sizeof(double));
         v->status = (uint32_t*)(base + o);
         BCK(cudaMemsetAsync(v->status, 0, 4 * sizeof(uint32_t), b->streams[0]));
         if (tensor) {
@@ -2953,7 +2956,7 @@ int batch_enqueue(qoa_batch_t b) {
         BCK(cudaEventRecord(b->events[i], b->streams[i]));
         BCK(cudaStreamWaitEvent(s0, b->events[i], 0));
     }
-    BCK(launch_arena_expz(f32, b->d_ejobs, b->n_ejobs, b->e_chunks, b->d_masks, b->d_epart, b->d_out, s0));
+    BCK(launch_arena_expz(f32, b->d_ejobs, b->n_ejobs, b->e_chunks, b->e_max_masks, b->d_masks, b->d_epart, b->d_out, s0));
     BCK(launch_sample_jobs(f32, b->d_sjobs, b->n_sjobs, b->d_shot_u, b->d_shot_out, s0));
     b->graph_jit = all_ready;
     return QOA_OK;
@@ -3047,11 +3050,13 @@ int qoa_create(uint32_t n, int precision, uint32_t flags, qoa_state_t* out) {
     };
     if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess)
         return fail(set_err(s, QOA_E_CUDA, "stream create failed"));
-    if (cudaMalloc(&s->scal, 16 * sizeof(double)) != cudaSuccess) return fail(set_err(s, QOA_E_OOM, "scalar alloc"));
+    if (cudaMalloc(&s->scal, SCAL_DOUBLES * sizeof(double)) != cudaSuccess) return fail(set_err(s, QOA_E_OOM, "scalar alloc"));
+    if (cudaMemsetAsync(s->scal, 0, SCAL_DOUBLES * sizeof(double), s->stream) != cudaSuccess)
+        return fail(set_err(s, QOA_E_CUDA, "scalar memset"));
     if (cudaMalloc(&s->status, 4 * sizeof(uint32_t)) != cudaSuccess) return fail(set_err(s, QOA_E_OOM, "status alloc"));
     if (cudaMemsetAsync(s->status, 0, 4 * sizeof(uint32_t), s->stream) != cudaSuccess)
         return fail(set_err(s, QOA_E_CUDA, "status memset"));
-    if (cudaMallocHost(&s->host_scal, 16 * sizeof(double)) != cudaSuccess) return fail(set_err(s, QOA_E_OOM, "pinned alloc"));
+    if (cudaMallocHost(&s->host_scal, (16 + EXPZ_MASKS) * sizeof(double)) != cudaSuccess) return fail(set_err(s, QOA_E_OOM, "pinned alloc"));
     int rc = alloc_state(s, n);
     if (rc) return fail(rc);
     rc = do_reset_all(s);
@@ -3180,19 +3185,23 @@ int qoa_expect_z(qoa_state_t s, const uint64_t* masks, size_t k, double* out) {
     int rc = check_handle(s);
     if (rc) return rc;
     if ((!masks || !out) && k) return set_err(s, QOA_E_ARG, "null argument");
-    for (size_t i = 0; i < k; i += 8) {
-        const uint32_t kk = (uint32_t)std::min<size_t>(8, k - i);
-        if (s->precision == QOA_PREC_F32)  // FP64 sums over the complex64 state
-            CK(launch_f32_expz((const float2*)s->amps, state_len(s), masks + i, kk, s->partials, s->scal + 8,
-                               s->scal, s->stream));
-        else
-            CK(launch_expz(s->amps, state_len(s), masks + i, kk, s->partials, s->scal + 8, s->scal, s->stream));
-        s->launches += 2;
-        CK(cudaMemcpyAsync(s->host_scal + 8, s->scal + 8, kk * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
+    const uint32_t blocks = expz_blocks(state_len(s));
+    for (size_t i = 0; i < k; i += EXPZ_MASKS) {
+        const uint32_t kk = (uint32_t)std::min<size_t>(EXPZ_MASKS, k - i);
+        ExpzMasks M;
+        std::memcpy(M.m, masks + i, kk * sizeof(uint64_t));
+        double* ws = nullptr;  // results, then partial sums
+        rc = workspace(s, (size_t)kk * (1 + blocks) * sizeof(double), &ws);
+        if (rc) return rc;
+        // FP64 sums over either precision
+        CK(launch_expz(s->amps, s->precision == QOA_PREC_F32, state_len(s), M, kk, s->scal, ws + kk, ticket(s), ws,
+                       s->stream));
+        s->launches++;
+        CK(cudaMemcpyAsync(s->host_scal + 16, ws, kk * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
         CK(cudaStreamSynchronize(s->stream));
-        for (uint32_t j = 0; j < kk; ++j) out[i + j] = s->host_scal[8 + j];
+        std::memcpy(out + i, s->host_scal + 16, kk * sizeof(double));
     }
-    return QOA_OK;
+    return workspace_done(s);
 }
 
 int qoa_get_state(qoa_state_t s, void* host, size_t bytes) {

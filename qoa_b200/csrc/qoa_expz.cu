@@ -10,7 +10,10 @@
 // cost per amplitude is 2 + 8 FP64 instructions whatever the number of masks,
 // up to 256 at once, where summing mask by mask costs a popcount, a select
 // and an add per amplitude and mask, and a sweep of the state per 8 masks.
-// It is bound by reading the state (HBM, or L2 where the state fits).
+// It is bound by reading the state (HBM, or L2 where the state fits). Measured
+// on B200 against sweeps of 8 masks: 27 qubits complex128, 16 masks 1573 ->
+// 313 us (6.9 TB/s); 23 qubits complex64, 45 masks 288 -> 29 us (2.3 TB/s, in
+// L2); 119 batch circuits of 13 to 20 qubits, 8 masks each 229 -> 82 us.
 #include <cuda_runtime.h>
 
 #include <stdint.h>

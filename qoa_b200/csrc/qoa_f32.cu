@@ -454,45 +454,7 @@ __global__ void k_f32_probs(const float2* __restrict__ a, uint64_t off, uint64_t
     }
 }
 
-__global__ void k_f32_expz_partials(const float2* __restrict__ a, uint64_t len, const ExpzMasks mk, uint32_t k,
-                                    double* __restrict__ partials) {
-    __shared__ double sh[8][32];
-    double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += (uint64_t)gridDim.x * blockDim.x) {
-        const float2 x = a[i];
-        const double p = (double)x.x * x.x + (double)x.y * x.y;
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] += (__popcll(i & mk.m[j]) & 1) ? -p : p;
-    }
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        double x = v[j];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-        if (lane == 0) sh[j][w] = x;
-    }
-    __syncthreads();
-    if (threadIdx.x < k) {
-        double t = 0.0;
-        for (int q = 0; q < (int)(blockDim.x >> 5); ++q) t += sh[threadIdx.x][q];
-        partials[(uint64_t)threadIdx.x * gridDim.x + blockIdx.x] = t;
-    }
-}
-
 int reduce_blocks(uint64_t len);
-cudaError_t launch_reduce_div(const double* partials, uint32_t count, uint32_t sets, double* out, const double* divide_by,
-                              cudaStream_t st);
-
-cudaError_t launch_f32_expz(const float2* a, uint64_t len, const uint64_t* masks, uint32_t k, double* partials,
-                            double* out, const double* norm2, cudaStream_t st) {
-    const int nb = reduce_blocks(len);
-    ExpzMasks mk{};
-    for (uint32_t j = 0; j < k && j < 8; ++j) mk.m[j] = masks[j];
-    k_f32_expz_partials<<<nb, 256, 0, st>>>(a, len, mk, k, partials);
-    return launch_reduce_div(partials, (uint32_t)nb, k, out, norm2, st);
-}
-
 cudaError_t launch_reduce_partials(const double* partials, uint32_t count, double* out, uint32_t* status,
                                    cudaStream_t st);
 

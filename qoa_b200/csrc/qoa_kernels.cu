@@ -10,7 +10,7 @@
 //
 // The rest: per-gate kernels over global memory (fallback, per-gate mode and
 // the vectorization.rs shims), the measurement reductions and collapse of
-// quantum_state.rs:399-458 and expectation values (shots: qoa_sample.cu).
+// quantum_state.rs:399-458 (shots: qoa_sample.cu, expectation values: qoa_expz.cu).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -576,25 +576,6 @@ __global__ void k_p01_partials(const double2* __restrict__ a, uint64_t len, uint
     block_store_partials<2>(v, partials, gridDim.x);
 }
 
-// Z-string sums for up to 8 masks per launch
-struct Masks8 {
-    uint64_t m[8];
-};
-
-__global__ void k_expz_partials(const double2* __restrict__ a, uint64_t len, const Masks8 mk, uint32_t k,
-                                double* __restrict__ partials) {
-    double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    uint64_t masks[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) masks[j] = (j < (int)k) ? mk.m[j] : 0ull;
-    for (uint64_t i = gtid(); i < len; i += gstride()) {
-        const double p = c_abs2(a[i]);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] += (__popcll(i & masks[j]) & 1) ? -p : p;
-    }
-    block_store_partials<8>(v, partials, gridDim.x);
-}
-
 // Final reduction: out[s] = sum_k partials[s*count + k] in a fixed order (one
 // block per set), then optional scaling by 1/norm2 and status bookkeeping.
 __global__ void k_reduce(const double* __restrict__ partials, uint32_t count, double* __restrict__ out,
@@ -770,22 +751,6 @@ cudaError_t launch_p01(const double2* a, uint64_t len, uint32_t q, double* parti
     const int nb = reduce_blocks(len);
     k_p01_partials<<<nb, 256, 0, st>>>(a, len, q, partials);
     k_reduce<<<2, 1024, 0, st>>>(partials, nb, out2, norm2, nullptr);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_expz(const double2* a, uint64_t len, const uint64_t* masks, uint32_t k, double* partials,
-                        double* out, const double* norm2, cudaStream_t st) {
-    const int nb = reduce_blocks(len);
-    Masks8 mk{};
-    for (uint32_t j = 0; j < k && j < 8; ++j) mk.m[j] = masks[j];
-    k_expz_partials<<<nb, 256, 0, st>>>(a, len, mk, k, partials);
-    k_reduce<<<k, 1024, 0, st>>>(partials, nb, out, norm2, nullptr);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_reduce_div(const double* partials, uint32_t count, uint32_t sets, double* out, const double* divide_by,
-                              cudaStream_t st) {
-    k_reduce<<<sets, 1024, 0, st>>>(partials, count, out, divide_by, nullptr);
     return cudaGetLastError();
 }
 

@@ -154,9 +154,16 @@ struct ArenaJob {
 // ---------------------------------------------------------------------------
 constexpr int MAX_F32_OPS = 256;
 
+// Masks of one expectation sweep (qoa_expz.cu).
+constexpr uint32_t EXPZ_MASKS = 256;
 struct ExpzMasks {
-    uint64_t m[8];
+    uint64_t m[EXPZ_MASKS];
 };
+
+// A handle's device scalars: [0] norm2, [1], [2] P0, P1, and the ticket word of
+// kernels whose last CTA finishes the reduction (0 between launches).
+constexpr int SCAL_TICKET = 16;
+constexpr int SCAL_DOUBLES = 17;
 
 struct F32Op {
     uint32_t kind;   // 0 = dense block, 1 = phase group
@@ -215,7 +222,7 @@ struct SmallOp {
     double2 m[4];    // SK_G1: m00 m01 m10 m11; SK_DIAG: d0, d1
 };
 
-// Arena circuits' <Z_mask>: chunk partial sums, then one CTA per circuit.
+// Arena circuits' <Z_mask>: sums per tile of EXPZ_CHUNK amplitudes, then one CTA per circuit.
 constexpr uint32_t EXPZ_CHUNK = 4096;
 constexpr uint32_t EXPZ_MAX_MASKS = 255;
 struct ExpzJob {
