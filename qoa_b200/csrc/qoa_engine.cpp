@@ -763,6 +763,7 @@ struct PlanEntry {
     std::vector<PassParams> built;
     std::vector<int> built_of;
     std::vector<std::string> bodies;
+    std::vector<JitKernel> kernels;  // of bodies, as the last request gave them
 };
 struct PlanCache {
     static constexpr size_t kEntries = 8;
@@ -770,29 +771,38 @@ struct PlanCache {
     std::unordered_map<uint64_t, uint8_t> seen;    // op lists seen once
 };
 
+// The words of each gate that its kind uses (the rest of m and pi is not
+// initialised).
 void plan_hash(const std::vector<Gate>& G, uint64_t key, uint64_t& h1, uint64_t& h2) {
     h1 = 1469598103934665603ull ^ key;
     h2 = 0x9e3779b97f4a7c15ull ^ (key * 0xff51afd7ed558ccdull);
-    auto mix = [&](const void* p, size_t nb) {
-        const unsigned char* c = (const unsigned char*)p;
-        for (size_t i = 0; i < nb; ++i) {
-            h1 = (h1 ^ c[i]) * 1099511628211ull;
-            h2 = (h2 ^ c[i]) * 0x100000001b3ull + (h2 >> 29);
+    auto mix = [&](uint64_t w) {
+        h1 = (h1 ^ w) * 0xff51afd7ed558ccdull;
+        h1 ^= h1 >> 32;
+        h2 = (h2 + w) * 0xc4ceb9fe1a85ec53ull;
+        h2 ^= h2 >> 29;
+    };
+    auto words = [&](const void* p, size_t nb) {
+        uint64_t w;
+        for (size_t i = 0; i + 8 <= nb; i += 8) {
+            std::memcpy(&w, (const unsigned char*)p + i, 8);
+            mix(w);
         }
     };
     for (const Gate& g : G) {
-        mix(&g.kind, sizeof g.kind);
-        mix(&g.sub, sizeof g.sub);
-        mix(&g.t, sizeof g.t);
-        mix(&g.t2, sizeof g.t2);
-        mix(&g.cmask, sizeof g.cmask);
-        const uint8_t neg = g.neg;
-        mix(&neg, 1);
-        mix(g.m, sizeof g.m);
-        mix(&g.nmask, sizeof g.nmask);
-        mix(&g.dmask, sizeof g.dmask);
-        mix(&g.u, sizeof g.u);
-        if (g.kind == K_PERM) mix(g.pi, sizeof g.pi);
+        mix((uint64_t)(uint8_t)g.kind | ((uint64_t)(uint8_t)g.sub << 8) | ((uint64_t)g.neg << 16) |
+            ((uint64_t)(uint16_t)g.t << 32) | ((uint64_t)(uint16_t)g.t2 << 48));
+        mix(g.cmask);
+        mix(g.nmask);
+        mix(g.dmask);
+        switch (g.kind) {
+            case K_G1: words(g.m, 4 * sizeof(double2)); break;
+            case K_DIAG: words(g.m, 2 * sizeof(double2)); break;
+            case K_U2: words(g.m, 16 * sizeof(double2)); break;
+            case K_MEASURE: words(&g.u, sizeof g.u); break;
+            case K_PERM: words(g.pi, sizeof g.pi); break;
+            default: break;
+        }
     }
 }
 
@@ -1782,8 +1792,8 @@ int run_pass(qoa_state_t s, const std::vector<Gate>& G, const Step& st) {
     return QOA_OK;
 }
 
-// A complex128 pass whose parameters were built ahead (with its generated
-// kernel requested): the generated kernel when it is ready, else k_pass.
+// A pass whose parameters were built ahead: its generated kernel when it is
+// ready, else the interpreter.
 int run_pass_built(qoa_state_t s, const PassParams& P, const JitKernel& jk) {
     const bool c64 = s->precision == QOA_PREC_F32;
     {
@@ -1955,6 +1965,12 @@ int execute_f32(qoa_state_t s, std::vector<Gate>& G) {
 // network) become one K_PERM step: a single in-place permutation pass instead
 // of several tile passes that only relabel.
 void merge_swap_blocks(std::vector<Gate>& G) {
+    size_t run = 0, longest = 0;
+    for (const Gate& g : G) {
+        run = g.kind == K_SWAP ? run + 1 : 0;
+        longest = std::max(longest, run);
+    }
+    if (longest < 3) return;
     std::vector<Gate> out;
     out.reserve(G.size());
     size_t i = 0;
@@ -2042,7 +2058,7 @@ int execute(qoa_state_t s, std::vector<Gate>& G) {
         while (j < G.size() && G[j].kind != K_QINIT) ++j;
         std::vector<Gate> seg(G.begin() + i, G.begin() + j);
         if (!per_gate) merge_swap_blocks(seg);
-        const bool prebuild = !per_gate && s->jit_mode != QOA_JIT_OFF && s->n >= s->jit_min_qubits;
+        const bool jit = !per_gate && s->jit_mode != QOA_JIT_OFF && s->n >= s->jit_min_qubits;
         // a repeated op list reuses its plan
         PlanEntry local;
         PlanEntry* pe = &local;
@@ -2050,7 +2066,7 @@ int execute(qoa_state_t s, std::vector<Gate>& G) {
         if (!per_gate && s->n > (uint32_t)TILE_BITS) {
             if (!s->plans) s->plans = std::make_shared<PlanCache>();
             PlanCache& pc = *static_cast<PlanCache*>(s->plans.get());
-            const uint64_t key = (uint64_t)s->n | ((uint64_t)c64 << 8) | ((uint64_t)prebuild << 9) |
+            const uint64_t key = (uint64_t)s->n | ((uint64_t)c64 << 8) | ((uint64_t)jit << 9) |
                                  ((uint64_t)(uint32_t)state_pass_budget(s) << 16);
             plan_hash(seg, key, local.h1, local.h2);
             for (auto& e : pc.entries)
@@ -2067,9 +2083,9 @@ int execute(qoa_state_t s, std::vector<Gate>& G) {
             pe->steps = schedule(seg, s->n, per_gate, false, state_pass_budget(s),
                                  slot_search_pays(s->n) || (s->flags & QOA_FLAG_SLOT_SEARCH));
             pe->built_of.assign(pe->steps.size(), -1);
-            // tile passes of a large state: built ahead, and their generated
-            // kernels requested from the compile cache
-            if (prebuild) {
+            // passes built ahead: for generated kernels, whose text is
+            // requested from the compile cache, and for a plan that is kept
+            if (jit || cache_it) {
                 size_t np = 0;
                 for (const Step& st : pe->steps) np += st.pass ? 1 : 0;
                 pe->built.resize(np);
@@ -2077,10 +2093,10 @@ int execute(qoa_state_t s, std::vector<Gate>& G) {
                 for (size_t k = 0; k < pe->steps.size(); ++k) {
                     if (!pe->steps[k].pass || build_pass(seg, pe->steps[k], s->n, pe->built[b], c64) != 0) continue;
                     pe->built_of[k] = (int)b;
-                    pe->bodies.push_back(c64 ? jit_pass32_body(pe->built[b]) : jit_pass_body(pe->built[b]));
+                    if (jit) pe->bodies.push_back(c64 ? jit_pass32_body(pe->built[b]) : jit_pass_body(pe->built[b]));
                     ++b;
                 }
-                pe->prebuilt = true;
+                pe->prebuilt = jit;
             }
             if (cache_it) {
                 PlanCache& pc = *static_cast<PlanCache*>(s->plans.get());
@@ -2092,13 +2108,18 @@ int execute(qoa_state_t s, std::vector<Gate>& G) {
         const std::vector<Step>& steps = pe->steps;
         const std::vector<PassParams>& built = pe->built;
         const std::vector<int>& built_of = pe->built_of;
-        std::vector<JitKernel> jk;
-        if (pe->prebuilt)
+        // once all of a kept plan's kernels are loaded they are not looked up
+        // again (a request hashes every kernel's text, ~0.5 ms for 16 passes)
+        std::vector<JitKernel>& jk = pe->kernels;
+        bool loaded = pe->prebuilt && jk.size() == pe->bodies.size();
+        for (size_t b = 0; loaded && b < jk.size(); ++b) loaded = jk[b].ready();
+        if (pe->prebuilt && !loaded)
             jk = jit_request(pe->bodies, s->jit_mode == QOA_JIT_SYNC ? JitWhen::WAIT : JitWhen::SECOND_SIGHTING);
+        const JitKernel none;  // a kept plan of a state that interprets its passes
         for (size_t k = 0; k < steps.size(); ++k) {
             const Step& st = steps[k];
             int rc;
-            if (st.pass && built_of[k] >= 0) rc = run_pass_built(s, built[built_of[k]], jk[built_of[k]]);
+            if (st.pass && built_of[k] >= 0) rc = run_pass_built(s, built[built_of[k]], pe->prebuilt ? jk[built_of[k]] : none);
             else if (st.pass) rc = run_pass(s, seg, st);
             else {
                 const Gate& g = seg[st.gates[0]];
