@@ -52,6 +52,7 @@ cudaError_t launch_collapse(double2* a, uint64_t len, uint32_t q, uint32_t outco
                             double* norm2_out, uint32_t* status, cudaStream_t st);
 cudaError_t launch_materialize(double2* a, uint64_t len, double* norm2, double* partials, uint32_t* status, cudaStream_t st);
 cudaError_t launch_set_scalar(double* p, double v, cudaStream_t st);
+cudaError_t launch_init_scalars(double* scal, uint32_t* status, cudaStream_t st);
 cudaError_t launch_probs(const double2* a, uint64_t off, uint64_t cnt, const double* norm2, double* out, cudaStream_t st);
 SampleLevels sample_levels(uint32_t n);
 cudaError_t launch_sample_tree(const void* a, bool f32, uint32_t n, const double* norm2, const SampleLevels& L, double* tree,
@@ -961,7 +962,8 @@ std::vector<Step> schedule(const std::vector<Gate>& G, uint32_t n, bool per_gate
 // one (Belady: keep the bits needed soonest). The load and the store need the
 // lanes on tile bits 0..4 (coalesced), so a pass that moved them ends with an
 // exchange back. Gates are rewritten into cheaper equivalents up to a scalar:
-//   H  -> (a0+a1, a0-a1): the 1/sqrt2 is restored by the pass renormalisation;
+//   H  -> (a0+a1, a0-a1): the 1/sqrt2 joins P.phase;
+//   RX, RY -> the larger of cos, sin factored out into P.phase;
 //   RZ -> e^{-i t/2} * diag(1, e^{i t}): the global phase joins P.phase;
 //   Z, CZ -> phase -1.
 // Diagonal factors that are constant over a thread's registers accumulate in
@@ -1389,7 +1391,10 @@ int build_pass(const std::vector<Gate>& G, const Step& st, uint32_t n, PassParam
             switch (sub) {
                 case G1_X: o->code = (uint8_t)(PC_XC + k); break;
                 case G1_Y: o->code = (uint8_t)(PC_YC + k); break;
-                case G1_HF: o->code = (uint8_t)(PC_HF + k); break;
+                case G1_HF:
+                    o->code = (uint8_t)(PC_HF + k);
+                    P.phase = d2(P.phase.x * M_SQRT1_2, P.phase.y * M_SQRT1_2);
+                    break;
                 case G1_RX: o->code = (uint8_t)(PC_RX + k); break;
                 case G1_RY: o->code = (uint8_t)(PC_RY + k); break;
                 default: o->code = (uint8_t)(PC_GEN + k); break;
@@ -1399,13 +1404,12 @@ int build_pass(const std::vector<Gate>& G, const Step& st, uint32_t n, PassParam
             o->coef = (uint16_t)ncoef;
             for (int j = 0; j < 4; ++j) P.coef[ncoef++] = g.m[j];
             if (sub == G1_RX || sub == G1_RY) {
-                // factor out the larger of |cos|, |sin|: its sign joins the
-                // global phase, its magnitude the renormalisation
+                // factor out the larger of |cos|, |sin| into the pass's scalar
                 const double c = g.m[0].x, sn = g.m[0].y;
                 const bool a_form = std::fabs(c) >= std::fabs(sn);
                 const double f = a_form ? c : sn;
                 P.coef[o->coef] = d2(a_form ? sn / c : c / sn, 0.0);
-                if (f < 0) P.phase = d2(-P.phase.x, -P.phase.y);
+                P.phase = d2(P.phase.x * f, P.phase.y * f);
                 if (!a_form) o->code = (uint8_t)((sub == G1_RX ? PC_RXB : PC_RYB) + k);
             }
         } else {  // K_DIAG
@@ -1770,48 +1774,90 @@ int run_gate(qoa_state_t s, const Gate& g) {
     return QOA_OK;
 }
 
-int run_pass(qoa_state_t s, const std::vector<Gate>& G, const Step& st) {
+int do_reset_all(qoa_state_t s);
+
+// How a pass takes its input's squared norm and whether it leaves its own.
+//   in   SCAL_* index: 0 the handle's norm2, SCAL_ONE a normalised input
+//        (the pass before was unitary), SCAL_ZERO |0..0>, which is not read
+//   out  norm partials and their sum into the handle's norm2
+struct PassNorm {
+    int in = 0;
+    bool out = true;
+    bool per_gate = false;  // set where the pass ran as per-gate kernels instead (norm2 is then valid)
+};
+
+// Every gate of the pass is unitary by its kind (not a caller's matrix) and
+// finite: with the factors of build_pass in P.phase, a normalised input gives
+// a normalised output (to rounding), so its norm need not be measured before
+// the next pass. Measured after the last of such a run, as the scale the run
+// has drifted by (of order 1e-16 a gate) belongs to all amplitudes alike.
+bool unitary_pass(const std::vector<Gate>& G, const Step& st) {
+    auto unit = [](double2 d) { return std::fabs(d.x * d.x + d.y * d.y - 1.0) < 1e-12; };
+    for (int gi : st.gates) {
+        const Gate& g = G[gi];
+        if (g.kind == K_DIAG) {
+            if (!g.neg && !(unit(g.m[0]) && (g.t < 0 || unit(g.m[1])))) return false;
+        } else if (g.kind == K_G1) {
+            if (g.sub == G1_GEN) return false;
+            if ((g.sub == G1_RX || g.sub == G1_RY) && !unit(g.m[0])) return false;
+        } else if (g.kind != K_SWAP) {
+            return false;
+        }
+    }
+    return true;
+}
+
+// Sums the pass's norm partials into norm2, where it left them.
+int finish_pass(qoa_state_t s, const PassNorm& nm) {
+    s->launches++;
+    if (!nm.out) return QOA_OK;
+    CK(launch_reduce_partials(s->partials, 1u << (s->n - TILE_BITS), s->scal, s->status, s->stream));
+    s->launches++;
+    return QOA_OK;
+}
+
+// A pass whose parameters were built ahead: its generated kernel when it is
+// ready, else the interpreter.
+int run_pass_built(qoa_state_t s, const PassParams& P, const JitKernel& jk, const PassNorm& nm) {
+    const bool c64 = s->precision == QOA_PREC_F32;
+    const double* in = s->scal + nm.in;
+    double* out = nm.out ? s->partials : nullptr;
+    {
+        Timer tm(s, 2.0 * std::ldexp(c64 ? 8.0 : 16.0, (int)s->n), c64 ? 3 : 0);
+        cudaError_t je = cudaErrorNotReady;
+        if (jk.ready()) {
+            je = jk.launch(s->amps, P, in, out, s->status + 3, s->stream);
+            if (je == cudaSuccess) s->jit_launches++;
+            else if (je != cudaErrorNotSupported) CK(je);
+        }
+        if (je != cudaSuccess) {  // not compiled yet, or its launch set-up unavailable: the interpreter
+            if (c64) CK(launch_pass_p32((float2*)s->amps, P, in, out, s->stream));
+            else CK(launch_pass(s->amps, P, in, out, s->stream));
+        }
+    }
+    return finish_pass(s, nm);
+}
+
+int run_pass(qoa_state_t s, const std::vector<Gate>& G, const Step& st, PassNorm& nm) {
     static thread_local PassParams P;
     if (build_pass(G, st, s->n, P, s->precision == QOA_PREC_F32) != 0) {
-        // op stream too long for one launch: fall back to per-gate kernels
+        // op stream too long for one launch: fall back to per-gate kernels,
+        // which read a written state and its norm
+        if (nm.in == SCAL_ZERO) {
+            int rc = do_reset_all(s);
+            if (rc) return rc;
+        } else if (nm.in == SCAL_ONE) {
+            CK(launch_set_scalar(s->scal, 1.0, s->stream));
+            s->launches++;
+        }
+        nm.per_gate = true;
         for (int gi : st.gates) {
             int rc = run_gate(s, G[gi]);
             if (rc) return rc;
         }
         return QOA_OK;
     }
-    if (s->precision == QOA_PREC_F32) {
-        Timer tm(s, 2.0 * std::ldexp(8.0, (int)s->n), 3);
-        CK(launch_pass_p32((float2*)s->amps, P, s->scal, s->partials, s->stream));
-    } else {
-        Timer tm(s, 2.0 * std::ldexp(16.0, (int)s->n), 0);
-        CK(launch_pass(s->amps, P, s->scal, s->partials, s->stream));
-    }
-    CK(launch_reduce_partials(s->partials, 1u << (s->n - TILE_BITS), s->scal, s->status, s->stream));
-    s->launches += 2;
-    return QOA_OK;
-}
-
-// A pass whose parameters were built ahead: its generated kernel when it is
-// ready, else the interpreter.
-int run_pass_built(qoa_state_t s, const PassParams& P, const JitKernel& jk) {
-    const bool c64 = s->precision == QOA_PREC_F32;
-    {
-        Timer tm(s, 2.0 * std::ldexp(c64 ? 8.0 : 16.0, (int)s->n), c64 ? 3 : 0);
-        cudaError_t je = cudaErrorNotReady;
-        if (jk.ready()) {
-            je = jk.launch(s->amps, P, s->scal, s->partials, s->status + 3, s->stream);
-            if (je == cudaSuccess) s->jit_launches++;
-            else if (je != cudaErrorNotSupported) CK(je);
-        }
-        if (je != cudaSuccess) {  // not compiled yet, or its launch set-up unavailable: the interpreter
-            if (c64) CK(launch_pass_p32((float2*)s->amps, P, s->scal, s->partials, s->stream));
-            else CK(launch_pass(s->amps, P, s->scal, s->partials, s->stream));
-        }
-    }
-    CK(launch_reduce_partials(s->partials, 1u << (s->n - TILE_BITS), s->scal, s->status, s->stream));
-    s->launches += 2;
-    return QOA_OK;
+    return run_pass_built(s, P, JitKernel(), nm);
 }
 
 // Reads norm2, P0, P1 of qubit q (logical probabilities) to the host.
@@ -2052,6 +2098,10 @@ int execute(qoa_state_t s, std::vector<Gate>& G) {
                 return set_err(s, QOA_E_OPCODE, "the FP32 precision form takes unitary ops only");
     const bool per_gate = (s->flags & QOA_FLAG_PER_GATE) != 0;
     // Split at QINIT (changes n) and run each segment through the scheduler.
+    // A reset to |0..0> is not written where a tile pass of this list follows
+    // it (the pass makes its input itself): one sweep of writes and one of
+    // reads less. reset_owed: such a reset has not been written yet.
+    bool reset_owed = false;
     size_t i = 0;
     while (i < G.size()) {
         size_t j = i;
@@ -2116,12 +2166,26 @@ int execute(qoa_state_t s, std::vector<Gate>& G) {
         if (pe->prebuilt && !loaded)
             jk = jit_request(pe->bodies, s->jit_mode == QOA_JIT_SYNC ? JitWhen::WAIT : JitWhen::SECOND_SIGHTING);
         const JitKernel none;  // a kept plan of a state that interprets its passes
+        PassNorm nm;           // nm.in: what the next pass takes
         for (size_t k = 0; k < steps.size(); ++k) {
             const Step& st = steps[k];
-            int rc;
-            if (st.pass && built_of[k] >= 0) rc = run_pass_built(s, built[built_of[k]], pe->prebuilt ? jk[built_of[k]] : none);
-            else if (st.pass) rc = run_pass(s, seg, st);
-            else {
+            int rc = QOA_OK;
+            if (!st.pass && reset_owed && seg[st.gates[0]].kind != K_RESETALL) {  // its kernel reads the state
+                if ((rc = do_reset_all(s))) return rc;
+                reset_owed = false;
+            }
+            if (st.pass) {
+                if (reset_owed) nm.in = SCAL_ZERO;
+                reset_owed = false;
+                // a pass after a unitary pass takes its input as normalised
+                nm.out = !(k + 1 < steps.size() && steps[k + 1].pass && unitary_pass(seg, st));
+                nm.per_gate = false;
+                if (built_of[k] >= 0)
+                    rc = run_pass_built(s, built[built_of[k]], pe->prebuilt ? jk[built_of[k]] : none, nm);
+                else
+                    rc = run_pass(s, seg, st, nm);
+                nm.in = nm.out || nm.per_gate ? 0 : SCAL_ONE;
+            } else {
                 const Gate& g = seg[st.gates[0]];
                 switch (g.kind) {
                     case K_MEASURE: {
@@ -2130,7 +2194,7 @@ int execute(qoa_state_t s, std::vector<Gate>& G) {
                         break;
                     }
                     case K_RESET: rc = do_reset_qubit(s, (uint32_t)g.t); break;
-                    case K_RESETALL: rc = do_reset_all(s); break;
+                    case K_RESETALL: reset_owed = true; break;  // a pass that follows starts from |0..0> unread
                     case K_PERM: rc = run_perm(s, g); break;
                     default: rc = run_gate(s, g);
                 }
@@ -2144,13 +2208,12 @@ int execute(qoa_state_t s, std::vector<Gate>& G) {
                 int rc = alloc_state(s, nn);
                 if (rc) return rc;
             }
-            int rc = do_reset_all(s);
-            if (rc) return rc;
+            reset_owed = true;
             ++j;
         }
         i = j;
     }
-    return QOA_OK;
+    return reset_owed ? do_reset_all(s) : QOA_OK;
 }
 
 int check_handle(qoa_state_t s) {
@@ -2903,10 +2966,9 @@ int batch_prepare(qoa_batch_t b) {
         v->partials_cap = partials_needed(c.n);
         o = al(o + v->partials_cap * sizeof(double));
         v->scal = (double*)(base + o);
-        BCK(cudaMemsetAsync(v->scal, 0, SCAL_DOUBLES * sizeof(double), b->streams[0]));
         o = al(o + SCAL_DOUBLES * sizeof(double));
         v->status = (uint32_t*)(base + o);
-        BCK(cudaMemsetAsync(v->status, 0, 4 * sizeof(uint32_t), b->streams[0]));
+        BCK(launch_init_scalars(v->scal, v->status, b->streams[0]));
         if (tensor) {
             rc = f32_prepare(v, c.gates);
             if (rc) { std::string m = v->err; qoa_destroy(v); return bset_err(b, rc, m.c_str()); }
@@ -3072,11 +3134,9 @@ int qoa_create(uint32_t n, int precision, uint32_t flags, qoa_state_t* out) {
     if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess)
         return fail(set_err(s, QOA_E_CUDA, "stream create failed"));
     if (cudaMalloc(&s->scal, SCAL_DOUBLES * sizeof(double)) != cudaSuccess) return fail(set_err(s, QOA_E_OOM, "scalar alloc"));
-    if (cudaMemsetAsync(s->scal, 0, SCAL_DOUBLES * sizeof(double), s->stream) != cudaSuccess)
-        return fail(set_err(s, QOA_E_CUDA, "scalar memset"));
     if (cudaMalloc(&s->status, 4 * sizeof(uint32_t)) != cudaSuccess) return fail(set_err(s, QOA_E_OOM, "status alloc"));
-    if (cudaMemsetAsync(s->status, 0, 4 * sizeof(uint32_t), s->stream) != cudaSuccess)
-        return fail(set_err(s, QOA_E_CUDA, "status memset"));
+    if (launch_init_scalars(s->scal, s->status, s->stream) != cudaSuccess)
+        return fail(set_err(s, QOA_E_CUDA, "scalar set-up"));
     if (cudaMallocHost(&s->host_scal, (16 + EXPZ_MASKS) * sizeof(double)) != cudaSuccess) return fail(set_err(s, QOA_E_OOM, "pinned alloc"));
     int rc = alloc_state(s, n);
     if (rc) return fail(rc);

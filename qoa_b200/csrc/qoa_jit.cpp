@@ -684,14 +684,13 @@ std::string jit_pass_body_streamed(const PassParams& P) {
         E.line("{");
         E.line("const uint64_t tb = g0 + (uint64_t)lane + ((wid & 1) ? 0x%llxull : 0ull) + ((wid & 2) ? 0x%llxull : 0ull);",
                ostride(m.warp[0]), ostride(m.warp[1]));
-        E.line("double ss = 0.0;");
         for (int v = 0; v < REGS; ++v) {
             unsigned long long off = 0;
             for (int k = 0; k < REG_BITS; ++k)
                 if ((v >> k) & 1) off += ostride(m.reg[k]);
-            E.line("{ const T x = c_mul(a[%d], pend); __stcs(amps + (tb + 0x%llxull), x); ss += c_abs2(x); }", v, off);
+            E.line("a[%d] = c_mul(a[%d], pend); __stcs(amps + (tb + 0x%llxull), a[%d]);", v, v, off, v);
         }
-        E.line("block_norm_partial(ss, red, partials + blk);");
+        E.line("if (partials) block_norm_partial(regs_abs2(a), red, partials + blk);");
         E.line("}");
     }
     E.line("}");  // tile loop
@@ -740,15 +739,14 @@ std::string jit_pass_body(const PassParams& P, bool arena) {
         E.line("{");
         E.line("const uint64_t tb = g0 + (uint64_t)lane + ((wid & 1) ? 0x%llxull : 0ull) + ((wid & 2) ? 0x%llxull : 0ull);",
                ostride(m.warp[0]), ostride(m.warp[1]));
-        if (!arena) E.line("double ss = 0.0;");
         for (int v = 0; v < REGS; ++v) {
             unsigned long long off = 0;
             for (int k = 0; k < REG_BITS; ++k)
                 if ((v >> k) & 1) off += ostride(m.reg[k]);
-            E.line("{ const T x = c_mul(a[%d], pend); __stcs(amps + (tb + 0x%llxull), x);%s }", v, off,
-                   arena ? "" : " ss += c_abs2(x);");
+            E.line("a[%d] = c_mul(a[%d], pend); __stcs(amps + (tb + 0x%llxull), a[%d]);", v, v, off, v);
         }
-        if (!arena) E.line("block_norm_partial(ss, red, partials + blk);");
+        // the squared norm, where the launch asks for it (after the last of a run of unitary passes)
+        if (!arena) E.line("if (partials) block_norm_partial(regs_abs2(a), red, partials + blk);");
         E.line("}");
     }
     E.line("}");
@@ -1076,7 +1074,7 @@ std::string jit_pass32_body_streamed(const PassParams& P) {
                    j, j, j, j, j, j);
             E.line("  __stcs(amps + (tb + 0x%llxull), a); __stcs(amps + (tb + 0x%llxull), b); }", off, off + r3);
         }
-        E.line("block_norm_partial(norm2_p(re, im), red, partials + blk);");
+        E.line("if (partials) block_norm_partial(norm2_p(re, im), red, partials + blk);");
         E.line("}");
     }
     E.line("}");  // tile loop
@@ -1161,7 +1159,7 @@ std::string jit_pass32_body(const PassParams& P, bool arena) {
                    j, j, j, j, j, j);
             E.line("  __stcs(amps + (tb + 0x%llxull), a); __stcs(amps + (tb + 0x%llxull), b); }", off, off + r3);
         }
-        if (!arena) E.line("block_norm_partial(norm2_p(re, im), red, partials + blk);");
+        if (!arena) E.line("if (partials) block_norm_partial(norm2_p(re, im), red, partials + blk);");
         E.line("}");
     }
     E.line("}");

@@ -6,7 +6,8 @@
 // qubits; TILE_BITS, REG_BITS and WARP_BITS in qoa_kernels.cuh). It replaces the per-gate sweeps of src/vectorization.rs:915-1260
 // plus the two normalize() sweeps that follow every gate
 // (src/runtime/quantum_state.rs:839-907): the pass scales its input by the
-// pending 1/||psi|| and leaves per-CTA partial sums of |a|^2 for the next one.
+// pending 1/||psi||, and the last pass of a run of unitary passes leaves
+// per-CTA partial sums of |a|^2 (partials == nullptr: none).
 //
 // The rest: per-gate kernels over global memory (fallback, per-gate mode and
 // the vectorization.rs shims), the measurement reductions and collapse of
@@ -251,6 +252,7 @@ __device__ __forceinline__ void pass_tile(T* __restrict__ amps, const PassParams
     // pass relabelled it); the last mapping has on lane i the tile bit stored
     // to qubit i, so the store is as coalesced as the load.
     double ss = 0.0;
+    const bool norm = partial_out != nullptr;  // uniform over the launch
     {
         const TileMap& mf = cur < 0 ? P.map0 : P.xmap[cur];
         uint64_t tb = g0 + (uint64_t)lane;
@@ -268,7 +270,7 @@ __device__ __forceinline__ void pass_tile(T* __restrict__ amps, const PassParams
                 if ((v >> k) & 1) g += rst[k];
             const T x = c_mul(a[v], pend);
             __stcs(amps + g, x);
-            ss += c_abs2(x);
+            if (norm) ss += c_abs2(x);
         }
     }
     if (!partial_out) return;
@@ -286,7 +288,7 @@ template <typename T>
 __global__ void __launch_bounds__(PASS_THREADS, PassOcc<T>::value)
 k_pass(T* __restrict__ amps, const __grid_constant__ PassParams P, const double* __restrict__ norm2_in,
        double* __restrict__ partials) {
-    pass_tile<T>(amps, P, *norm2_in, blockIdx.x, partials + blockIdx.x);
+    pass_tile<T>(amps, P, *norm2_in, blockIdx.x, partials ? partials + blockIdx.x : nullptr);
 }
 
 // Arena pass: one launch runs one pass of each of many circuits, whose states
@@ -656,6 +658,13 @@ __global__ void k_materialize(double2* __restrict__ a, uint64_t len, const doubl
 
 __global__ void k_set_scalar(double* p, double v) { *p = v; }
 
+// a fresh handle's scalars (norm2 = 1, the constants, ticket 0) and status words
+__global__ void k_init_scalars(double* scal, uint32_t* status) {
+    const int i = threadIdx.x;
+    if (i < SCAL_DOUBLES) scal[i] = (i == 0 || i == SCAL_ONE) ? 1.0 : 0.0;
+    if (i < 4) status[i] = 0;
+}
+
 // Probabilities of [off, off+cnt) scaled by 1/norm2 (|0..0> when invalid).
 __global__ void k_probs(const double2* __restrict__ a, uint64_t off, uint64_t cnt, const double* __restrict__ norm2_in,
                         double* __restrict__ out) {
@@ -783,6 +792,11 @@ cudaError_t launch_materialize(double2* a, uint64_t len, double* norm2, double* 
 
 cudaError_t launch_set_scalar(double* p, double v, cudaStream_t st) {
     k_set_scalar<<<1, 1, 0, st>>>(p, v);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_init_scalars(double* scal, uint32_t* status, cudaStream_t st) {
+    k_init_scalars<<<1, 32, 0, st>>>(scal, status);
     return cudaGetLastError();
 }
 

@@ -47,7 +47,7 @@ struct PassAngle {
 };
 
 // 2x2 forms. Coefficients at coef[c..]:
-//   G1_HF  (a0+a1, a0-a1): the Hadamard with its 1/sqrt2 left to the pass renormalisation
+//   G1_HF  (a0+a1, a0-a1): the Hadamard with its 1/sqrt2 left to PassParams::phase
 //   G1_X   swap; G1_Y (-i a1, i a0)
 //   G1_RX  [[al, -i be], [-i be, al]]  al = coef.x, be = coef.y
 //   G1_RY  [[al, -be], [be, al]]
@@ -120,7 +120,7 @@ struct PassParams {
     uint32_t nops;
     uint32_t ncoef;
     uint32_t pad_;
-    double2 phase;                    // global phase of the factored gates of this pass
+    double2 phase;                    // product of the scalars factored out of this pass's gates
     uint8_t slot_qubit[HIGH_SLOTS];   // global qubit of each high slot (at load)
     uint8_t out_qubit[TILE_BITS];     // global qubit each tile bit is stored to (SWAPs relabel tile bits)
     uint8_t outer_qubits[64];         // qubits outside the tile, ascending (n - TILE_BITS of them)
@@ -163,7 +163,10 @@ struct ExpzMasks {
 // A handle's device scalars: [0] norm2, [1], [2] P0, P1, and the ticket word of
 // kernels whose last CTA finishes the reduction (0 between launches).
 constexpr int SCAL_TICKET = 16;
-constexpr int SCAL_DOUBLES = 17;
+// constants a pass may read as its input's squared norm: 1 (the input is
+// normalised) and 0 (the input is |0..0>, not read)
+constexpr int SCAL_ONE = 17, SCAL_ZERO = 18;
+constexpr int SCAL_DOUBLES = 19;
 
 struct F32Op {
     uint32_t kind;   // 0 = dense block, 1 = phase group

@@ -592,7 +592,7 @@ k_pass_p32x2(float2* __restrict__ amps, const __grid_constant__ PassParams P, co
 __global__ void __launch_bounds__(PASS_THREADS, QOA_PASS_OCC32)
 k_pass_p32(float2* __restrict__ amps, const __grid_constant__ PassParams P, const double* __restrict__ norm2_in,
            double* __restrict__ partials) {
-    pass_tile_p32(amps, P, *norm2_in, blockIdx.x, partials + blockIdx.x);
+    pass_tile_p32(amps, P, *norm2_in, blockIdx.x, partials ? partials + blockIdx.x : nullptr);
 }
 
 __global__ void __launch_bounds__(PASS_THREADS, QOA_PASS_OCC32)

@@ -214,6 +214,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* mb, uint32_t parity, uint32_
     }
 }
 
+// Squared norm of a thread's registers, summed in register order.
+__device__ __forceinline__ double regs_abs2(const double2 (&a)[REGS]) {
+    double ss = 0.0;
+#pragma unroll
+    for (int v = 0; v < REGS; ++v) ss += c_abs2(a[v]);
+    return ss;
+}
+
 // Sum of the block's per-thread squared norms into *out (thread 0 writes).
 __device__ __forceinline__ void block_norm_partial(double ss, double* red, double* out) {
     const int lane = threadIdx.x & 31;
