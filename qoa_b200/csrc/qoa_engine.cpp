@@ -84,9 +84,12 @@ cudaError_t launch_arena_expz(bool f32, const ExpzJob* jobs, uint32_t njobs, uin
                               const uint64_t* masks, double* partials, double* out, cudaStream_t st);
 cudaError_t launch_sample_jobs(bool f32, const SampleJob* jobs, uint32_t njobs, const double* u,
                                unsigned long long* out, cudaStream_t st);
-cudaError_t launch_small_batch(bool f32, const SmallCircuit* circs, uint32_t count, const SmallOp* ops,
-                               const uint64_t* masks, double* out, unsigned int* counter, int max_n, int threads,
+cudaError_t launch_small_batch(bool f32, const SmallCircuit* circs, uint32_t count, const SmallChunkRef* chunks,
+                               const SmallOp* ops, const double2* coef, const uint64_t* masks, double* out, unsigned int* counter, int max_n, int threads,
                                int ctas_per_sm, cudaStream_t st);
+template <int NC>
+cudaError_t launch_small_state(void* amps, bool f32, uint32_t n, const double* norm2_in, const SmallProgram<NC>& P,
+                               double* norm2, uint32_t* status, cudaStream_t st);
 cudaError_t launch_compare(const void* a, bool af32, const void* b, bool bf32, uint64_t len, const double* na,
                            const double* nb, double* partials, double* out3, cudaStream_t st);
 }  // namespace qoa
@@ -1745,6 +1748,183 @@ int build_f32_pass(const std::vector<Gate>& G, const Step& st, uint32_t n, F32Pa
     return 0;
 }
 
+// ---------------------------------------------------------- small circuits
+struct SmallList {
+    std::vector<SmallOp> ops;
+    std::vector<double2> coef;
+    std::vector<SmallChunkRef> chunks;
+};
+
+// The sweeps of a gate list on n qubits (unitary gates only), appended to out
+// as chunks. Greedy like the pass scheduler: a gate joins the open sweep when
+// no waiting gate blocks it and its non-diagonal qubits are among the sweep's
+// three, claiming free ones in the order gates ask for them; the scan looks at
+// most kSmallScan gates ahead.
+constexpr size_t kSmallScan = 96;
+constexpr int kSmallSweepOps = 96, kSmallSweepCoef = 224;  // a sweep takes at most about half a chunk
+
+void small_program(const std::vector<Gate>& G, size_t begin, size_t end, uint32_t n, SmallList& out) {
+    const uint32_t full = (1u << n) - 1;
+    // what the scan reads of a gate, and a list of the waiting ones (a Gate is
+    // ~350 bytes, and each is scanned some ten times)
+    struct Scan {
+        uint16_t nmask, dmask, next;
+        uint8_t nops, ncoef;
+    };
+    static thread_local std::vector<Scan> scan;
+    static thread_local std::vector<int> mine;
+    constexpr size_t kBlock = 60000;  // next is 16 bits: longer lists go in blocks
+    if (end - begin > kBlock) {
+        for (size_t b0 = begin; b0 < end; b0 += kBlock) small_program(G, b0, std::min(end, b0 + kBlock), n, out);
+        return;
+    }
+    const uint32_t count = (uint32_t)(end - begin);
+    scan.resize(count + 1);
+    for (uint32_t i = 0; i < count; ++i) {
+        const Gate& g = G[begin + i];
+        const int o = g.kind == K_SWAP ? 3 : g.kind == K_DIAG ? 2 : 1;
+        const int nc = g.kind == K_U2 ? 16 : g.kind == K_G1 ? 4 : 8;  // a diagonal may become a table
+        scan[i] = Scan{(uint16_t)g.nmask, (uint16_t)g.dmask, (uint16_t)(i + 1), (uint8_t)o, (uint8_t)nc};
+    }
+    uint32_t head = 0;  // first waiting gate (count: none)
+    SmallChunkRef* c = nullptr;
+    auto close = [&] {  // chunks start on an even record
+        if (out.ops.size() & 1) out.ops.push_back(SmallOp{});
+    };
+    while (true) {
+        if (head >= count) return close();
+        uint32_t regs32 = 0, bN = 0, bD = 0;
+        int nops = 1, ncoef = 0;
+        mine.clear();
+        uint32_t prev = count;  // last gate passed over (count: none yet)
+        uint32_t i = head;
+        for (uint32_t seen = 0; i < count && seen < kSmallScan; ++seen) {
+            const Scan g = scan[i];
+            const uint32_t r = regs32 | g.nmask;
+            if (!(g.nmask & (bN | bD)) && !(g.dmask & bN) && __builtin_popcount(r) <= 3 && nops + g.nops <= kSmallSweepOps &&
+                ncoef + g.ncoef <= kSmallSweepCoef) {
+                regs32 = r;
+                nops += g.nops;
+                ncoef += g.ncoef;
+                mine.push_back((int)(begin + i));
+                if (prev == count) head = g.next;
+                else scan[prev].next = g.next;
+            } else {
+                bN |= g.nmask;
+                bD |= g.dmask;
+                prev = i;
+                if ((bN & full) == full) break;
+            }
+            i = g.next;
+        }
+        uint64_t regs = regs32;
+        for (uint32_t q = 0; __builtin_popcountll(regs) < 3; ++q) regs |= 1ull << q;
+        int qs[3], bit_of[64];
+        for (int q = 0; q < 64; ++q) bit_of[q] = -1;
+        {
+            int k = 0;
+            for (uint64_t m = regs; m; m &= m - 1) {
+                qs[k] = __builtin_ctzll(m);
+                bit_of[qs[k]] = k;
+                ++k;
+            }
+        }
+        if (!c || c->nops + nops > SMALL_CHUNK_OPS || c->ncoef + ncoef > SMALL_CHUNK_COEF) {
+            close();
+            out.chunks.push_back(SmallChunkRef{(uint32_t)out.ops.size(), 0, (uint32_t)out.coef.size(), 0});
+            c = &out.chunks.back();
+        }
+        const size_t sw = out.ops.size();
+        out.ops.push_back(SmallOp{SO_SWEEP, 0, 0, (uint32_t)(qs[0] | (qs[1] << 8) | (qs[2] << 16))});
+        c->nops++;
+        auto emit = [&](uint8_t code, int k, uint64_t cmask, const double2* m, int nm) {
+            uint32_t cl = 0;
+            for (int j = 0; j < 3; ++j)
+                if ((cmask >> qs[j]) & 1) cl |= 1u << j;
+            out.ops.push_back(SmallOp{code, (uint8_t)(k | (cl << 4)), (uint16_t)c->ncoef, (uint32_t)(cmask & ~regs)});
+            c->nops++;
+            for (int j = 0; j < nm; ++j) out.coef.push_back(m[j]);
+            c->ncoef += (uint32_t)nm;
+            out.ops[sw].coef++;
+        };
+        // Diagonal gates commute with one another: those on register qubits
+        // alone collect in a table over the 8 register indices until a 2x2
+        // gate on one of their qubits, those on none in the thread's factor.
+        double2 tab[8];
+        uint64_t tab_on = 0;   // register qubits the table depends on
+        const Gate* one = nullptr;  // its only gate
+        auto local = [&](uint64_t mask) {
+            int l = 0;
+            for (int j = 0; j < 3; ++j)
+                if ((mask >> qs[j]) & 1) l |= 1 << j;
+            return l;
+        };
+        auto factor = [&](const Gate& g, int v) -> double2 {  // of register index v (conditions and selector in regs)
+            const int cl = local(g.cmask);
+            if ((v & cl) != cl) return d2(1, 0);
+            if (g.neg) return d2(-1, 0);
+            return g.t >= 0 && ((v >> bit_of[g.t]) & 1) ? g.m[1] : g.m[0];
+        };
+        auto flush_tab = [&] {
+            if (!tab_on) return;
+            if (!one) emit(SO_TAB, 0, 0, tab, 8);
+            else if (one->neg) emit(SO_NEG, 0, one->cmask, nullptr, 0);
+            else if (one->t < 0) emit(SO_DIAG, 0, one->cmask, one->m, 1);
+            else emit(SO_SELR, bit_of[one->t], one->cmask, one->m, 2);
+            tab_on = 0;
+        };
+        for (int gi : mine) {
+            const Gate& g = G[gi];
+            if (g.kind != K_DIAG && (tab_on & (g.nmask | g.dmask))) flush_tab();
+            if (g.kind == K_G1) {
+                const int k = bit_of[g.t];
+                switch (g.sub) {
+                    case G1_H: emit(SO_H, k, g.cmask, g.m, 1); break;
+                    case G1_RX: emit(SO_RX, k, g.cmask, g.m, 1); break;
+                    case G1_RY: emit(SO_RY, k, g.cmask, g.m, 1); break;
+                    case G1_X: emit(SO_X, k, g.cmask, nullptr, 0); break;
+                    case G1_Y: emit(SO_Y, k, g.cmask, nullptr, 0); break;
+                    default: emit(SO_GEN, k, g.cmask, g.m, 4); break;
+                }
+            } else if (g.kind == K_DIAG) {
+                const uint64_t on = g.cmask | (g.t >= 0 ? 1ull << g.t : 0);
+                if (!(on & ~regs)) {
+                    for (int v = 0; v < 8; ++v) {
+                        const double2 f = factor(g, v);
+                        tab[v] = tab_on ? d2(tab[v].x * f.x - tab[v].y * f.y, tab[v].x * f.y + tab[v].y * f.x) : f;
+                    }
+                    one = tab_on ? nullptr : &g;
+                    tab_on |= on;
+                } else if (!(on & regs)) {
+                    if (g.neg) emit(SO_PNEG, 0, g.cmask, nullptr, 0);
+                    else if (g.t < 0) emit(SO_PDIAG, 0, g.cmask, g.m, 1);
+                    else emit(SO_PSEL, g.t, g.cmask, g.m, 2);
+                    out.ops[sw].k = 1;
+                } else if (g.neg) {
+                    emit(SO_NEG, 0, g.cmask, nullptr, 0);
+                } else if (g.t < 0) {
+                    emit(SO_DIAG, 0, g.cmask, g.m, 1);
+                } else {  // a selector with conditions, split between the two: d0, then d1 / d0 where the selector is 1
+                    const double2 d0 = g.m[0], d1 = g.m[1];
+                    const double s2 = d0.x * d0.x + d0.y * d0.y;
+                    const double2 r = d2((d1.x * d0.x + d1.y * d0.y) / s2, (d1.y * d0.x - d1.x * d0.y) / s2);
+                    emit(SO_DIAG, 0, g.cmask, &d0, 1);
+                    emit(SO_DIAG, 0, g.cmask | (1ull << g.t), &r, 1);
+                }
+            } else if (g.kind == K_SWAP) {  // three controlled X
+                const uint64_t a = 1ull << g.t, b = 1ull << g.t2;
+                emit(SO_X, bit_of[g.t2], g.cmask | a, nullptr, 0);
+                emit(SO_X, bit_of[g.t], g.cmask | b, nullptr, 0);
+                emit(SO_X, bit_of[g.t2], g.cmask | a, nullptr, 0);
+            } else {  // K_U2, t < t2
+                const int lo = bit_of[g.t], hi = bit_of[g.t2];
+                emit(SO_U2, lo + hi - 1, g.cmask, g.m, 16);
+            }
+        }
+        flush_tab();
+    }
+}
+
 // ------------------------------------------------------------- execution
 GGate to_ggate(const Gate& g) {
     GGate k;
@@ -1858,6 +2038,36 @@ int run_pass(qoa_state_t s, const std::vector<Gate>& G, const Step& st, PassNorm
         return QOA_OK;
     }
     return run_pass_built(s, P, JitKernel(), nm);
+}
+
+// Runs a small state's chunks, up to three a launch; a reset that is owed is
+// made by the first launch (in: SCAL_* index, as PassNorm::in).
+template <int NC>
+cudaError_t launch_chunks(qoa_state_t s, const SmallList& L, size_t k, size_t cnt, int in) {
+    static thread_local SmallProgram<NC> P;
+    P.nchunks = (uint32_t)cnt;
+    const SmallChunkRef &a = L.chunks[k], &z = L.chunks[k + cnt - 1];
+    for (size_t j = 0; j < cnt; ++j) {
+        P.ref[j] = L.chunks[k + j];
+        P.ref[j].op_start -= a.op_start;
+        P.ref[j].coef_start -= a.coef_start;
+    }
+    std::memcpy(P.ops, &L.ops[a.op_start], (z.op_start + z.nops - a.op_start) * sizeof(SmallOp));
+    if (z.coef_start + z.ncoef > a.coef_start)
+        std::memcpy(P.coef, &L.coef[a.coef_start], (z.coef_start + z.ncoef - a.coef_start) * sizeof(double2));
+    return launch_small_state(s->amps, s->precision == QOA_PREC_F32, s->n, s->scal + in, P, s->scal, s->status, s->stream);
+}
+
+int run_small(qoa_state_t s, const SmallList& L, int in) {
+    for (size_t k = 0; k < L.chunks.size();) {
+        Timer tm(s, 2.0 * std::ldexp(s->precision == QOA_PREC_F32 ? 8.0 : 16.0, (int)s->n), 1);
+        const size_t cnt = std::min<size_t>(3, L.chunks.size() - k);
+        CK(cnt == 1 ? launch_chunks<1>(s, L, k, cnt, in) : launch_chunks<3>(s, L, k, cnt, in));
+        s->launches++;
+        k += cnt;
+        in = 0;
+    }
+    return QOA_OK;
 }
 
 // Reads norm2, P0, P1 of qubit q (logical probabilities) to the host.
@@ -2089,6 +2299,152 @@ int state_pass_budget(qoa_state_t s) {
     return s->pass_budget ? s->pass_budget : env;
 }
 
+// A measurement or reset of an op list. reset_owed: a reset to |0..0> that has
+// not been written (see execute).
+int run_barrier(qoa_state_t s, const Gate& g, bool& reset_owed) {
+    if (g.kind == K_RESETALL) {
+        reset_owed = true;
+        return QOA_OK;
+    }
+    if (reset_owed) {
+        const int rc = do_reset_all(s);
+        if (rc) return rc;
+        reset_owed = false;
+    }
+    if (g.kind == K_MEASURE) {
+        const double u = g.u >= 0 ? g.u : next_meas_uniform(s);
+        return do_measure(s, (uint32_t)g.t, u, nullptr);
+    }
+    return do_reset_qubit(s, (uint32_t)g.t);
+}
+
+// States small enough run whole in shared memory, unless generated pass
+// kernels or searched plans are asked for at their size. Up to 10 qubits there
+// are no tile passes; at 11 the shared-memory launch wins at every length
+// measured (33 to 513 gates: 25-150 us against 37-169); at 12 it wins up to
+// ~200 gates (30-52 against 40-63 us) and loses on long lists of full layers
+// (561 gates 200 against 163 us, once the plan is kept), at 13 one SM's FP64
+// rate would bound it.
+bool small_route(qoa_state_t s) {
+    if (s->flags & QOA_FLAG_PER_GATE) return false;
+    if (s->n < (uint32_t)TILE_BITS) return true;
+    return s->n <= (uint32_t)SMALL_STATE_MAX && !(s->flags & QOA_FLAG_SLOT_SEARCH) &&
+           (s->jit_mode == QOA_JIT_OFF || s->n < s->jit_min_qubits);
+}
+
+int run_small_list(qoa_state_t s, const std::vector<Gate>& seg, bool& reset_owed) {
+    size_t a = 0;
+    while (a < seg.size()) {
+        size_t b = a;
+        while (b < seg.size() && seg[b].kind <= K_U2) ++b;
+        int rc;
+        if (b > a) {
+            SmallList list;
+            small_program(seg, a, b, s->n, list);
+            rc = run_small(s, list, reset_owed ? SCAL_ZERO : 0);
+            reset_owed = false;
+        } else {
+            rc = run_barrier(s, seg[b++], reset_owed);
+        }
+        if (rc) return rc;
+        a = b;
+    }
+    return QOA_OK;
+}
+
+// A gate list through the pass scheduler.
+int run_planned(qoa_state_t s, std::vector<Gate>& seg, bool& reset_owed) {
+    const bool c64 = s->precision == QOA_PREC_F32;
+    const bool per_gate = (s->flags & QOA_FLAG_PER_GATE) != 0;
+    if (!per_gate) merge_swap_blocks(seg);
+    const bool jit = !per_gate && s->jit_mode != QOA_JIT_OFF && s->n >= s->jit_min_qubits;
+    // a repeated op list reuses its plan
+    PlanEntry local;
+    PlanEntry* pe = &local;
+    bool cache_it = false;
+    if (!per_gate && s->n > (uint32_t)TILE_BITS) {
+        if (!s->plans) s->plans = std::make_shared<PlanCache>();
+        PlanCache& pc = *static_cast<PlanCache*>(s->plans.get());
+        const uint64_t key = (uint64_t)s->n | ((uint64_t)c64 << 8) | ((uint64_t)jit << 9) |
+                             ((uint64_t)(uint32_t)state_pass_budget(s) << 16);
+        plan_hash(seg, key, local.h1, local.h2);
+        for (auto& e : pc.entries)
+            if (e.h1 == local.h1 && e.h2 == local.h2) pe = &e;
+        if (pe == &local) {
+            if (pc.seen.size() > 4096) pc.seen.clear();
+            cache_it = pc.seen[local.h1]++ > 0;
+        }
+    }
+    const bool fresh = pe == &local;
+    if (fresh) {
+        // the plan depends on the op list and the size only, so a list
+        // executed again gives bit-identical results
+        pe->steps = schedule(seg, s->n, per_gate, false, state_pass_budget(s),
+                             slot_search_pays(s->n) || (s->flags & QOA_FLAG_SLOT_SEARCH));
+        pe->built_of.assign(pe->steps.size(), -1);
+        // passes built ahead: for generated kernels, whose text is
+        // requested from the compile cache, and for a plan that is kept
+        if (jit || cache_it) {
+            size_t np = 0;
+            for (const Step& st : pe->steps) np += st.pass ? 1 : 0;
+            pe->built.resize(np);
+            size_t b = 0;
+            for (size_t k = 0; k < pe->steps.size(); ++k) {
+                if (!pe->steps[k].pass || build_pass(seg, pe->steps[k], s->n, pe->built[b], c64) != 0) continue;
+                pe->built_of[k] = (int)b;
+                if (jit) pe->bodies.push_back(c64 ? jit_pass32_body(pe->built[b]) : jit_pass_body(pe->built[b]));
+                ++b;
+            }
+            pe->prebuilt = jit;
+        }
+        if (cache_it) {
+            PlanCache& pc = *static_cast<PlanCache*>(s->plans.get());
+            if (pc.entries.size() >= PlanCache::kEntries) pc.entries.pop_front();
+            pc.entries.push_back(std::move(local));
+            pe = &pc.entries.back();
+        }
+    }
+    const std::vector<Step>& steps = pe->steps;
+    const std::vector<PassParams>& built = pe->built;
+    const std::vector<int>& built_of = pe->built_of;
+    // once all of a kept plan's kernels are loaded they are not looked up
+    // again (a request hashes every kernel's text, ~0.5 ms for 16 passes)
+    std::vector<JitKernel>& jk = pe->kernels;
+    bool loaded = pe->prebuilt && jk.size() == pe->bodies.size();
+    for (size_t b = 0; loaded && b < jk.size(); ++b) loaded = jk[b].ready();
+    if (pe->prebuilt && !loaded)
+        jk = jit_request(pe->bodies, s->jit_mode == QOA_JIT_SYNC ? JitWhen::WAIT : JitWhen::SECOND_SIGHTING);
+    const JitKernel none;  // a kept plan of a state that interprets its passes
+    PassNorm nm;           // nm.in: what the next pass takes
+    for (size_t k = 0; k < steps.size(); ++k) {
+        const Step& st = steps[k];
+        int rc = QOA_OK;
+        if (st.pass) {
+            if (reset_owed) nm.in = SCAL_ZERO;
+            reset_owed = false;
+            // a pass after a unitary pass takes its input as normalised
+            nm.out = !(k + 1 < steps.size() && steps[k + 1].pass && unitary_pass(seg, st));
+            nm.per_gate = false;
+            if (built_of[k] >= 0)
+                rc = run_pass_built(s, built[built_of[k]], pe->prebuilt ? jk[built_of[k]] : none, nm);
+            else
+                rc = run_pass(s, seg, st, nm);
+            nm.in = nm.out || nm.per_gate ? 0 : SCAL_ONE;
+        } else {
+            const Gate& g = seg[st.gates[0]];
+            if (is_barrier(g) && g.kind != K_PERM) {
+                rc = run_barrier(s, g, reset_owed);
+            } else {
+                if (reset_owed) rc = do_reset_all(s);  // the kernel reads the state
+                reset_owed = false;
+                if (!rc) rc = g.kind == K_PERM ? run_perm(s, g) : run_gate(s, g);
+            }
+        }
+        if (rc) return rc;
+    }
+    return QOA_OK;
+}
+
 int execute(qoa_state_t s, std::vector<Gate>& G) {
     const bool c64 = s->precision == QOA_PREC_F32;
     if (c64 && (s->flags & QOA_FLAG_F32_TENSOR)) return execute_f32(s, G);
@@ -2096,7 +2452,6 @@ int execute(qoa_state_t s, std::vector<Gate>& G) {
         for (const Gate& g : G)
             if (g.kind > K_U2 && g.kind != K_RESETALL)
                 return set_err(s, QOA_E_OPCODE, "the FP32 precision form takes unitary ops only");
-    const bool per_gate = (s->flags & QOA_FLAG_PER_GATE) != 0;
     // Split at QINIT (changes n) and run each segment through the scheduler.
     // A reset to |0..0> is not written where a tile pass of this list follows
     // it (the pass makes its input itself): one sweep of writes and one of
@@ -2107,100 +2462,8 @@ int execute(qoa_state_t s, std::vector<Gate>& G) {
         size_t j = i;
         while (j < G.size() && G[j].kind != K_QINIT) ++j;
         std::vector<Gate> seg(G.begin() + i, G.begin() + j);
-        if (!per_gate) merge_swap_blocks(seg);
-        const bool jit = !per_gate && s->jit_mode != QOA_JIT_OFF && s->n >= s->jit_min_qubits;
-        // a repeated op list reuses its plan
-        PlanEntry local;
-        PlanEntry* pe = &local;
-        bool cache_it = false;
-        if (!per_gate && s->n > (uint32_t)TILE_BITS) {
-            if (!s->plans) s->plans = std::make_shared<PlanCache>();
-            PlanCache& pc = *static_cast<PlanCache*>(s->plans.get());
-            const uint64_t key = (uint64_t)s->n | ((uint64_t)c64 << 8) | ((uint64_t)jit << 9) |
-                                 ((uint64_t)(uint32_t)state_pass_budget(s) << 16);
-            plan_hash(seg, key, local.h1, local.h2);
-            for (auto& e : pc.entries)
-                if (e.h1 == local.h1 && e.h2 == local.h2) pe = &e;
-            if (pe == &local) {
-                if (pc.seen.size() > 4096) pc.seen.clear();
-                cache_it = pc.seen[local.h1]++ > 0;
-            }
-        }
-        const bool fresh = pe == &local;
-        if (fresh) {
-            // the plan depends on the op list and the size only, so a list
-            // executed again gives bit-identical results
-            pe->steps = schedule(seg, s->n, per_gate, false, state_pass_budget(s),
-                                 slot_search_pays(s->n) || (s->flags & QOA_FLAG_SLOT_SEARCH));
-            pe->built_of.assign(pe->steps.size(), -1);
-            // passes built ahead: for generated kernels, whose text is
-            // requested from the compile cache, and for a plan that is kept
-            if (jit || cache_it) {
-                size_t np = 0;
-                for (const Step& st : pe->steps) np += st.pass ? 1 : 0;
-                pe->built.resize(np);
-                size_t b = 0;
-                for (size_t k = 0; k < pe->steps.size(); ++k) {
-                    if (!pe->steps[k].pass || build_pass(seg, pe->steps[k], s->n, pe->built[b], c64) != 0) continue;
-                    pe->built_of[k] = (int)b;
-                    if (jit) pe->bodies.push_back(c64 ? jit_pass32_body(pe->built[b]) : jit_pass_body(pe->built[b]));
-                    ++b;
-                }
-                pe->prebuilt = jit;
-            }
-            if (cache_it) {
-                PlanCache& pc = *static_cast<PlanCache*>(s->plans.get());
-                if (pc.entries.size() >= PlanCache::kEntries) pc.entries.pop_front();
-                pc.entries.push_back(std::move(local));
-                pe = &pc.entries.back();
-            }
-        }
-        const std::vector<Step>& steps = pe->steps;
-        const std::vector<PassParams>& built = pe->built;
-        const std::vector<int>& built_of = pe->built_of;
-        // once all of a kept plan's kernels are loaded they are not looked up
-        // again (a request hashes every kernel's text, ~0.5 ms for 16 passes)
-        std::vector<JitKernel>& jk = pe->kernels;
-        bool loaded = pe->prebuilt && jk.size() == pe->bodies.size();
-        for (size_t b = 0; loaded && b < jk.size(); ++b) loaded = jk[b].ready();
-        if (pe->prebuilt && !loaded)
-            jk = jit_request(pe->bodies, s->jit_mode == QOA_JIT_SYNC ? JitWhen::WAIT : JitWhen::SECOND_SIGHTING);
-        const JitKernel none;  // a kept plan of a state that interprets its passes
-        PassNorm nm;           // nm.in: what the next pass takes
-        for (size_t k = 0; k < steps.size(); ++k) {
-            const Step& st = steps[k];
-            int rc = QOA_OK;
-            if (!st.pass && reset_owed && seg[st.gates[0]].kind != K_RESETALL) {  // its kernel reads the state
-                if ((rc = do_reset_all(s))) return rc;
-                reset_owed = false;
-            }
-            if (st.pass) {
-                if (reset_owed) nm.in = SCAL_ZERO;
-                reset_owed = false;
-                // a pass after a unitary pass takes its input as normalised
-                nm.out = !(k + 1 < steps.size() && steps[k + 1].pass && unitary_pass(seg, st));
-                nm.per_gate = false;
-                if (built_of[k] >= 0)
-                    rc = run_pass_built(s, built[built_of[k]], pe->prebuilt ? jk[built_of[k]] : none, nm);
-                else
-                    rc = run_pass(s, seg, st, nm);
-                nm.in = nm.out || nm.per_gate ? 0 : SCAL_ONE;
-            } else {
-                const Gate& g = seg[st.gates[0]];
-                switch (g.kind) {
-                    case K_MEASURE: {
-                        const double u = g.u >= 0 ? g.u : next_meas_uniform(s);
-                        rc = do_measure(s, (uint32_t)g.t, u, nullptr);
-                        break;
-                    }
-                    case K_RESET: rc = do_reset_qubit(s, (uint32_t)g.t); break;
-                    case K_RESETALL: reset_owed = true; break;  // a pass that follows starts from |0..0> unread
-                    case K_PERM: rc = run_perm(s, g); break;
-                    default: rc = run_gate(s, g);
-                }
-            }
-            if (rc) return rc;
-        }
+        const int src = seg.empty() ? QOA_OK : small_route(s) ? run_small_list(s, seg, reset_owed) : run_planned(s, seg, reset_owed);
+        if (src) return src;
         if (j < G.size()) {  // QINIT
             const uint32_t nn = (uint32_t)G[j].t;
             if (nn != s->n) {
@@ -2329,7 +2592,9 @@ struct qoa_batch_s {
     std::vector<cudaEvent_t> events;
     void* arena = nullptr;
     SmallCircuit* d_small = nullptr;
+    SmallChunkRef* d_chunks = nullptr;
     SmallOp* d_ops = nullptr;
+    double2* d_coef = nullptr;
     uint64_t* d_masks = nullptr;   // every circuit's masks, in order of addition
     double* d_out = nullptr;
     unsigned int* d_counter = nullptr;
@@ -2398,33 +2663,8 @@ int bset_err(qoa_batch_t b, int code, const char* msg) {
         }                                                                           \
     } while (0)
 
-bool small_ok(const Gate& g) { return g.kind == K_G1 || g.kind == K_DIAG || g.kind == K_SWAP; }
-
-SmallOp to_small(const Gate& g) {
-    SmallOp o;
-    memset(&o, 0, sizeof o);
-    o.cmask = (uint32_t)g.cmask;
-    if (g.kind == K_G1) {
-        o.kind = SK_G1;
-        o.t = (uint8_t)g.t;
-        cplx m[4];
-        g1_exact(g, m);
-        for (int k = 0; k < 4; ++k) o.m[k] = d2(m[k].real(), m[k].imag());
-    } else if (g.kind == K_DIAG) {
-        o.kind = SK_DIAG;
-        o.t = g.t >= 0 ? (uint8_t)g.t : 255;
-        if (g.neg) o.m[0] = o.m[1] = d2(-1, 0);
-        else {
-            o.m[0] = g.m[0];
-            o.m[1] = g.t >= 0 ? g.m[1] : g.m[0];
-        }
-    } else {
-        o.kind = SK_SWAP;
-        o.t = (uint8_t)g.t;
-        o.t2 = (uint8_t)g.t2;
-    }
-    return o;
-}
+// tensor batches refuse U2 on circuits below a tile, as their blocks do not take it there
+bool small_ok(const Gate& g, bool tensor) { return g.kind < K_U2 || (g.kind == K_U2 && !tensor); }
 
 template <typename T>
 void dfree(T*& p, cudaStream_t st) {
@@ -2505,7 +2745,7 @@ void batch_free_device(qoa_batch_t b) {
     // every stream of a run is joined into stream 0, so frees ordered there
     // follow all of the batch's work
     cudaStream_t st = b->streams.empty() ? nullptr : b->streams[0];
-    dfree(b->arena, st); dfree(b->d_small, st); dfree(b->d_ops, st); dfree(b->d_masks, st); dfree(b->d_out, st);
+    dfree(b->arena, st); dfree(b->d_small, st); dfree(b->d_chunks, st); dfree(b->d_ops, st); dfree(b->d_coef, st); dfree(b->d_masks, st); dfree(b->d_out, st);
     dfree(b->d_counter, st); dfree(b->d_params, st); dfree(b->d_f32, st); dfree(b->d_jobs, st); dfree(b->d_tstart, st);
     dfree(b->d_ejobs, st); dfree(b->d_epart, st);
     dfree(b->d_shot_u, st); dfree(b->d_shot_out, st); dfree(b->d_sjobs, st); dfree(b->d_trees, st);
@@ -2607,7 +2847,7 @@ int batch_prepare(qoa_batch_t b) {
     auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
 
     std::vector<SmallCircuit> sc;
-    std::vector<SmallOp> sops;
+    SmallList slist;
     std::vector<uint64_t> masks;
     std::vector<uint32_t> mask_start(b->circs.size());
     for (size_t i = 0; i < b->circs.size(); ++i) {
@@ -2633,7 +2873,7 @@ int batch_prepare(qoa_batch_t b) {
     for (size_t i = 0; i < NC; ++i) {
         const auto& c = b->circs[i];
         bool small = c.n <= smax || (tensor && c.n < (uint32_t)TILE_BITS);
-        for (const Gate& g : c.gates) small = small && small_ok(g);
+        for (const Gate& g : c.gates) small = small && small_ok(g, tensor);
         is_small[i] = small;
     }
     // Tile-pass route, planned on all host cores: schedule every candidate
@@ -2642,9 +2882,12 @@ int batch_prepare(qoa_batch_t b) {
     std::vector<char> all_pass(NC, 0), built_ok(NC, 0);
     std::vector<size_t> pbase(NC, 0);
     if (!tensor) {
-        parallel_for(NC, [&](size_t i) {
+        std::vector<size_t> cands;
+        for (size_t i = 0; i < NC; ++i)
+            if (!is_small[i] && b->circs[i].n >= (uint32_t)TILE_BITS && !b->circs[i].gates.empty()) cands.push_back(i);
+        parallel_for(cands.size(), [&](size_t x) {
+            const size_t i = cands[x];
             const auto& c = b->circs[i];
-            if (is_small[i] || c.n < (uint32_t)TILE_BITS || c.gates.empty()) return;
             steps_of[i] = schedule(c.gates, c.n, false, false, budget);
             bool ok = true;
             for (const Step& st : steps_of[i]) ok = ok && st.pass;
@@ -2689,9 +2932,9 @@ int batch_prepare(qoa_batch_t b) {
             c.route = R_SMALL;
             SmallCircuit d;
             d.n = c.n;
-            d.op_start = (uint32_t)sops.size();
-            for (const Gate& g : c.gates) sops.push_back(to_small(g));
-            d.op_count = (uint32_t)c.gates.size();
+            d.chunk_start = (uint32_t)slist.chunks.size();
+            small_program(c.gates, 0, c.gates.size(), c.n, slist);
+            d.chunk_count = (uint32_t)slist.chunks.size() - d.chunk_start;
             d.mask_start = mask_start[i];
             d.mask_count = (uint32_t)c.masks.size();
             d.out_start = c.out_start;
@@ -2769,7 +3012,9 @@ int batch_prepare(qoa_batch_t b) {
             ++k;
         }
         if ((rc = upload(b, b->d_small, sc))) return rc;
-        if ((rc = upload(b, b->d_ops, sops))) return rc;
+        if ((rc = upload(b, b->d_chunks, slist.chunks))) return rc;
+        if ((rc = upload(b, b->d_ops, slist.ops))) return rc;
+        if ((rc = upload(b, b->d_coef, slist.coef))) return rc;
     }
     if (shot_total) {
         std::vector<SampleJob> sj;
@@ -2990,7 +3235,7 @@ int batch_enqueue(qoa_batch_t b) {
     for (uint32_t i = 1; i < ns; ++i) BCK(cudaStreamWaitEvent(b->streams[i], b->events[0], 0));
     // small circuits beside the arena rounds
     if (b->nsmall) {
-        BCK(launch_small_batch(f32, b->d_small, b->nsmall, b->d_ops, b->d_masks, b->d_out, b->d_counter,
+        BCK(launch_small_batch(f32, b->d_small, b->nsmall, b->d_chunks, b->d_ops, b->d_coef, b->d_masks, b->d_out, b->d_counter,
                                (int)b->small_max_n_used, (int)b->tune.small_threads, (int)b->tune.small_ctas_per_sm,
                                b->streams[ns > 1 ? 1 : 0]));
     }

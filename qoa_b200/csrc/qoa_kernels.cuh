@@ -209,20 +209,56 @@ struct F32PassParams {
 };
 
 // ---------------------------------------------------------------------------
-// Batched small circuits (qoa_batch.cu): whole state in shared memory
+// Small states (qoa_small.cu): whole state in shared memory
 // ---------------------------------------------------------------------------
 constexpr int SMALL_MAX_F64 = 12;  // 2^12 complex128 = 64 KB
 constexpr int SMALL_MAX_F32 = 13;  // 2^13 complex64 = 64 KB
 
-enum SmallKind : uint8_t { SK_G1 = 0, SK_DIAG = 1, SK_SWAP = 2 };
+// A handle's op lists on up to this many qubits run whole in shared memory too.
+constexpr int SMALL_STATE_MAX = 12;
 
+// One record of a small circuit (qoa_small.cu). SO_SWEEP opens a sweep: its
+// three register qubits (ascending, one byte each of co) and in coef the
+// number of gate records that follow. Gates: k = register bit in the low four
+// bits (SO_PSEL: the selecting qubit; SO_U2: 0, 1, 2 for the register-bit
+// pairs 01, 02, 12) and register-bit conditions in the high four; co =
+// conditions on the other qubits; coef = first coefficient.
+enum SmallCode : uint8_t {
+    SO_SWEEP = 0, SO_H, SO_RX, SO_RY, SO_GEN, SO_X, SO_Y,
+    SO_NEG,   // -1
+    SO_DIAG,  // coef[0]
+    SO_SELR,  // coef[register bit k]
+    SO_TAB,   // coef[register index]: a product of phases on register qubits
+    SO_U2,
+    // phases of a whole thread, collected in one factor that the sweep's end
+    // applies (SO_SWEEP's k = 1 where there are any)
+    SO_PNEG, SO_PDIAG,
+    SO_PSEL,  // coef[index bit k]
+};
 struct SmallOp {
-    uint8_t kind;
-    uint8_t sub;
-    uint8_t t;       // target / selector (255: none)
-    uint8_t t2;
-    uint32_t cmask;  // condition: every bit set
-    double2 m[4];    // SK_G1: m00 m01 m10 m11; SK_DIAG: d0, d1
+    uint8_t code;
+    uint8_t k;
+    uint16_t coef;
+    uint32_t co;
+};
+// Whole sweeps, as many as fit in SMALL_CHUNK_OPS records and SMALL_CHUNK_COEF
+// coefficients; a kernel stages one chunk at a time. op_start is even, so that
+// records are copied as 16-byte words.
+constexpr int SMALL_CHUNK_OPS = 256;
+constexpr int SMALL_CHUNK_COEF = 448;
+struct SmallChunkRef {
+    uint32_t op_start, nops, coef_start, ncoef;
+};
+struct alignas(16) SmallChunk {
+    SmallOp ops[SMALL_CHUNK_OPS];
+    double2 coef[SMALL_CHUNK_COEF];
+};
+template <int NC>
+struct SmallProgram {  // a launch's parameter: NC chunks, or fewer
+    uint32_t nchunks, pad_[3];
+    SmallChunkRef ref[NC];  // into ops and coef
+    SmallOp ops[NC * SMALL_CHUNK_OPS];
+    double2 coef[NC * SMALL_CHUNK_COEF];
 };
 
 // Arena circuits' <Z_mask>: sums per tile of EXPZ_CHUNK amplitudes, then one CTA per circuit.
@@ -240,7 +276,7 @@ struct ExpzJob {
 
 struct SmallCircuit {
     uint32_t n;
-    uint32_t op_start, op_count;
+    uint32_t chunk_start, chunk_count;
     uint32_t mask_start, mask_count;
     uint32_t out_start;
     void* state_out;  // where the final state is written (circuits that are sampled), else null
