@@ -76,7 +76,7 @@ cudaError_t launch_pass_p32_arena(const ArenaJob* jobs, uint32_t njobs, const ui
                                   int max_nops, int max_ncoef, cudaStream_t st);
 cudaError_t launch_gate_c64(float2* a, uint64_t len, const GGate& g, cudaStream_t st);
 cudaError_t launch_pass_arena(const ArenaJob* jobs, uint32_t njobs, const uint32_t* tile_start, uint32_t tiles,
-                              int max_nops, int max_ncoef, cudaStream_t st);
+                              int max_nops, int max_ncoef, bool any_u2, cudaStream_t st);
 cudaError_t launch_f32_pass_arena(const ArenaJob* jobs, uint32_t njobs, const uint32_t* tile_start, uint32_t tiles,
                                   const float* mats, const F32PhaseOp* pops, const F32Angle* angles,
                                   const F32Phase* phases, const float2* tables, uint32_t* status, cudaStream_t st);
@@ -272,8 +272,10 @@ inline double2 from_polar(double r, double t) { return d2(r * std::cos(t), r * s
 
 // Tile passes take every diagonal gate and the 2x2 gates; a controlled 2x2
 // must be X or Y (CNOT, Toffoli, CY), which is all the instruction set makes.
-bool is_pass_gate(const Gate& g) {
+// Complex128 passes also take 4x4 gates (u2).
+bool is_pass_gate(const Gate& g, bool u2) {
     if (g.kind == K_DIAG) return true;
+    if (g.kind == K_U2) return u2;
     if (g.kind == K_SWAP) return g.cmask == 0;  // a relabelling of two tile bits
     return g.kind == K_G1 && (g.cmask == 0 || g.sub == G1_X || g.sub == G1_Y);
 }
@@ -826,7 +828,7 @@ uint64_t tile_need(const Gate& g, bool f32) {
 // slot_weight 0: in-order greedy only; w > 0: slot search scoring a
 // diagonal gate 1 and any other gate w.
 std::vector<Step> schedule_pass_order(const std::vector<Gate>& G, uint32_t n, bool per_gate, bool f32,
-                                      int gate_budget, int slot_weight) {
+                                      int gate_budget, int slot_weight, bool u2) {
     const bool slot_search = slot_weight > 0;
     std::vector<Step> steps;
     const size_t N = G.size();
@@ -837,7 +839,7 @@ std::vector<Step> schedule_pass_order(const std::vector<Gate>& G, uint32_t n, bo
         while (first < N && done[first]) ++first;
         if (first >= N) break;
         const Gate& g0 = G[first];
-        if (!tiles || !(f32 ? is_pass_gate_f32(g0) : is_pass_gate(g0))) {
+        if (!tiles || !(f32 ? is_pass_gate_f32(g0) : is_pass_gate(g0, u2))) {
             Step st;
             st.gates.push_back((int)first);
             done[first] = 1;
@@ -855,17 +857,20 @@ std::vector<Step> schedule_pass_order(const std::vector<Gate>& G, uint32_t n, bo
             int budget_ops = MAX_PASS_OPS / 3;  // room for the exchanges and flushes
             if (gate_budget > 0 && gate_budget < budget_ops) budget_ops = gate_budget;
             int budget_coef = MAX_PASS_COEF - 8;
+            int budget_u2 = MAX_XCHG / 2;  // a 4x4 may need an exchange of its own
             for (size_t i = first; i < N; ++i) {
                 if (done[i]) continue;
                 const Gate& g = G[i];
                 if (is_barrier(g)) break;
-                bool ok = (f32 ? is_pass_gate_f32(g) : is_pass_gate(g)) && !(g.nmask & (bN | bD)) && !(g.dmask & bN);
+                bool ok = (f32 ? is_pass_gate_f32(g) : is_pass_gate(g, u2)) && !(g.nmask & (bN | bD)) && !(g.dmask & bN);
                 if (ok) {
                     const uint64_t need = tile_need(g, f32) & ~tile;
                     const int k = __builtin_popcountll(need);
-                    const int nc = g.kind == K_G1 ? 4 : 2;  // a selector diagonal becomes two phase ops
-                    if (nslots + k > HIGH_SLOTS || budget_ops < 1 || budget_coef < nc) ok = false;
+                    const int nc = g.kind == K_U2 ? 16 : g.kind == K_G1 ? 4 : 2;  // a selector diagonal becomes two phase ops
+                    const int u = g.kind == K_U2 && !f32 ? 1 : 0;
+                    if (nslots + k > HIGH_SLOTS || budget_ops < 1 || budget_coef < nc || budget_u2 < u) ok = false;
                     else {
+                        budget_u2 -= u;
                         tile |= need;
                         nslots += k;
                         budget_ops -= 1;
@@ -944,15 +949,15 @@ std::vector<Step> schedule_pass_order(const std::vector<Gate>& G, uint32_t n, bo
 bool slot_search_pays(uint32_t n) { return n >= 26; }
 
 std::vector<Step> schedule(const std::vector<Gate>& G, uint32_t n, bool per_gate, bool f32 = false,
-                           int gate_budget = 0, bool search_wanted = false) {
+                           int gate_budget = 0, bool search_wanted = false, bool u2 = false) {
     static const bool search_on = [] {
         const char* v = getenv("QOA_SCHED_SEARCH");
         return !(v && v[0] == '0');
     }();
-    std::vector<Step> best = schedule_pass_order(G, n, per_gate, f32, gate_budget, 0);
+    std::vector<Step> best = schedule_pass_order(G, n, per_gate, f32, gate_budget, 0, u2);
     if (!search_wanted || !search_on || per_gate || n <= (uint32_t)TILE_BITS || best.size() < 2) return best;
     for (int w : {1, 2}) {
-        std::vector<Step> t = schedule_pass_order(G, n, per_gate, f32, gate_budget, w);
+        std::vector<Step> t = schedule_pass_order(G, n, per_gate, f32, gate_budget, w, u2);
         if (t.size() < best.size()) best.swap(t);
     }
     return best;
@@ -1001,14 +1006,15 @@ int build_pass(const std::vector<Gate>& G, const Step& st, uint32_t n, PassParam
 
     // register demand per gate (tile bit of each 2x2 target)
     const int ng = (int)st.gates.size();
-    std::vector<int> need(ng, -1);
+    std::vector<int> need(ng, -1), need2(ng, -1);  // (need2: the higher qubit of a 4x4)
     int final_q[TILE_BITS];  // qubit each tile bit is stored to
     {
         int tb_sim[64];
         std::memcpy(tb_sim, tb_of, sizeof tb_of);
         for (int i = 0; i < ng; ++i) {
             const Gate& g = G[st.gates[i]];
-            if (g.kind == K_G1) need[i] = tb_sim[g.t];
+            if (g.kind == K_G1 || g.kind == K_U2) need[i] = tb_sim[g.t];
+            if (g.kind == K_U2) need2[i] = tb_sim[g.t2];
             else if (g.kind == K_SWAP) relabel(tb_sim, g);
         }
         for (int q = 0; q < 64; ++q)
@@ -1023,7 +1029,7 @@ int build_pass(const std::vector<Gate>& G, const Step& st, uint32_t n, PassParam
             if (final_q[t] < LANE_BITS) continue;
             int uses = 0, first = 1 << 30;
             for (int i = 0; i < ng; ++i)
-                if (need[i] == t) { ++uses; first = std::min(first, i); }
+                if (need[i] == t || need2[i] == t) { ++uses; first = std::min(first, i); }
             if (uses < best_uses || (uses == best_uses && first > best_first)) {
                 best_uses = uses; best_first = first; pin = t;
             }
@@ -1036,6 +1042,7 @@ int build_pass(const std::vector<Gate>& G, const Step& st, uint32_t n, PassParam
     for (int i = ng - 1; i >= 0; --i) {
         nu[i] = nu[i + 1];
         if (need[i] >= 0) nu[i][need[i]] = i;
+        if (need2[i] >= 0) nu[i][need2[i]] = i;
     }
     auto next_use = [&](int from, int t) { return from >= ng ? (1 << 30) : nu[from][t]; };
 
@@ -1245,10 +1252,10 @@ int build_pass(const std::vector<Gate>& G, const Step& st, uint32_t n, PassParam
         m = nm;
         return true;
     };
-    // bring tile bit `must` into the registers
-    auto make_reg = [&](int i, int must) -> bool {
+    // bring tile bit `must` (and `must2`) into the registers
+    auto make_reg = [&](int i, int must, int must2 = -1) -> bool {
         std::vector<std::pair<int, int>> c;
-        for (int t = 0; t < TILE_BITS; ++t) c.push_back({t == must ? -1 : (t == pin ? -2 : next_use(i, t)), t});
+        for (int t = 0; t < TILE_BITS; ++t) c.push_back({t == must || t == must2 ? -1 : (t == pin ? -2 : next_use(i, t)), t});
         std::sort(c.begin(), c.end());
         bool want[TILE_BITS] = {};
         for (int k = 0; k < REG_BITS; ++k) want[c[k].second] = true;
@@ -1276,7 +1283,7 @@ int build_pass(const std::vector<Gate>& G, const Step& st, uint32_t n, PassParam
         }
         // register positions by next use: the last register bit goes to the
         // tile bit needed last (the complex64 pass pairs amplitudes along it)
-        auto key = [&](uint8_t x) { return x == pin ? (1 << 30) + 1 : (x == must ? -1 : next_use(i, x)); };
+        auto key = [&](uint8_t x) { return x == pin ? (1 << 30) + 1 : (x == must || x == must2 ? -1 : next_use(i, x)); };
         std::stable_sort(nm.reg, nm.reg + REG_BITS, [&](uint8_t x, uint8_t y) { return key(x) < key(y); });
         if (!getenv("QOA_NO_ORDER_LANES")) order_lanes(nm);
         return exchange_to(nm);
@@ -1362,6 +1369,33 @@ int build_pass(const std::vector<Gate>& G, const Step& st, uint32_t n, PassParam
         if (g.kind == K_SWAP) {
             if (g.cmask || tbit(g.t) < 0 || tbit(g.t2) < 0) return -1;
             relabel(tb_of, g);
+            continue;
+        }
+        if (g.kind == K_U2) {
+            const int tl = tbit(g.t), th = tbit(g.t2);
+            auto reg_of = [&](int t) {
+                for (int j = 0; j < REG_BITS; ++j)
+                    if (m.reg[j] == t) return j;
+                return -1;
+            };
+            if (tl < 0 || th < 0) return -1;
+            if ((reg_of(tl) < 0 || reg_of(th) < 0) && !make_reg(i, tl, th)) return -1;
+            const int kl = reg_of(tl), kh = reg_of(th);
+            const uint32_t touch = (1u << kl) | (1u << kh);
+            if ((tab_bits & touch) && !flush_tab()) return -1;
+            if ((mx_bits & touch) && !flush_mx()) return -1;
+            if ((ang_reg_bits & touch) && !flush_ang_reg(ang_reg_bits & touch)) return -1;
+            PassOp* o = new_op();
+            if (!o || ncoef + 16 > MAX_PASS_COEF) return -1;
+            const int a = std::min(kl, kh), b = std::max(kl, kh);
+            P.has_u2 = 1;
+            o->code = (uint8_t)(PC_U2 + (a == 0 ? b - 1 : a == 1 ? b + 1 : 5));
+            o->coef = (uint16_t)ncoef;
+            // basis 2 * bit(b) + bit(a): rows and columns 1, 2 change places where the qubits' order is the other
+            static const int ord[2][4] = {{0, 1, 2, 3}, {0, 2, 1, 3}};
+            const int* p = ord[kl > kh];
+            for (int r = 0; r < 4; ++r)
+                for (int c = 0; c < 4; ++c) P.coef[ncoef++] = g.m[4 * p[r] + p[c]];
             continue;
         }
         if (g.kind == K_G1) {
@@ -2258,6 +2292,40 @@ void merge_swap_blocks(std::vector<Gate>& G) {
     G.swap(out);
 }
 
+// Controlled SWAPs as CNOT, Toffoli, CNOT, which tile passes take: the
+// controlled kernel is a sweep of the state by itself and splits the passes
+// around it.
+void split_controlled_swaps(std::vector<Gate>& G) {
+    size_t extra = 0;
+    for (const Gate& g : G) extra += g.kind == K_SWAP && g.cmask ? 2 : 0;
+    if (!extra) return;
+    std::vector<Gate> out;
+    out.reserve(G.size() + extra);
+    auto x = [&](const Gate& g, int t, uint64_t cm) {
+        Gate o;
+        o.kind = K_G1;
+        o.sub = G1_X;
+        o.t = t;
+        o.cmask = cm;
+        o.m[0] = o.m[3] = d2(0, 0);
+        o.m[1] = o.m[2] = d2(1, 0);
+        o.nmask = 1ull << t;
+        o.dmask = cm;
+        o.src = g.src;
+        out.push_back(o);
+    };
+    for (const Gate& g : G) {
+        if (g.kind != K_SWAP || !g.cmask) {
+            out.push_back(g);
+            continue;
+        }
+        x(g, g.t2, 1ull << g.t);
+        x(g, g.t, g.cmask | (1ull << g.t2));
+        x(g, g.t2, 1ull << g.t);
+    }
+    G.swap(out);
+}
+
 int run_perm(qoa_state_t s, const Gate& g) {
     const uint32_t n = s->n;
     PermParams P;
@@ -2356,7 +2424,10 @@ int run_small_list(qoa_state_t s, const std::vector<Gate>& seg, bool& reset_owed
 int run_planned(qoa_state_t s, std::vector<Gate>& seg, bool& reset_owed) {
     const bool c64 = s->precision == QOA_PREC_F32;
     const bool per_gate = (s->flags & QOA_FLAG_PER_GATE) != 0;
-    if (!per_gate) merge_swap_blocks(seg);
+    if (!per_gate) {
+        merge_swap_blocks(seg);
+        split_controlled_swaps(seg);
+    }
     const bool jit = !per_gate && s->jit_mode != QOA_JIT_OFF && s->n >= s->jit_min_qubits;
     // a repeated op list reuses its plan
     PlanEntry local;
@@ -2380,7 +2451,7 @@ int run_planned(qoa_state_t s, std::vector<Gate>& seg, bool& reset_owed) {
         // the plan depends on the op list and the size only, so a list
         // executed again gives bit-identical results
         pe->steps = schedule(seg, s->n, per_gate, false, state_pass_budget(s),
-                             slot_search_pays(s->n) || (s->flags & QOA_FLAG_SLOT_SEARCH));
+                             slot_search_pays(s->n) || (s->flags & QOA_FLAG_SLOT_SEARCH), !c64);
         pe->built_of.assign(pe->steps.size(), -1);
         // passes built ahead: for generated kernels, whose text is
         // requested from the compile cache, and for a plan that is kept
@@ -2609,7 +2680,7 @@ struct qoa_batch_s {
     // one launch of a generated arena kernel: njobs jobs of one structure
     // from job_off, 2^lt tiles each
     struct Group { uint32_t job_off, njobs, lt; int kernel; int stream; };
-    struct Round { uint32_t job_off, njobs, tiles; int max_nops, max_ncoef; std::vector<Group> groups; };
+    struct Round { uint32_t job_off, njobs, tiles; int max_nops, max_ncoef; std::vector<Group> groups; bool any_u2 = false; };
     std::vector<Round> rounds;
     std::vector<JitKernel> jit_kernels;  // by structure
     // a round's generated launches spread over stream 0 and these
@@ -2887,8 +2958,9 @@ int batch_prepare(qoa_batch_t b) {
             if (!is_small[i] && b->circs[i].n >= (uint32_t)TILE_BITS && !b->circs[i].gates.empty()) cands.push_back(i);
         parallel_for(cands.size(), [&](size_t x) {
             const size_t i = cands[x];
-            const auto& c = b->circs[i];
-            steps_of[i] = schedule(c.gates, c.n, false, false, budget);
+            auto& c = b->circs[i];
+            split_controlled_swaps(c.gates);
+            steps_of[i] = schedule(c.gates, c.n, false, false, budget, false, !f32);
             bool ok = true;
             for (const Step& st : steps_of[i]) ok = ok && st.pass;
             all_pass[i] = ok;
@@ -3120,6 +3192,7 @@ int batch_prepare(qoa_batch_t b) {
             if (!tensor) {
                 R.max_nops = std::max(R.max_nops, (int)p64[pi].nops);
                 R.max_ncoef = std::max(R.max_ncoef, (int)p64[pi].ncoef);
+                R.any_u2 = R.any_u2 || p64[pi].has_u2;
             }
         }
         if (R.groups.size() > 1) {
@@ -3278,7 +3351,7 @@ int batch_enqueue(qoa_batch_t b) {
                                       R.max_nops, R.max_ncoef, s0));
         else
             BCK(launch_pass_arena(b->d_jobs + R.job_off, R.njobs, b->d_tstart + R.job_off, R.tiles,
-                                  R.max_nops, R.max_ncoef, s0));
+                                  R.max_nops, R.max_ncoef, R.any_u2, s0));
     }
     for (uint32_t i = 1; i < ns; ++i) {
         BCK(cudaEventRecord(b->events[i], b->streams[i]));

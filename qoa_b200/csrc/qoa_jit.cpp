@@ -466,6 +466,9 @@ const TileMap* emit_ops128(Emit& E, const PassParams& P, bool arena, const char*
             E.line("g1r<%s, %d>(a, %s + %u);", g1_name(code), code & 3, cf, c);
         } else if (code >= PC_RXB && code < PC_DIAG_TA) {
             E.line("g1r<%s, %d>(a, %s + %u);", g1_name(code), code & 3, cf, c);
+        } else if (code >= PC_U2 && code < PC_U2 + 6) {
+            static const int lo[6] = {0, 0, 0, 1, 1, 2}, hi[6] = {1, 2, 3, 2, 3, 3};
+            E.line("g2r<%d, %d>(a, %s + %u);", lo[code - PC_U2], hi[code - PC_U2], cf, c);
         } else if (code >= PC_XC && code < PC_RXB) {
             E.line("g1rc<%s, %d>(a, %s, 0x%xu);", (code & ~3) == PC_XC ? "G1_X" : "G1_Y", code & 3,
                    tcond(tm).c_str(), cr);

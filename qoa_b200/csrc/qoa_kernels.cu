@@ -35,7 +35,10 @@ __device__ __forceinline__ uint64_t tstride(const PassParams& P, uint32_t t) {
 // null, receives the tile's squared norm after the pass. The pass's
 // coefficients are built in FP64 on the host; a complex64 pass rounds them
 // once when it stages them.
-template <typename T>
+// U2: whether the op stream may hold 4x4 gates (PassParams::has_u2). They have a
+// kernel of their own because they spill: in the one kernel they cost every
+// pass 13 % (arena rounds of a batch 3350 against 3794 us).
+template <bool U2, typename T>
 __device__ __forceinline__ void pass_tile(T* __restrict__ amps, const PassParams& P, const double nrm,
                                           const uint64_t blk, double* __restrict__ partial_out) {
     using R = typename CT<T>::R;
@@ -128,6 +131,12 @@ __device__ __forceinline__ void pass_tile(T* __restrict__ amps, const PassParams
             QOA_K4(PC_XC, bool tp; const uint32_t cr = conds(tp); g1rc<G1_X, K>(a, tp, cr))
             QOA_K4(PC_YC, bool tp; const uint32_t cr = conds(tp); g1rc<G1_Y, K>(a, tp, cr))
 #undef QOA_K4
+            case PC_U2 + 0: if constexpr (U2) g2r<0, 1, true>(a, m); break;
+            case PC_U2 + 1: if constexpr (U2) g2r<0, 2, true>(a, m); break;
+            case PC_U2 + 2: if constexpr (U2) g2r<0, 3, true>(a, m); break;
+            case PC_U2 + 3: if constexpr (U2) g2r<1, 2, true>(a, m); break;
+            case PC_U2 + 4: if constexpr (U2) g2r<1, 3, true>(a, m); break;
+            case PC_U2 + 5: if constexpr (U2) g2r<2, 3, true>(a, m); break;
             case PC_DIAG_T: {
                 bool tp;
                 conds(tp);
@@ -284,11 +293,11 @@ __device__ __forceinline__ void pass_tile(T* __restrict__ amps, const PassParams
 #endif
 template <typename T> struct PassOcc { static constexpr int value = QOA_PASS_OCC64; };
 
-template <typename T>
+template <typename T, bool U2>
 __global__ void __launch_bounds__(PASS_THREADS, PassOcc<T>::value)
 k_pass(T* __restrict__ amps, const __grid_constant__ PassParams P, const double* __restrict__ norm2_in,
        double* __restrict__ partials) {
-    pass_tile<T>(amps, P, *norm2_in, blockIdx.x, partials ? partials + blockIdx.x : nullptr);
+    pass_tile<U2, T>(amps, P, *norm2_in, blockIdx.x, partials ? partials + blockIdx.x : nullptr);
 }
 
 // Arena pass: one launch runs one pass of each of many circuits, whose states
@@ -296,7 +305,7 @@ k_pass(T* __restrict__ amps, const __grid_constant__ PassParams P, const double*
 // j is the last job with tile_start[j] <= b. Squared norms are not tracked: a
 // batched circuit is unitary, its start |0..0> is synthesised by its first
 // pass, and its consumers normalise.
-template <typename T>
+template <typename T, bool U2>
 __global__ void __launch_bounds__(PASS_THREADS, PassOcc<T>::value)
 k_pass_arena(const ArenaJob* __restrict__ jobs, uint32_t njobs, const uint32_t* __restrict__ tile_start) {
     const uint32_t b = blockIdx.x;
@@ -307,7 +316,7 @@ k_pass_arena(const ArenaJob* __restrict__ jobs, uint32_t njobs, const uint32_t* 
         else hi = mid - 1;
     }
     const ArenaJob J = jobs[lo];
-    pass_tile<T>(reinterpret_cast<T*>(J.amps), *reinterpret_cast<const PassParams*>(J.params),
+    pass_tile<U2, T>(reinterpret_cast<T*>(J.amps), *reinterpret_cast<const PassParams*>(J.params),
                  J.fresh ? 0.0 : 1.0, b - tile_start[lo], nullptr);
 }
 
@@ -685,33 +694,41 @@ static int grid_for(uint64_t work, int threads, int max_blocks) {
     return (int)b;
 }
 
-template <typename T>
-static cudaError_t launch_pass_t(T* amps, const PassParams& P, const double* norm2_in, double* partials,
+template <bool U2>
+static cudaError_t launch_pass_u(double2* amps, const PassParams& P, const double* norm2_in, double* partials,
                                  cudaStream_t st) {
-    const int tile_bytes = (1 << TILE_BITS) * (int)sizeof(T);
-    const int smem = tile_bytes + (int)P.nops * 16 + (int)P.ncoef * (int)sizeof(T);
-    cudaError_t e = cudaFuncSetAttribute(k_pass<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         tile_bytes + MAX_PASS_OPS * 16 + MAX_PASS_COEF * (int)sizeof(T));
+    const int tile_bytes = (1 << TILE_BITS) * (int)sizeof(double2);
+    const int smem = tile_bytes + (int)P.nops * 16 + (int)P.ncoef * (int)sizeof(double2);
+    cudaError_t e = cudaFuncSetAttribute(k_pass<double2, U2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         tile_bytes + MAX_PASS_OPS * 16 + MAX_PASS_COEF * (int)sizeof(double2));
     if (e != cudaSuccess) return e;
     const unsigned blocks = 1u << (P.n - TILE_BITS);
-    k_pass<T><<<blocks, PASS_THREADS, smem, st>>>(amps, P, norm2_in, partials);
+    k_pass<double2, U2><<<blocks, PASS_THREADS, smem, st>>>(amps, P, norm2_in, partials);
     return cudaGetLastError();
 }
 cudaError_t launch_pass(double2* amps, const PassParams& P, const double* norm2_in, double* partials,
                         cudaStream_t st) {
-    return launch_pass_t<double2>(amps, P, norm2_in, partials, st);
+    return P.has_u2 ? launch_pass_u<true>(amps, P, norm2_in, partials, st)
+                    : launch_pass_u<false>(amps, P, norm2_in, partials, st);
 }
-cudaError_t launch_pass_arena(const ArenaJob* jobs, uint32_t njobs, const uint32_t* tile_start, uint32_t tiles,
-                              int max_nops, int max_ncoef, cudaStream_t st) {
-    if (!njobs || !tiles) return cudaSuccess;
+template <bool U2>
+static cudaError_t launch_pass_arena_u(const ArenaJob* jobs, uint32_t njobs, const uint32_t* tile_start, uint32_t tiles,
+                                       int max_nops, int max_ncoef, cudaStream_t st) {
     const int esz = (int)sizeof(double2);
     const int tile_bytes = (1 << TILE_BITS) * esz;
     const int smem = tile_bytes + max_nops * 16 + max_ncoef * esz;
     const int smax = tile_bytes + MAX_PASS_OPS * 16 + MAX_PASS_COEF * esz;
-    cudaError_t e = cudaFuncSetAttribute(k_pass_arena<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax);
+    cudaError_t e = cudaFuncSetAttribute(k_pass_arena<double2, U2>, cudaFuncAttributeMaxDynamicSharedMemorySize, smax);
     if (e != cudaSuccess) return e;
-    k_pass_arena<double2><<<tiles, PASS_THREADS, smem, st>>>(jobs, njobs, tile_start);
+    k_pass_arena<double2, U2><<<tiles, PASS_THREADS, smem, st>>>(jobs, njobs, tile_start);
     return cudaGetLastError();
+}
+// any_u2: some job's pass has 4x4 gates
+cudaError_t launch_pass_arena(const ArenaJob* jobs, uint32_t njobs, const uint32_t* tile_start, uint32_t tiles,
+                              int max_nops, int max_ncoef, bool any_u2, cudaStream_t st) {
+    if (!njobs || !tiles) return cudaSuccess;
+    return any_u2 ? launch_pass_arena_u<true>(jobs, njobs, tile_start, tiles, max_nops, max_ncoef, st)
+                  : launch_pass_arena_u<false>(jobs, njobs, tile_start, tiles, max_nops, max_ncoef, st);
 }
 template <typename T>
 static cudaError_t launch_gate_t(T* a, uint64_t len, const GGate& g, cudaStream_t st) {

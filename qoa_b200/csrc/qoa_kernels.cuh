@@ -83,7 +83,8 @@ enum PassCode : uint8_t {
     PC_RYB = 36,      // +k (PC_RY carries the A form)
     PC_DIAG_TA = 40,  // pending factor *= angle phase `coef` where the thread condition holds
     PC_DIAG_MA = 41,  // registers with (v & cond_reg) == cond_reg *= angle phase `coef`
-    PC_NCODES = 42,
+    PC_U2 = 42,       // + register-bit pair (01, 02, 03, 12, 13, 23): 4x4, coef[c..c+15] row-major (complex128 passes)
+    PC_NCODES = 48,
 };
 
 // One op of a pass (16 bytes). The first 32-bit word (code, k, coef) is all
@@ -119,7 +120,7 @@ struct PassParams {
     uint32_t n;                       // qubits
     uint32_t nops;
     uint32_t ncoef;
-    uint32_t pad_;
+    uint32_t has_u2;                  // 1: some op is PC_U2 + k
     double2 phase;                    // product of the scalars factored out of this pass's gates
     uint8_t slot_qubit[HIGH_SLOTS];   // global qubit of each high slot (at load)
     uint8_t out_qubit[TILE_BITS];     // global qubit each tile bit is stored to (SWAPs relabel tile bits)

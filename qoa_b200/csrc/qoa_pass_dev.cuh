@@ -121,6 +121,30 @@ __device__ __forceinline__ void g1rc(T (&a)[REGS], bool tp, uint32_t creg) {
         if (!(v & (1 << K)) && (v & creg) == creg) g1_pair<SUB>(a[v], a[v | (1 << K)], z, z, z, z);
 }
 
+// 4x4 on register bits L < H, basis 2 * bit(H) + bit(L), matrix row-major.
+// REREAD: each coefficient is read again for every group of four (from shared
+// memory), where holding all 16 would spill (the interpreter).
+template <int L, int H, bool REREAD = false, typename T>
+__device__ __forceinline__ void g2r(T (&a)[REGS], const T* __restrict__ m) {
+#pragma unroll
+    for (int v = 0; v < REGS; ++v) {
+        if (v & ((1 << L) | (1 << H))) continue;
+        const T x[4] = {a[v], a[v | (1 << L)], a[v | (1 << H)], a[v | (1 << L) | (1 << H)]};
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            T s = c_mul(m[4 * r], x[0]);
+#pragma unroll
+            for (int k = 1; k < 4; ++k) {
+                const T c = m[4 * r + k];
+                s.x = fma(c.x, x[k].x, s.x); s.x = fma(-c.y, x[k].y, s.x);
+                s.y = fma(c.x, x[k].y, s.y); s.y = fma(c.y, x[k].x, s.y);
+                if (REREAD) asm volatile("" ::: "memory");
+            }
+            a[v | ((r & 1) << L) | ((r >> 1) << H)] = s;
+        }
+    }
+}
+
 template <typename T>
 __device__ __forceinline__ void diag_m(T (&a)[REGS], bool tp, uint32_t creg, T d) {
     if (!tp) return;
