@@ -2636,6 +2636,10 @@ inline bool shim_bit_ok(size_t b) { return b < 64; }
 // everything into a CUDA graph; later runs replay it.
 enum BatchRoute { R_SMALL = 0, R_ARENA = 1, R_VIEW = 2 };
 constexpr int kRoundStreams = 4;  // extra streams of a round's generated launches
+// What a structure must serve in a batch to be compiled in the default mode.
+// 1024 tiles are 2^21 amplitudes: a generated pass over them saves ~25 us a run.
+constexpr uint32_t kJitMinJobs = 8;
+constexpr uint64_t kJitMinTiles = 1024;
 
 struct qoa_batch_s {
     int precision = QOA_PREC_F64;
@@ -2680,7 +2684,9 @@ struct qoa_batch_s {
     // one launch of a generated arena kernel: njobs jobs of one structure
     // from job_off, 2^lt tiles each
     struct Group { uint32_t job_off, njobs, lt; int kernel; int stream; };
-    struct Round { uint32_t job_off, njobs, tiles; int max_nops, max_ncoef; std::vector<Group> groups; bool any_u2 = false; };
+    struct Round { uint32_t job_off, njobs, tiles; int max_nops, max_ncoef; std::vector<Group> groups; bool any_u2 = false;
+                   // jobs without a generated kernel of their own, the round's first ones (0 where there are no groups)
+                   uint32_t left_jobs = 0, left_tiles = 0; };
     std::vector<Round> rounds;
     std::vector<JitKernel> jit_kernels;  // by structure
     // a round's generated launches spread over stream 0 and these
@@ -3149,11 +3155,29 @@ int batch_prepare(qoa_batch_t b) {
                 }
                 shape_of[pi] = found;
             }
-        // in the default mode a structure must serve at least 8 passes of
-        // the batch to be worth its compile (~0.3 s of host time)
-        size_t npass = 0;
-        for (auto& v : pass_idx) npass += v.size();
-        if (b->tune.jit == QOA_JIT_ASYNC && reps.size() * 8 > npass) jit = false;
+        // in the default mode a structure must serve at least kJitMinJobs
+        // passes of the batch, or kJitMinTiles tiles, to be worth its compile
+        // (~0.3 s of one host core); the others stay on the interpreter,
+        // beside the generated launches
+        if (b->tune.jit == QOA_JIT_ASYNC) {
+            std::vector<uint32_t> uses(reps.size(), 0), kept;
+            std::vector<uint64_t> tiles(reps.size(), 0);
+            for (auto& v : pass_idx)
+                for (uint32_t pi : v) {
+                    uses[shape_of[pi]]++;
+                    tiles[shape_of[pi]] += 1ull << (p64[pi].n - TILE_BITS);
+                }
+            std::vector<int> id(reps.size(), -1);
+            for (size_t k = 0; k < reps.size(); ++k)
+                if (uses[k] >= kJitMinJobs || tiles[k] >= kJitMinTiles) {
+                    id[k] = (int)kept.size();
+                    kept.push_back(reps[k]);
+                }
+            for (int& sid : shape_of)
+                if (sid >= 0) sid = id[sid];
+            reps.swap(kept);
+            jit = !reps.empty();
+        }
     }
     if (jit) {
         std::vector<std::string> bodies(reps.size());
@@ -3174,7 +3198,8 @@ int batch_prepare(qoa_batch_t b) {
         for (size_t i : order) {
             const auto& c = b->circs[i];
             const uint32_t pi = pass_idx[i][r];
-            if (jit) {
+            if (jit && shape_of[pi] < 0) R.left_jobs++;  // (first in order)
+            if (jit && shape_of[pi] >= 0) {
                 if (R.groups.empty() || R.groups.back().kernel != shape_of[pi])
                     R.groups.push_back({(uint32_t)jobs.size(), 0, c.n - (uint32_t)TILE_BITS, shape_of[pi], 0});
                 R.groups.back().njobs++;
@@ -3193,15 +3218,17 @@ int batch_prepare(qoa_batch_t b) {
                 R.max_nops = std::max(R.max_nops, (int)p64[pi].nops);
                 R.max_ncoef = std::max(R.max_ncoef, (int)p64[pi].ncoef);
                 R.any_u2 = R.any_u2 || p64[pi].has_u2;
+                if (shape_of[pi] < 0) R.left_tiles += 1u << (c.n - TILE_BITS);
             }
         }
-        if (R.groups.size() > 1) {
+        if (!R.groups.empty() && R.groups.size() + (R.left_jobs ? 1 : 0) > 1) {
             // longest-processing-time-first over 1 + kRoundStreams streams
             std::vector<size_t> idx(R.groups.size());
             for (size_t g = 0; g < idx.size(); ++g) idx[g] = g;
             auto work = [&](size_t g) { return (double)R.groups[g].njobs * std::ldexp(1.0, (int)R.groups[g].lt); };
             std::sort(idx.begin(), idx.end(), [&](size_t x, size_t y) { return work(x) > work(y); });
-            double load[1 + kRoundStreams] = {};
+            // (the interpreter's share runs on stream 0, at about half the rate)
+            double load[1 + kRoundStreams] = {2.0 * R.left_tiles};
             for (size_t g : idx) {
                 int best = 0;
                 for (int k = 1; k <= kRoundStreams; ++k)
@@ -3324,34 +3351,37 @@ int batch_enqueue(qoa_batch_t b) {
     bool all_ready = !b->jit_kernels.empty();
     for (const auto& k : b->jit_kernels) all_ready = all_ready && k.ready();
     for (const auto& R : b->rounds) {
-        if (all_ready && !R.groups.empty()) {
-            const bool fork = R.groups.size() > 1 && !b->rstreams.empty();
-            if (fork) {
-                BCK(cudaEventRecord(b->revents[0], s0));
-                for (cudaStream_t st : b->rstreams) BCK(cudaStreamWaitEvent(st, b->revents[0], 0));
-            }
-            for (const auto& Gp : R.groups) {
-                cudaStream_t st = (fork && Gp.stream > 0) ? b->rstreams[Gp.stream - 1] : s0;
-                BCK(b->jit_kernels[Gp.kernel].launch_arena(b->d_jobs + Gp.job_off, Gp.njobs, Gp.lt, st));
-            }
-            if (fork)
-                for (size_t k = 0; k < b->rstreams.size(); ++k) {
-                    BCK(cudaEventRecord(b->revents[1 + k], b->rstreams[k]));
-                    BCK(cudaStreamWaitEvent(s0, b->revents[1 + k], 0));
-                }
+        // the interpreter's arena launch over the round's first njobs jobs
+        auto interpret = [&](uint32_t njobs, uint32_t tiles) -> cudaError_t {
+            const ArenaJob* jobs = b->d_jobs + R.job_off;
+            const uint32_t* ts = b->d_tstart + R.job_off;
+            if (tensor)
+                return launch_f32_pass_arena(jobs, njobs, ts, tiles, (const float*)(fb + b->f32_off[0]),
+                                             (const F32PhaseOp*)(fb + b->f32_off[1]), (const F32Angle*)(fb + b->f32_off[2]),
+                                             (const F32Phase*)(fb + b->f32_off[3]), (const float2*)(fb + b->f32_off[4]),
+                                             b->d_counter + 1, s0);
+            if (f32) return launch_pass_p32_arena(jobs, njobs, ts, tiles, R.max_nops, R.max_ncoef, s0);
+            return launch_pass_arena(jobs, njobs, ts, tiles, R.max_nops, R.max_ncoef, R.any_u2, s0);
+        };
+        if (!all_ready || R.groups.empty()) {
+            BCK(interpret(R.njobs, R.tiles));
             continue;
         }
-        if (tensor)
-            BCK(launch_f32_pass_arena(b->d_jobs + R.job_off, R.njobs, b->d_tstart + R.job_off, R.tiles,
-                                      (const float*)(fb + b->f32_off[0]), (const F32PhaseOp*)(fb + b->f32_off[1]),
-                                      (const F32Angle*)(fb + b->f32_off[2]), (const F32Phase*)(fb + b->f32_off[3]),
-                                      (const float2*)(fb + b->f32_off[4]), b->d_counter + 1, s0));
-        else if (f32)
-            BCK(launch_pass_p32_arena(b->d_jobs + R.job_off, R.njobs, b->d_tstart + R.job_off, R.tiles,
-                                      R.max_nops, R.max_ncoef, s0));
-        else
-            BCK(launch_pass_arena(b->d_jobs + R.job_off, R.njobs, b->d_tstart + R.job_off, R.tiles,
-                                  R.max_nops, R.max_ncoef, R.any_u2, s0));
+        const bool fork = R.groups.size() + (R.left_jobs ? 1 : 0) > 1 && !b->rstreams.empty();
+        if (fork) {
+            BCK(cudaEventRecord(b->revents[0], s0));
+            for (cudaStream_t st : b->rstreams) BCK(cudaStreamWaitEvent(st, b->revents[0], 0));
+        }
+        for (const auto& Gp : R.groups) {
+            cudaStream_t st = (fork && Gp.stream > 0) ? b->rstreams[Gp.stream - 1] : s0;
+            BCK(b->jit_kernels[Gp.kernel].launch_arena(b->d_jobs + Gp.job_off, Gp.njobs, Gp.lt, st));
+        }
+        if (R.left_jobs) BCK(interpret(R.left_jobs, R.left_tiles));
+        if (fork)
+            for (size_t k = 0; k < b->rstreams.size(); ++k) {
+                BCK(cudaEventRecord(b->revents[1 + k], b->rstreams[k]));
+                BCK(cudaStreamWaitEvent(s0, b->revents[1 + k], 0));
+            }
     }
     for (uint32_t i = 1; i < ns; ++i) {
         BCK(cudaEventRecord(b->events[i], b->streams[i]));
