@@ -963,6 +963,26 @@ std::vector<Step> schedule(const std::vector<Gate>& G, uint32_t n, bool per_gate
     return best;
 }
 
+// A complex64 pass's coefficients as its kernels read them (coef32).
+void round_coef(PassParams& P) {
+    std::vector<float2> f(P.ncoef);
+    for (uint32_t i = 0; i < P.ncoef; ++i) {
+        f[i].x = (float)P.coef[i].x;
+        f[i].y = (float)P.coef[i].y;
+    }
+    for (uint32_t o = 0; o < P.nops; ++o) {
+        const PassOp& op = P.ops[o];
+        if (op.code == PC_DIAG_TAB)
+            for (int j = 0; j < REGS / 2; ++j) {
+                float2 &a = f[op.coef + j], &b = f[op.coef + j + REGS / 2];
+                std::swap(a.y, b.x);  // (x_j, y_j), (x_j+8, y_j+8) -> (x_j, x_j+8), (y_j, y_j+8)
+            }
+        if (op.code == PC_DIAG_MX || op.code == PC_DIAG_TM) o += op.k;
+    }
+    std::memset((void*)P.coef, 0, P.ncoef * sizeof(double2));
+    std::memcpy((void*)P.coef, f.data(), f.size() * sizeof(float2));
+}
+
 // Builds the kernel op stream of a pass. The tile's TILE_BITS index bits
 // (tile bit t < 5 = qubit t, tile bit 5 + s = high slot s) are assigned to
 // lane / register / warp roles; every 2x2 gate must act on a register bit, so
@@ -1500,6 +1520,7 @@ int build_pass(const std::vector<Gate>& G, const Step& st, uint32_t n, PassParam
     }
     P.nops = (uint32_t)nops;
     P.ncoef = (uint32_t)ncoef;
+    if (pair_pin) round_coef(P);
     return 0;
 }
 

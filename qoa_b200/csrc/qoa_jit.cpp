@@ -381,7 +381,8 @@ void emit_head(Emit& E, const PassParams& P, bool c64, bool arena) {
     E.line("typedef %s T;", T);
     E.line("__shared__ __align__(16) T tile[1 << TILE_BITS];");
     if (!arena) E.line("__shared__ double red[PASS_THREADS / 32];");
-    if (c64 || arena) E.line("__shared__ __align__(16) T scoef[%u];", P.ncoef ? P.ncoef : 1);
+    if (arena) E.line("__shared__ __align__(16) T scoef[%u];", P.ncoef ? P.ncoef : 1);
+    else if (c64) E.line("const float2* const scoef = coef32(P);");
     if (P.nang) E.line("__shared__ T sang[%u];", P.nang);
     E.line("const int lane = threadIdx.x & 31;");
     E.line("const int wid = threadIdx.x >> 5;");
@@ -414,9 +415,8 @@ void emit_head(Emit& E, const PassParams& P, bool c64, bool arena) {
         }
         E.line("const uint64_t g0 = %s;", g.c_str());
     }
-    if (c64)
-        E.line("for (uint32_t i = threadIdx.x; i < %uu; i += PASS_THREADS) scoef[i] = make_float2((float)P.coef[i].x, (float)P.coef[i].y);",
-               P.ncoef);
+    if (c64 && arena)
+        E.line("for (uint32_t i = threadIdx.x; i < %uu; i += PASS_THREADS) scoef[i] = coef32(P)[i];", P.ncoef);
     else if (arena)
         E.line("for (uint32_t i = threadIdx.x; i < %uu; i += PASS_THREADS) scoef[i] = P.coef[i];", P.ncoef);
     if (P.nang) E.line("pass_angles(P, blk, sang);");
@@ -758,12 +758,13 @@ std::string jit_pass_body(const PassParams& P, bool arena) {
 
 // The complex64 form: the packed FP32 tile pass of qoa_pass32.cu
 // (pass_tile_p32) for the same PassParams. Registers hold re[j] / im[j] =
-// packed (amplitude j, amplitude j + 8); coefficients are rounded to float
-// once per CTA into shared memory, as the interpreter stages them.
-// The op stream of a complex64 pass (packed FP32 registers re[8] / im[8],
-// coefficients in scoef, register tables in stab at tab_at[op]); returns
-// the mapping in force at its end.
-const TileMap* emit_ops64(Emit& E, const PassParams& P, bool arena, const std::vector<uint32_t>& tab_at) {
+// packed (amplitude j, amplitude j + 8). Coefficients (scoef) come straight
+// from the parameter's constant bank (a copy staged in shared memory cost a
+// load per use in passes bound by issue: 23-qubit energy evaluation 701 against
+// 512 us, 29-qubit QFT with its shots 13.2 against 10.7 ms), in the arena form
+// from a staged copy.
+// This emits the op stream and returns the mapping in force at its end.
+const TileMap* emit_ops64(Emit& E, const PassParams& P, bool arena) {
     // one pair-exchange layout for the whole pass, when every exchange keeps
     // the same pairing bit and one layout serves all of them
     Swizzle zp;
@@ -856,8 +857,7 @@ const TileMap* emit_ops64(Emit& E, const PassParams& P, bool arena, const std::v
                     // a pair whose two factors are exactly 1 is left alone
                     for (int j = 0; j < 8; ++j)
                         if (((tm >> j) | (tm >> (j + 8))) & 1)
-                            E.line("cmul2(re[%d], im[%d], stab[%u], stab[%u]);", j, j, 16 * tab_at[oi] + j,
-                                   16 * tab_at[oi] + 8 + j);
+                            E.line("cmul2(re[%d], im[%d], pkc(scoef[%u]), pkc(scoef[%u]));", j, j, c + j, c + 8 + j);
                     break;
                 case PC_FLUSH:
                     E.line("{ const u64p cr = bc(pend.x), ci = bc(pend.y);");
@@ -949,36 +949,13 @@ std::string jit_pass32_body_streamed(const PassParams& P) {
     E.line("extern __shared__ __align__(128) unsigned char qoa_dsm[];");
     E.line("__shared__ __align__(8) uint64_t mbar[2];");
     E.line("__shared__ double red[PASS_THREADS / 32];");
-    E.line("__shared__ __align__(16) T scoef[%u];", P.ncoef ? P.ncoef : 1);
+    E.line("const float2* const scoef = coef32(P);");
     if (P.nang) E.line("__shared__ T sang[%u];", P.nang);
     E.line("const int lane = threadIdx.x & 31;");
     E.line("const int wid = threadIdx.x >> 5;");
     E.line("const double nrm = *norm2_in;");
     E.line("const bool valid = nrm > 1e-12;");
     E.line("const uint64_t ntiles = 1ull << %d;", lt);
-    E.line("for (uint32_t i = threadIdx.x; i < %uu; i += PASS_THREADS) scoef[i] = make_float2((float)P.coef[i].x, (float)P.coef[i].y);",
-           P.ncoef);
-    std::vector<uint32_t> tab_at(P.nops, 0);
-    {
-        uint32_t ntab = 0;
-        for (uint32_t oi = 0; oi < P.nops; ++oi) {
-            const int code = P.ops[oi].code;
-            if (code == PC_DIAG_TAB) tab_at[oi] = ntab++;
-            if (code == PC_DIAG_MX || code == PC_DIAG_TM) oi += P.ops[oi].k;
-        }
-        if (ntab) {
-            E.line("__shared__ u64p stab[%u];", 16 * ntab);
-            for (uint32_t oi = 0; oi < P.nops; ++oi) {
-                const PassOp& op = P.ops[oi];
-                if (op.code == PC_DIAG_TAB) {
-                    const uint32_t t = tab_at[oi], c = op.coef;
-                    E.line("if (threadIdx.x < 8) { const int j = threadIdx.x; const double2 x = P.coef[%u + j], y = P.coef[%u + j];", c, c + 8);
-                    E.line("  stab[%u + j] = pk((float)x.x, (float)y.x); stab[%u + j] = pk((float)x.y, (float)y.y); }", 16 * t, 16 * t + 8);
-                }
-                if (op.code == PC_DIAG_MX || op.code == PC_DIAG_TM) oi += op.k;
-            }
-        }
-    }
     {
         std::string g = "0ull";
         char b[128];
@@ -1059,7 +1036,7 @@ std::string jit_pass32_body_streamed(const PassParams& P) {
     E.line("__syncthreads();");
     E.line("if (valid && wid == 0 && blk + gridDim.x < ntiles) issue(blk + gridDim.x, (int)((it + 1u) & 1u));");
 
-    const TileMap* cur = emit_ops64(E, P, false, tab_at);
+    const TileMap* cur = emit_ops64(E, P, false);
 
     {
         const TileMap& m = *cur;
@@ -1089,29 +1066,6 @@ std::string jit_pass32_body(const PassParams& P, bool arena) {
     if (!arena && stream_f32()) return jit_pass32_body_streamed(P);
     Emit E;
     emit_head(E, P, true, arena);
-    // register tables (PC_DIAG_TAB): staged once per CTA already packed as
-    // (factor j, factor j + 8) pairs, real parts then imaginary parts
-    std::vector<uint32_t> tab_at(P.nops, 0);
-    {
-        uint32_t ntab = 0;
-        for (uint32_t oi = 0; oi < P.nops; ++oi) {
-            const int code = P.ops[oi].code;
-            if (code == PC_DIAG_TAB) tab_at[oi] = ntab++;
-            if (code == PC_DIAG_MX || code == PC_DIAG_TM) oi += P.ops[oi].k;
-        }
-        if (ntab) {
-            E.line("__shared__ u64p stab[%u];", 16 * ntab);
-            for (uint32_t oi = 0; oi < P.nops; ++oi) {
-                const PassOp& op = P.ops[oi];
-                if (op.code == PC_DIAG_TAB) {
-                    const uint32_t t = tab_at[oi], c = op.coef;
-                    E.line("if (threadIdx.x < 8) { const int j = threadIdx.x; const double2 x = P.coef[%u + j], y = P.coef[%u + j];", c, c + 8);
-                    E.line("  stab[%u + j] = pk((float)x.x, (float)y.x); stab[%u + j] = pk((float)x.y, (float)y.y); }", 16 * t, 16 * t + 8);
-                }
-                if (op.code == PC_DIAG_MX || op.code == PC_DIAG_TM) oi += op.k;
-            }
-        }
-    }
     E.line("const bool valid = nrm > 1e-12;");
     E.line("float2 pend = valid ? make_float2((float)(P.phase.x / sqrt(nrm)), (float)(P.phase.y / sqrt(nrm)))");
     E.line("                    : make_float2((float)P.phase.x, (float)P.phase.y);");
@@ -1143,9 +1097,9 @@ std::string jit_pass32_body(const PassParams& P, bool arena) {
         E.line("}");
         E.line("}");
     }
-    E.line("__syncthreads();");
+    if (P.nang || arena) E.line("__syncthreads();");
 
-    const TileMap* cur = emit_ops64(E, P, arena, tab_at);
+    const TileMap* cur = emit_ops64(E, P, arena);
     {
         const TileMap& m = *cur;
         auto ostride = [&](int t) -> unsigned long long { return 1ull << P.out_qubit[t]; };

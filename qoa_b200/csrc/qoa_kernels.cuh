@@ -135,6 +135,15 @@ struct PassParams {
 };
 static_assert(sizeof(PassParams) <= 32000, "PassParams travels as a kernel parameter (32 KB limit)");
 
+// The coefficients of a complex64 pass: the host rounds them to float2 in
+// place (from the start of coef), so that the kernels read them as they are —
+// the generated ones straight from the parameter's constant bank. A
+// PC_DIAG_TAB table is stored as the packed pairs its products take: entries
+// 0..7 the real parts of factors (j, j + 8), entries 8..15 their imaginary parts.
+#if defined(__CUDACC__) || defined(__CUDACC_RTC__)
+__device__ __forceinline__ const float2* coef32(const PassParams& P) { return reinterpret_cast<const float2*>(P.coef); }
+#endif
+
 #ifndef __CUDACC_RTC__
 static_assert(offsetof(PassParams, ops) % 16 == 0 && offsetof(PassParams, coef) % 16 == 0,
               "the op stream and coefficients are staged with 16-byte loads");

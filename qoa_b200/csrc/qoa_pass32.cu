@@ -49,7 +49,7 @@ __device__ __forceinline__ void pass_tile_p32(float2* __restrict__ amps, const P
         const uint4* gops = reinterpret_cast<const uint4*>(P.ops);
         for (uint32_t i = threadIdx.x; i < nops; i += PASS_THREADS) sops[i] = gops[i];
         for (uint32_t i = threadIdx.x; i < P.ncoef; i += PASS_THREADS)
-            scoef[i] = make_float2((float)P.coef[i].x, (float)P.coef[i].y);
+            scoef[i] = coef32(P)[i];
     }
     __shared__ float2 sang[MAX_ANG_OPS];
     for (uint32_t ai = threadIdx.x; ai < P.nang; ai += PASS_THREADS) {
@@ -168,8 +168,8 @@ __device__ __forceinline__ void pass_tile_p32(float2* __restrict__ amps, const P
             case PC_DIAG_TAB:
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                    const float2 c0 = m[j], c1 = m[j + 8];
-                    cmul2(re[j], im[j], pk(c0.x, c1.x), pk(c0.y, c1.y));
+                    const float2 cr = m[j], ci = m[j + 8];
+                    cmul2(re[j], im[j], pk(cr.x, cr.y), pk(ci.x, ci.y));
                 }
                 break;
             case PC_DIAG_TM: {
@@ -317,7 +317,7 @@ __device__ __forceinline__ void pass_tile_p32x2(float2* __restrict__ amps, const
         const uint4* gops = reinterpret_cast<const uint4*>(P.ops);
         for (uint32_t i = threadIdx.x; i < nops; i += PASS_THREADS) sops[i] = gops[i];
         for (uint32_t i = threadIdx.x; i < P.ncoef; i += PASS_THREADS)
-            scoef[i] = make_float2((float)P.coef[i].x, (float)P.coef[i].y);
+            scoef[i] = coef32(P)[i];
     }
     __shared__ float2 sang[2][MAX_ANG_OPS];
     for (uint32_t x = threadIdx.x; x < 2 * P.nang; x += PASS_THREADS) {
@@ -440,8 +440,8 @@ __device__ __forceinline__ void pass_tile_p32x2(float2* __restrict__ amps, const
             case PC_DIAG_TAB:
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                    const float2 c0 = m[j], c1 = m[j + 8];
-                    const u64p cr = pk(c0.x, c1.x), ci = pk(c0.y, c1.y);
+                    const float2 t0 = m[j], t1 = m[j + 8];
+                    const u64p cr = pk(t0.x, t0.y), ci = pk(t1.x, t1.y);
                     cmul2(re[0][j], im[0][j], cr, ci);
                     cmul2(re[1][j], im[1][j], cr, ci);
                 }

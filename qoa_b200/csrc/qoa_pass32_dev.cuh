@@ -18,6 +18,7 @@ __device__ __forceinline__ u64p pk(float lo, float hi) {
 }
 __device__ __forceinline__ float lo(u64p a) { return __uint_as_float((unsigned)a); }
 __device__ __forceinline__ float hi(u64p a) { return __uint_as_float((unsigned)(a >> 32)); }
+__device__ __forceinline__ u64p pkc(float2 c) { return pk(c.x, c.y); }
 __device__ __forceinline__ u64p bc(float x) { return pk(x, x); }
 
 __device__ __forceinline__ u64p add2(u64p a, u64p b) {
