@@ -41,16 +41,18 @@ cudaError_t launch_pass(double2* amps, const PassParams& P, const double* norm2_
 cudaError_t launch_gate(double2* a, uint64_t len, const GGate& g, cudaStream_t st);
 cudaError_t launch_swapnet(void* a, bool c64, const PermParams& P, cudaStream_t st);
 int reduce_blocks(uint64_t len);
-cudaError_t launch_norm(const double2* a, uint64_t len, double* partials, double* out, uint32_t* status, cudaStream_t st);
-cudaError_t launch_p01(const double2* a, uint64_t len, uint32_t q, double* partials, double* out2, const double* norm2,
-                       cudaStream_t st);
+cudaError_t launch_norm(const void* a, bool f32, uint64_t len, double* partials, unsigned int* ticket, double* out,
+                        uint32_t* status, cudaStream_t st);
+cudaError_t launch_p01(const double2* a, uint64_t len, uint32_t q, double* partials, unsigned int* ticket, double* out2,
+                       const double* norm2, cudaStream_t st);
 uint32_t expz_blocks(uint64_t len);
 cudaError_t launch_expz(const void* a, bool f32, uint64_t len, const ExpzMasks& M, uint32_t k, const double* norm2,
                         double* partials, unsigned int* ticket, double* out, cudaStream_t st);
 cudaError_t launch_reduce_partials(const double* partials, uint32_t count, double* out, uint32_t* status, cudaStream_t st);
 cudaError_t launch_collapse(double2* a, uint64_t len, uint32_t q, uint32_t outcome, double f, double* partials,
-                            double* norm2_out, uint32_t* status, cudaStream_t st);
-cudaError_t launch_materialize(double2* a, uint64_t len, double* norm2, double* partials, uint32_t* status, cudaStream_t st);
+                            unsigned int* ticket, double* norm2_out, uint32_t* status, cudaStream_t st);
+cudaError_t launch_materialize(void* a, bool f32, uint64_t len, double* norm2, double* partials, unsigned int* ticket,
+                               uint32_t* status, cudaStream_t st);
 cudaError_t launch_set_scalar(double* p, double v, cudaStream_t st);
 cudaError_t launch_init_scalars(double* scal, uint32_t* status, cudaStream_t st);
 cudaError_t launch_probs(const double2* a, uint64_t off, uint64_t cnt, const double* norm2, double* out, cudaStream_t st);
@@ -63,10 +65,6 @@ cudaError_t launch_f32_pass(float2* amps, const F32PassParams& P, const float* m
                             const F32Angle* angles, const F32Phase* phases, const float2* tables,
                             const double* norm2_in, double* partials, uint32_t* status, cudaStream_t st);
 cudaError_t launch_f32_reset(float2* a, uint64_t len, cudaStream_t st);
-cudaError_t launch_f32_norm(const float2* a, uint64_t len, double* partials, double* out, uint32_t* status,
-                            cudaStream_t st);
-cudaError_t launch_f32_materialize(float2* a, uint64_t len, double* norm2, double* partials, uint32_t* status,
-                                   cudaStream_t st);
 cudaError_t launch_f32_probs(const float2* a, uint64_t off, uint64_t cnt, const double* norm2, double* out,
                              cudaStream_t st);
 cudaError_t launch_random_state(void* a, bool f32, uint64_t len, uint64_t seed, cudaStream_t st);
@@ -2204,8 +2202,8 @@ int run_small(qoa_state_t s, const SmallList& L, int in) {
 
 // Reads norm2, P0, P1 of qubit q (logical probabilities) to the host.
 int read_p01(qoa_state_t s, uint32_t q, double& p0, double& p1, double& norm2) {
-    CK(launch_p01(s->amps, state_len(s), q, s->partials, s->scal + 1, s->scal, s->stream));
-    s->launches += 2;
+    CK(launch_p01(s->amps, state_len(s), q, s->partials, ticket(s), s->scal + 1, s->scal, s->stream));
+    s->launches++;
     CK(cudaMemcpyAsync(s->host_scal, s->scal, 3 * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     norm2 = s->host_scal[0];
@@ -2253,9 +2251,9 @@ int do_measure(qoa_state_t s, uint32_t q, double u, uint32_t* outcome) {
         if (rc) return rc;
         norm2 = 1.0;
     }
-    CK(launch_collapse(s->amps, state_len(s), q, res, f / std::sqrt(norm2), s->partials, s->scal, s->status,
-                       s->stream));
-    s->launches += 2;
+    CK(launch_collapse(s->amps, state_len(s), q, res, f / std::sqrt(norm2), s->partials, ticket(s), s->scal,
+                       s->status, s->stream));
+    s->launches++;
     return QOA_OK;
 }
 
@@ -2267,8 +2265,8 @@ int do_reset_qubit(qoa_state_t s, uint32_t q) {
     if (!(norm2 > 1e-12)) return do_reset_all(s);
     if (p0 > 1e-12) {
         CK(launch_collapse(s->amps, state_len(s), q, 0, (1.0 / std::sqrt(p0)) / std::sqrt(norm2), s->partials,
-                           s->scal, s->status, s->stream));
-        s->launches += 2;
+                           ticket(s), s->scal, s->status, s->stream));
+        s->launches++;
         return QOA_OK;
     }
     return do_reset_all(s);
@@ -2659,6 +2657,7 @@ std::mutex g_shim_mu;
 double2* g_shim_buf = nullptr;
 size_t g_shim_cap = 0;
 double* g_shim_scr = nullptr;
+unsigned int* shim_ticket() { return reinterpret_cast<unsigned int*>(g_shim_scr + 7); }
 cudaStream_t g_shim_stream = nullptr;
 int g_shim_dev = -1;
 
@@ -2677,7 +2676,9 @@ int shim_begin(double* amps, size_t len, double2** dev) {
         if (g_shim_scr) cudaFree(g_shim_scr);
         g_shim_buf = nullptr; g_shim_scr = nullptr; g_shim_cap = 0;
         CK(cudaMalloc(&g_shim_buf, len * sizeof(double2)));
+        // results, the ticket word (0 between launches), then partial sums
         CK(cudaMalloc(&g_shim_scr, (size_t)(2 * reduce_blocks(len) + 8) * sizeof(double)));
+        CK(cudaMemsetAsync(g_shim_scr, 0, 8 * sizeof(double), g_shim_stream));
         g_shim_cap = len;
     }
     if (len) CK(cudaMemcpyAsync(g_shim_buf, amps, len * sizeof(double2), cudaMemcpyHostToDevice, g_shim_stream));
@@ -3737,11 +3738,9 @@ int qoa_get_state(qoa_state_t s, void* host, size_t bytes) {
     const size_t esz = s->precision == QOA_PREC_F32 ? sizeof(float2) : sizeof(double2);
     if (!host || bytes != state_len(s) * esz)
         return set_err(s, QOA_E_ARG, "get_state needs %llu bytes", (unsigned long long)(state_len(s) * esz));
-    if (s->precision == QOA_PREC_F32)
-        CK(launch_f32_materialize((float2*)s->amps, state_len(s), s->scal, s->partials, s->status, s->stream));
-    else
-        CK(launch_materialize(s->amps, state_len(s), s->scal, s->partials, s->status, s->stream));
-    s->launches += 2;
+    CK(launch_materialize(s->amps, s->precision == QOA_PREC_F32, state_len(s), s->scal, s->partials, ticket(s), s->status,
+                          s->stream));
+    s->launches++;
     CK(cudaMemcpyAsync(host, s->amps, bytes, cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     return QOA_OK;
@@ -3754,11 +3753,9 @@ int qoa_set_state(qoa_state_t s, const void* host, size_t bytes) {
     if (!host || bytes != state_len(s) * esz)
         return set_err(s, QOA_E_ARG, "set_state needs %llu bytes", (unsigned long long)(state_len(s) * esz));
     CK(cudaMemcpyAsync(s->amps, host, bytes, cudaMemcpyHostToDevice, s->stream));
-    if (s->precision == QOA_PREC_F32)
-        CK(launch_f32_norm((const float2*)s->amps, state_len(s), s->partials, s->scal, nullptr, s->stream));
-    else
-        CK(launch_norm(s->amps, state_len(s), s->partials, s->scal, nullptr, s->stream));
-    s->launches += 2;
+    CK(launch_norm(s->amps, s->precision == QOA_PREC_F32, state_len(s), s->partials, ticket(s), s->scal, nullptr,
+                   s->stream));
+    s->launches++;
     // set_state_vector normalises at once (quantum_state.rs:1143): a zero or
     // NaN vector becomes |0..0> before any gate sees it.
     CK(cudaMemcpyAsync(s->host_scal, s->scal, sizeof(double), cudaMemcpyDeviceToHost, s->stream));
@@ -3775,9 +3772,8 @@ int qoa_set_random_state(qoa_state_t s, uint64_t seed) {
     if (rc) return rc;
     const bool f32 = s->precision == QOA_PREC_F32;
     CK(launch_random_state(s->amps, f32, state_len(s), seed, s->stream));
-    if (f32) CK(launch_f32_norm((const float2*)s->amps, state_len(s), s->partials, s->scal, nullptr, s->stream));
-    else CK(launch_norm(s->amps, state_len(s), s->partials, s->scal, nullptr, s->stream));
-    s->launches += 3;
+    CK(launch_norm(s->amps, f32, state_len(s), s->partials, ticket(s), s->scal, nullptr, s->stream));
+    s->launches += 2;
     CK(cudaStreamSynchronize(s->stream));
     return QOA_OK;
 }
@@ -4522,13 +4518,13 @@ int qoa_vec_apply_reset(double* amps, size_t len, size_t bit) {
     int rc = shim_begin(amps, len, &dev);
     if (rc) return rc;
     if (len) {
-        CK(launch_p01(dev, len, (uint32_t)bit, g_shim_scr + 8, g_shim_scr, nullptr, g_shim_stream));
+        CK(launch_p01(dev, len, (uint32_t)bit, g_shim_scr + 8, shim_ticket(), g_shim_scr, nullptr, g_shim_stream));
         double p[2];
         CK(cudaMemcpyAsync(p, g_shim_scr, sizeof p, cudaMemcpyDeviceToHost, g_shim_stream));
         CK(cudaStreamSynchronize(g_shim_stream));
         if (p[0] > 1e-12) {
-            CK(launch_collapse(dev, len, (uint32_t)bit, 0, 1.0 / std::sqrt(p[0]), g_shim_scr + 8, g_shim_scr + 2,
-                               nullptr, g_shim_stream));
+            CK(launch_collapse(dev, len, (uint32_t)bit, 0, 1.0 / std::sqrt(p[0]), g_shim_scr + 8, shim_ticket(),
+                               g_shim_scr + 2, nullptr, g_shim_stream));
         } else {
             GGate k;
             memset(&k, 0, sizeof k);

@@ -407,38 +407,6 @@ __global__ void k_f32_reset(float2* a, uint64_t len) {
         a[i] = make_float2(i == 0 ? 1.f : 0.f, 0.f);
 }
 
-__global__ void k_f32_norm_partials(const float2* __restrict__ a, uint64_t len, double* __restrict__ partials) {
-    __shared__ double sh[32];
-    double v = 0.0;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += (uint64_t)gridDim.x * blockDim.x) {
-        const float2 x = a[i];
-        v += (double)x.x * x.x + (double)x.y * x.y;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int k = 0; k < (int)(blockDim.x >> 5); ++k) t += sh[k];
-        partials[blockIdx.x] = t;
-    }
-}
-
-__global__ void k_f32_materialize(float2* __restrict__ a, uint64_t len, const double* __restrict__ norm2_in) {
-    const double nrm = *norm2_in;
-    const bool valid = nrm > 1e-12;
-    const float s = valid ? (float)(1.0 / sqrt(nrm)) : 0.f;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += (uint64_t)gridDim.x * blockDim.x) {
-        if (valid) {
-            const float2 x = a[i];
-            a[i] = make_float2(x.x * s, x.y * s);
-        } else {
-            a[i] = make_float2(i == 0 ? 1.f : 0.f, 0.f);
-        }
-    }
-}
-
 __global__ void k_f32_probs(const float2* __restrict__ a, uint64_t off, uint64_t cnt, const double* __restrict__ norm2_in,
                             double* __restrict__ out) {
     const double nrm = *norm2_in;
@@ -454,10 +422,6 @@ __global__ void k_f32_probs(const float2* __restrict__ a, uint64_t off, uint64_t
     }
 }
 
-int reduce_blocks(uint64_t len);
-cudaError_t launch_reduce_partials(const double* partials, uint32_t count, double* out, uint32_t* status,
-                                   cudaStream_t st);
-
 static int f32_grid(uint64_t len) {
     uint64_t b = (len + 255) / 256;
     if (b > 148 * 16) b = 148 * 16;
@@ -467,17 +431,6 @@ static int f32_grid(uint64_t len) {
 cudaError_t launch_f32_reset(float2* a, uint64_t len, cudaStream_t st) {
     k_f32_reset<<<f32_grid(len), 256, 0, st>>>(a, len);
     return cudaGetLastError();
-}
-cudaError_t launch_f32_norm(const float2* a, uint64_t len, double* partials, double* out, uint32_t* status,
-                            cudaStream_t st) {
-    const int nb = reduce_blocks(len);
-    k_f32_norm_partials<<<nb, 256, 0, st>>>(a, len, partials);
-    return launch_reduce_partials(partials, (uint32_t)nb, out, status, st);
-}
-cudaError_t launch_f32_materialize(float2* a, uint64_t len, double* norm2, double* partials, uint32_t* status,
-                                   cudaStream_t st) {
-    k_f32_materialize<<<f32_grid(len), 256, 0, st>>>(a, len, norm2);
-    return launch_f32_norm(a, len, partials, norm2, status, st);
 }
 cudaError_t launch_f32_probs(const float2* a, uint64_t off, uint64_t cnt, const double* norm2, double* out,
                              cudaStream_t st) {

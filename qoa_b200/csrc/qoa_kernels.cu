@@ -568,15 +568,59 @@ __device__ __forceinline__ void block_store_partials(double (&v)[NB], double* __
     }
 }
 
-// sum |a|^2 (scaled by s^2) per block
-__global__ void k_norm_partials(const double2* __restrict__ a, uint64_t len, double* __restrict__ partials) {
+// True in the CTA that arrives last at the ticket (which returns to 0 by
+// itself), after every CTA's partial sums are visible to it.
+__device__ __forceinline__ bool last_block(unsigned int* ticket) {
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+// The sum of a set's per-CTA partials in a fixed order (all threads of one
+// CTA call it; thread 0 has the result).
+__device__ __forceinline__ double sum_partials(const double* partials) {
+    __shared__ double sh[32];
+    double x = 0.0;
+    for (uint32_t i = threadIdx.x; i < gridDim.x; i += blockDim.x) x += __ldcg(partials + i);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = x;
+    __syncthreads();
+    double t = 0.0;
+    if (threadIdx.x == 0)
+        for (uint32_t w = 0; w < (blockDim.x >> 5); ++w) t += sh[w];
+    return t;
+}
+// norm2 of a kernel's output, with its status bookkeeping
+__device__ __forceinline__ void finish_norm(const double* partials, unsigned int* ticket, double* norm2, uint32_t* status) {
+    if (!last_block(ticket)) return;
+    const double t = sum_partials(partials);
+    if (threadIdx.x == 0) {
+        *norm2 = t;
+        if (status) {
+            if (t != t) atomicOr(&status[0], 1u);
+            if (!(t > 1e-12)) atomicAdd(&status[2], 1u);
+        }
+    }
+}
+
+// sum |a|^2: partial sums per CTA, added by the last one
+template <typename T>
+__global__ void k_norm(const T* __restrict__ a, uint64_t len, double* __restrict__ partials, unsigned int* ticket,
+                       double* __restrict__ norm2, uint32_t* __restrict__ status) {
     double v[1] = {0.0};
     for (uint64_t i = gtid(); i < len; i += gstride()) v[0] += c_abs2(a[i]);
     block_store_partials<1>(v, partials, gridDim.x);
+    finish_norm(partials, ticket, norm2, status);
 }
 
-// P(bit q = 0), P(bit q = 1) of the stored vector (unscaled) per block
-__global__ void k_p01_partials(const double2* __restrict__ a, uint64_t len, uint32_t q, double* __restrict__ partials) {
+// P(bit q = 0), P(bit q = 1) of the stored vector, divided by norm2 (null: not divided)
+__global__ void k_p01(const double2* __restrict__ a, uint64_t len, uint32_t q, double* __restrict__ partials,
+                      unsigned int* ticket, const double* __restrict__ norm2, double* __restrict__ out) {
     double v[2] = {0.0, 0.0};
     const uint64_t m = 1ull << q;
     for (uint64_t i = gtid(); i < len; i += gstride()) {
@@ -585,6 +629,13 @@ __global__ void k_p01_partials(const double2* __restrict__ a, uint64_t len, uint
         else v[0] += p;
     }
     block_store_partials<2>(v, partials, gridDim.x);
+    if (!last_block(ticket)) return;
+    const double d = norm2 ? *norm2 : 1.0;
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+        const double t = sum_partials(partials + (uint64_t)s * gridDim.x);
+        if (threadIdx.x == 0) out[s] = d > 1e-12 ? t / d : 0.0;
+    }
 }
 
 // Final reduction: out[s] = sum_k partials[s*count + k] in a fixed order (one
@@ -625,9 +676,10 @@ __global__ void k_reduce(const double* __restrict__ partials, uint32_t count, do
 
 // Collapse for measure / reset_qubit: keep bit q == outcome scaled by `f`
 // (already including the pending 1/||psi||), zero the other branch, and leave
-// norm partials of the result.
+// the squared norm of the result.
 __global__ void k_collapse(double2* __restrict__ a, uint64_t len, uint32_t q, uint32_t outcome, double f,
-                           double* __restrict__ partials) {
+                           double* __restrict__ partials, unsigned int* ticket, double* __restrict__ norm2,
+                           uint32_t* __restrict__ status) {
     double v[1] = {0.0};
     const uint64_t m = 1ull << q;
     for (uint64_t i = gtid(); i < len; i += gstride()) {
@@ -642,27 +694,32 @@ __global__ void k_collapse(double2* __restrict__ a, uint64_t len, uint32_t q, ui
         v[0] += c_abs2(x);
     }
     block_store_partials<1>(v, partials, gridDim.x);
+    finish_norm(partials, ticket, norm2, status);
 }
 
-// Materialise the pending normalisation in place (or reset to |0..0>).
-__global__ void k_materialize(double2* __restrict__ a, uint64_t len, const double* __restrict__ norm2_in,
-                              double* __restrict__ partials) {
+// Materialise the pending normalisation in place (or reset to |0..0>). norm2
+// is read by every CTA before the last of them writes it.
+template <typename T>
+__global__ void k_materialize(T* __restrict__ a, uint64_t len, double* norm2, double* __restrict__ partials,
+                              unsigned int* ticket, uint32_t* __restrict__ status) {
+    using R = typename CT<T>::R;
     double v[1] = {0.0};
-    const double nrm = *norm2_in;
+    const double nrm = *reinterpret_cast<volatile double*>(norm2);
     const bool valid = nrm > 1e-12;
-    const double s = valid ? 1.0 / sqrt(nrm) : 0.0;
+    const R s = valid ? (R)(1.0 / sqrt(nrm)) : (R)0;
     for (uint64_t i = gtid(); i < len; i += gstride()) {
-        double2 x;
+        T x;
         if (valid) {
             x = a[i];
-            x = make_double2(x.x * s, x.y * s);
+            x = CT<T>::mk(x.x * s, x.y * s);
         } else {
-            x = make_double2(i == 0 ? 1.0 : 0.0, 0.0);
+            x = CT<T>::mk(i == 0 ? (R)1 : (R)0, (R)0);
         }
         a[i] = x;
         v[0] += c_abs2(x);
     }
     block_store_partials<1>(v, partials, gridDim.x);
+    finish_norm(partials, ticket, norm2, status);
 }
 
 __global__ void k_set_scalar(double* p, double v) { *p = v; }
@@ -764,19 +821,17 @@ cudaError_t launch_gate_c64(float2* a, uint64_t len, const GGate& g, cudaStream_
 // Partial-sum grid: fixed per length so that reductions are deterministic.
 int reduce_blocks(uint64_t len) { return grid_for(len, 256, 148 * 8); }
 
-cudaError_t launch_norm(const double2* a, uint64_t len, double* partials, double* out, uint32_t* status,
-                        cudaStream_t st) {
+cudaError_t launch_norm(const void* a, bool f32, uint64_t len, double* partials, unsigned int* ticket, double* out,
+                        uint32_t* status, cudaStream_t st) {
     const int nb = reduce_blocks(len);
-    k_norm_partials<<<nb, 256, 0, st>>>(a, len, partials);
-    k_reduce<<<1, 1024, 0, st>>>(partials, nb, out, nullptr, status);
+    if (f32) k_norm<<<nb, 256, 0, st>>>((const float2*)a, len, partials, ticket, out, status);
+    else k_norm<<<nb, 256, 0, st>>>((const double2*)a, len, partials, ticket, out, status);
     return cudaGetLastError();
 }
 
-cudaError_t launch_p01(const double2* a, uint64_t len, uint32_t q, double* partials, double* out2,
+cudaError_t launch_p01(const double2* a, uint64_t len, uint32_t q, double* partials, unsigned int* ticket, double* out2,
                        const double* norm2, cudaStream_t st) {
-    const int nb = reduce_blocks(len);
-    k_p01_partials<<<nb, 256, 0, st>>>(a, len, q, partials);
-    k_reduce<<<2, 1024, 0, st>>>(partials, nb, out2, norm2, nullptr);
+    k_p01<<<reduce_blocks(len), 256, 0, st>>>(a, len, q, partials, ticket, norm2, out2);
     return cudaGetLastError();
 }
 
@@ -792,18 +847,16 @@ cudaError_t launch_reduce_partials(const double* partials, uint32_t count, doubl
 }
 
 cudaError_t launch_collapse(double2* a, uint64_t len, uint32_t q, uint32_t outcome, double f, double* partials,
-                            double* norm2_out, uint32_t* status, cudaStream_t st) {
-    const int nb = reduce_blocks(len);
-    k_collapse<<<nb, 256, 0, st>>>(a, len, q, outcome, f, partials);
-    k_reduce<<<1, 1024, 0, st>>>(partials, nb, norm2_out, nullptr, status);
+                            unsigned int* ticket, double* norm2_out, uint32_t* status, cudaStream_t st) {
+    k_collapse<<<reduce_blocks(len), 256, 0, st>>>(a, len, q, outcome, f, partials, ticket, norm2_out, status);
     return cudaGetLastError();
 }
 
-cudaError_t launch_materialize(double2* a, uint64_t len, double* norm2, double* partials, uint32_t* status,
-                               cudaStream_t st) {
+cudaError_t launch_materialize(void* a, bool f32, uint64_t len, double* norm2, double* partials, unsigned int* ticket,
+                               uint32_t* status, cudaStream_t st) {
     const int nb = reduce_blocks(len);
-    k_materialize<<<nb, 256, 0, st>>>(a, len, norm2, partials);
-    k_reduce<<<1, 1024, 0, st>>>(partials, nb, norm2, nullptr, status);
+    if (f32) k_materialize<<<nb, 256, 0, st>>>((float2*)a, len, norm2, partials, ticket, status);
+    else k_materialize<<<nb, 256, 0, st>>>((double2*)a, len, norm2, partials, ticket, status);
     return cudaGetLastError();
 }
 

@@ -28,7 +28,6 @@ namespace qoa {
 namespace {
 
 constexpr uint32_t ROOT_BITS = 8;  // a warp's gather: 8 values a lane
-constexpr uint32_t FOLD_BITS = 6;  // 64 loads a thread
 
 // value j of a level: the amplitudes themselves, or a stored level
 template <typename T>
@@ -240,13 +239,16 @@ int fold_grid(uint32_t lo) {
 }  // namespace
 
 // The stored levels of an n-qubit state's tree, the largest first: n - 8
-// bits split evenly into steps of at most 6 (64 loads a thread; 8-bit steps
-// left too few threads on states of 12 to 20 qubits), the root step takes 8.
+// bits split evenly into steps, the root step takes 8. Steps of at most 4 bits
+// (16 loads a thread) up to 22 qubits, where 6-bit steps leave too few threads
+// (20 qubits: 26 + 10 us in two launches), of 6 above, where fewer launches
+// and 1/64 of the state of scratch count.
 SampleLevels sample_levels(uint32_t n) {
     SampleLevels L{};
+    const uint32_t step = n <= 22 ? 4 : 6;
     uint32_t rest = n > ROOT_BITS ? n - ROOT_BITS : 0, at = n;
     uint64_t off = 0;
-    for (uint32_t steps = (rest + FOLD_BITS - 1) / FOLD_BITS; steps; --steps) {
+    for (uint32_t steps = (rest + step - 1) / step; steps; --steps) {
         const uint32_t b = (rest + steps - 1) / steps;
         rest -= b;
         at -= b;
