@@ -39,6 +39,7 @@
 namespace qoa {
 cudaError_t launch_pass(double2* amps, const PassParams& P, const double* norm2_in, double* partials, cudaStream_t st);
 cudaError_t launch_gate(double2* a, uint64_t len, const GGate& g, cudaStream_t st);
+uint32_t swapnet_low(bool c64);
 cudaError_t launch_swapnet(void* a, bool c64, const PermParams& P, cudaStream_t st);
 int reduce_blocks(uint64_t len);
 cudaError_t launch_norm(const void* a, bool f32, uint64_t len, double* partials, unsigned int* ticket, double* out,
@@ -2428,7 +2429,7 @@ int run_perm(qoa_state_t s, const Gate& g) {
     memset(&P, 0, sizeof P);
     P.n = n;
     bool in_a[64] = {};
-    const uint32_t low = std::min<uint32_t>(LANE_BITS, n);
+    const uint32_t low = std::min<uint32_t>(swapnet_low(s->precision == QOA_PREC_F32), n);
     for (uint32_t q = 0; q < low; ++q) {
         P.tq[P.na++] = (uint8_t)q;
         in_a[q] = true;
@@ -2439,9 +2440,17 @@ int run_perm(qoa_state_t s, const Gate& g) {
                 P.tq[P.na++] = (uint8_t)q;
                 in_a[q] = true;
             }
+    // Tile numbers count a qubit and its partner in turn, lowest first, so that
+    // the tiles in flight lie next to each other in memory and so do their
+    // partner tiles (with plain ascending qubits every run of the partners was
+    // alone in its DRAM page).
     uint32_t no = 0;
     for (uint32_t q = 0; q < n; ++q)
-        if (!in_a[q]) P.oq[no++] = (uint8_t)q;
+        for (uint32_t x : {q, (uint32_t)g.pi[q]})
+            if (!in_a[x]) {
+                P.oq[no++] = (uint8_t)x;
+                in_a[x] = true;
+            }
     for (uint32_t q = 0; q < n; ++q) P.pi[q] = g.pi[q];
     for (uint32_t k = 0; k < P.na; ++k)
         for (uint32_t k2 = 0; k2 < P.na; ++k2)

@@ -418,8 +418,19 @@ __global__ void k_reset_all(T* __restrict__ a, uint64_t len) {
 // ------------------------------------------------------------ SWAP blocks
 // out[pi(i)] = in[i] for an involution pi of the qubits (disjoint SWAPs). The
 // norm is unchanged, so no partial sums are written.
+// Tile of a swap network: `low` lowest qubits and their partners; each access is
+// a run of 2^low amplitudes, 512 bytes in both precisions. What bounds it is
+// DRAM locality: a partner tile's runs are far apart, so the tiles in flight
+// have to be neighbours on both sides (the tile numbering of run_perm). Measured
+// on B200: 29 qubits complex64 2490 -> 1692 us (5.1 TB/s; 1777 with five
+// qubits), 28 qubits complex128 2235 -> 1555 us (5.5 TB/s). More resident CTAs
+// (6 or 8 an SM) did not help.
+template <typename T> struct SwapNet;
+template <> struct SwapNet<double2> { static constexpr int low = 5, tile = 1 << 10, threads = 256; };
+template <> struct SwapNet<float2> { static constexpr int low = 6, tile = 1 << 12, threads = 512; };
+
 template <typename T>
-__global__ void __launch_bounds__(256) k_swapnet(T* __restrict__ a, const __grid_constant__ PermParams P) {
+__global__ void __launch_bounds__(SwapNet<T>::threads) k_swapnet(T* __restrict__ a, const __grid_constant__ PermParams P) {
     extern __shared__ __align__(16) unsigned char sw_smem[];
     const uint32_t tn = 1u << P.na;
     T* s0 = reinterpret_cast<T*>(sw_smem);
@@ -478,9 +489,9 @@ __global__ void __launch_bounds__(256) k_swapnet(T* __restrict__ a, const __grid
         t_pb[c][x] = pb;
     }
     __syncthreads();
-    // shared-memory slot of tile index j: its low five bits XORed with the
-    // next five, so the permuted reads of a warp spread over the banks
-    auto sp = [](uint32_t j) { return j ^ ((j >> 5) & 31u); };
+    // shared-memory slot of tile index j: its low five bits XORed with five of
+    // the partners' bits, so the permuted reads of a warp spread over the banks
+    auto sp = [](uint32_t j) { return j ^ ((j >> SwapNet<T>::low) & 31u); };
     // persistent: CTA walks tiles b, b + gridDim.x, ...; a tile whose partner
     // (its outer bits permuted) comes first is moved by the partner's turn
     for (uint64_t b = blockIdx.x; b < ntiles; b += gridDim.x) {
@@ -493,13 +504,13 @@ __global__ void __launch_bounds__(256) k_swapnet(T* __restrict__ a, const __grid
         for (uint32_t c = 0; c < nchunk; ++c) po |= t_o[c][(uint32_t)(pb >> (8 * c)) & 255u];
         if (pb < b) continue;  // uniform over the CTA
         const bool two = pb != b;
-        // all of the thread's loads first (tn <= 1024: at most 4 per tile),
-        // so that they are in flight together
-        constexpr int kMax = 1024 / 256;
+        // all of the thread's loads first, so that they are in flight together
+        constexpr uint32_t kThreads = SwapNet<T>::threads;
+        constexpr int kMax = SwapNet<T>::tile / kThreads;
         T x0[kMax], x1[kMax];
 #pragma unroll
         for (int r = 0; r < kMax; ++r) {
-            const uint32_t j = threadIdx.x + 256u * (uint32_t)r;
+            const uint32_t j = threadIdx.x + kThreads * (uint32_t)r;
             if (j < tn) {
                 const uint64_t g = glo[j & ((1u << hl) - 1)] | ghi[j >> hl];
                 x0[r] = __ldcs(a + (o | g));
@@ -508,7 +519,7 @@ __global__ void __launch_bounds__(256) k_swapnet(T* __restrict__ a, const __grid
         }
 #pragma unroll
         for (int r = 0; r < kMax; ++r) {
-            const uint32_t j = threadIdx.x + 256u * (uint32_t)r;
+            const uint32_t j = threadIdx.x + kThreads * (uint32_t)r;
             if (j < tn) {
                 s0[sp(j)] = x0[r];
                 if (two) s1[sp(j)] = x1[r];
@@ -517,7 +528,7 @@ __global__ void __launch_bounds__(256) k_swapnet(T* __restrict__ a, const __grid
         __syncthreads();
 #pragma unroll
         for (int r = 0; r < kMax; ++r) {
-            const uint32_t j = threadIdx.x + 256u * (uint32_t)r;
+            const uint32_t j = threadIdx.x + kThreads * (uint32_t)r;
             if (j < tn) {
                 const uint32_t src = slo[j & ((1u << hl) - 1)] | shi[j >> hl];
                 const uint64_t g = glo[j & ((1u << hl) - 1)] | ghi[j >> hl];
@@ -529,22 +540,30 @@ __global__ void __launch_bounds__(256) k_swapnet(T* __restrict__ a, const __grid
     }
 }
 
+uint32_t swapnet_low(bool c64) { return c64 ? SwapNet<float2>::low : SwapNet<double2>::low; }
+
 cudaError_t launch_swapnet(void* a, bool c64, const PermParams& P, cudaStream_t st) {
-    // the outer-bit tables cover 32 bits; a tile holds at most 1024 amplitudes
-    if (P.n - P.na > 32 || P.na > 10) return cudaErrorInvalidValue;
+    // the outer-bit tables cover 32 bits
+    if (P.n - P.na > 32 || P.na > 2 * swapnet_low(c64)) return cudaErrorInvalidValue;
     const uint64_t tiles = 1ull << (P.n - P.na);
     const size_t smem = ((size_t)2 << P.na) * (c64 ? sizeof(float2) : sizeof(double2));
+    const int threads = c64 ? SwapNet<float2>::threads : SwapNet<double2>::threads;
     // persistent: as many CTAs as are resident at once, so none waits for a
     // slot behind CTAs that walk their whole share of the tiles
     int dev = 0, sms = 148, per_sm = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaError_t e = c64 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_swapnet<float2>, 256, smem)
-                        : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_swapnet<double2>, 256, smem);
+    cudaError_t e = c64 ? cudaFuncSetAttribute(k_swapnet<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               2 * SwapNet<float2>::tile * (int)sizeof(float2))
+                        : cudaFuncSetAttribute(k_swapnet<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               2 * SwapNet<double2>::tile * (int)sizeof(double2));
+    if (e != cudaSuccess) return e;
+    e = c64 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_swapnet<float2>, threads, smem)
+            : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_swapnet<double2>, threads, smem);
     if (e != cudaSuccess) return e;
     const unsigned blocks = (unsigned)std::min<uint64_t>(tiles, (uint64_t)sms * (uint64_t)std::max(per_sm, 1));
-    if (c64) k_swapnet<float2><<<blocks, 256, smem, st>>>((float2*)a, P);
-    else k_swapnet<double2><<<blocks, 256, smem, st>>>((double2*)a, P);
+    if (c64) k_swapnet<float2><<<blocks, threads, smem, st>>>((float2*)a, P);
+    else k_swapnet<double2><<<blocks, threads, smem, st>>>((double2*)a, P);
     return cudaGetLastError();
 }
 
