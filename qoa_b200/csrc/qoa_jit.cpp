@@ -361,6 +361,23 @@ uint32_t swz_base_bits(const Swizzle& z, const TileMap& m, const int* pos) {
 
 }  // namespace
 
+// Tile origin of tile number `b`: its bits deposited into the outer qubits,
+// one shift per run of consecutive qubits.
+std::string origin_expr(const PassParams& P, const char* b) {
+    std::string g = "0ull";
+    const int nout = (int)P.n - TILE_BITS;
+    char t[128];
+    for (int k = 0; k < nout;) {
+        int len = 1;
+        while (k + len < nout && P.outer_qubits[k + len] == P.outer_qubits[k] + len) ++len;
+        snprintf(t, sizeof t, " | (((%s >> %d) & 0x%llxull) << %d)", b, k,
+                 (unsigned long long)((len >= 64) ? ~0ull : ((1ull << len) - 1)), P.outer_qubits[k]);
+        g += t;
+        k += len;
+    }
+    return g;
+}
+
 // Kernel head shared by both precisions: the signature, shared memory, the
 // thread's lane / warp / tile number, the amplitude pointer, the pass
 // parameters P and the input's squared norm nrm. Single-state form: P is the
@@ -399,22 +416,7 @@ void emit_head(Emit& E, const PassParams& P, bool c64, bool arena) {
     }
     E.line("const uint32_t tw = (uint32_t)lane | ((uint32_t)wid << %d) | ((uint32_t)blk << %d);", LANE_BITS,
            LANE_BITS + WARP_BITS);
-    // tile origin: the tile number's bits deposited into the outer qubits,
-    // one shift per run of consecutive qubits
-    {
-        std::string g = "0ull";
-        const int nout = (int)P.n - TILE_BITS;
-        char b[128];
-        for (int k = 0; k < nout;) {
-            int len = 1;
-            while (k + len < nout && P.outer_qubits[k + len] == P.outer_qubits[k] + len) ++len;
-            snprintf(b, sizeof b, " | (((blk >> %d) & 0x%llxull) << %d)", k,
-                     (unsigned long long)((len >= 64) ? ~0ull : ((1ull << len) - 1)), P.outer_qubits[k]);
-            g += b;
-            k += len;
-        }
-        E.line("const uint64_t g0 = %s;", g.c_str());
-    }
+    E.line("const uint64_t g0 = %s;", origin_expr(P, "blk").c_str());
     if (c64 && arena)
         E.line("for (uint32_t i = threadIdx.x; i < %uu; i += PASS_THREADS) scoef[i] = coef32(P)[i];", P.ncoef);
     else if (arena)
@@ -597,19 +599,7 @@ std::string jit_pass_body_streamed(const PassParams& P) {
     E.line("const bool valid = nrm > 1e-12;");
     E.line("const uint64_t ntiles = 1ull << %d;", lt);
     // tile origin of tile number b: its bits deposited into the outer qubits
-    {
-        std::string g = "0ull";
-        char b[128];
-        for (int k = 0; k < lt;) {
-            int len = 1;
-            while (k + len < lt && P.outer_qubits[k + len] == P.outer_qubits[k] + len) ++len;
-            snprintf(b, sizeof b, " | (((b >> %d) & 0x%llxull) << %d)", k,
-                     (unsigned long long)((len >= 64) ? ~0ull : ((1ull << len) - 1)), P.outer_qubits[k]);
-            g += b;
-            k += len;
-        }
-        E.line("auto origin = [](uint64_t b) -> uint64_t { return %s; };", g.c_str());
-    }
+    E.line("auto origin = [](uint64_t b) -> uint64_t { return %s; };", origin_expr(P, "b").c_str());
     // rows of a tile: the lowest r high slots on qubits 5 .. 4 + r make runs
     // of 32 << r consecutive amplitudes, 64 >> r runs per tile
     int r = 0;
@@ -701,6 +691,33 @@ std::string jit_pass_body_streamed(const PassParams& P) {
     return E.s;
 }
 
+// Tiles ahead whose rows a complex128 pass prefetches into L2: one wave of
+// resident CTAs (148 SMs), so that a tile's loads meet L2 when its CTA starts.
+// Two waves ahead gain half as much.
+constexpr unsigned kPrefetchTiles = 148 * JIT_OCC;
+
+// After a tile's own loads: prefetches the rows (runs of 32 amplitudes, longer
+// where the lowest high slots are qubits 5, 6, ...) of the tile one wave on.
+// Only states that L2 (126 MB) does not hold. 27 qubits: 10.83 -> 10.60 ms for
+// 11 passes; complex64 passes lose by it (29 qubits 7.91 -> 8.05 ms for 4).
+void emit_prefetch(Emit& E, const PassParams& P) {
+    const unsigned esz = sizeof(double2), ahead = kPrefetchTiles;
+    if (((uint64_t)esz << P.n) <= (96ull << 20)) return;
+    int r = 0;
+    while (r < HIGH_SLOTS && P.slot_qubit[r] == LANE_BITS + r) ++r;
+    std::string off = "0ull";
+    char b[96];
+    for (int k = r; k < HIGH_SLOTS; ++k) {
+        snprintf(b, sizeof b, " + ((threadIdx.x & %uu) ? 0x%llxull : 0ull)", 1u << (k - r),
+                 (unsigned long long)(1ull << P.slot_qubit[k]));
+        off += b;
+    }
+    E.line("if (threadIdx.x < %du && blk + %uu < gridDim.x) {", 64 >> r, ahead);
+    E.line("const uint64_t nb = blk + %uu;", ahead);
+    E.line("prefetch_l2(amps + ((%s) + %s), %uu);", origin_expr(P, "nb").c_str(), off.c_str(), esz * (32u << r));
+    E.line("}");
+}
+
 std::string jit_pass_body(const PassParams& P, bool arena) {
     if (!arena && stream_f64()) return jit_pass_body_streamed(P);
     Emit E;
@@ -726,6 +743,7 @@ std::string jit_pass_body(const PassParams& P, bool arena) {
         }
         E.line("if (valid) {");
         for (int v = 0; v < REGS; ++v) E.line("a[%d] = __ldcs(amps + (tb + 0x%llxull));", v, off[v]);
+        if (!arena) emit_prefetch(E, P);
         E.line("} else {");
         for (int v = 0; v < REGS; ++v) E.line("a[%d] = make_double2(tb + 0x%llxull == 0 ? 1.0 : 0.0, 0.0);", v, off[v]);
         E.line("}");
@@ -956,19 +974,7 @@ std::string jit_pass32_body_streamed(const PassParams& P) {
     E.line("const double nrm = *norm2_in;");
     E.line("const bool valid = nrm > 1e-12;");
     E.line("const uint64_t ntiles = 1ull << %d;", lt);
-    {
-        std::string g = "0ull";
-        char b[128];
-        for (int k = 0; k < lt;) {
-            int len = 1;
-            while (k + len < lt && P.outer_qubits[k + len] == P.outer_qubits[k] + len) ++len;
-            snprintf(b, sizeof b, " | (((b >> %d) & 0x%llxull) << %d)", k,
-                     (unsigned long long)((len >= 64) ? ~0ull : ((1ull << len) - 1)), P.outer_qubits[k]);
-            g += b;
-            k += len;
-        }
-        E.line("auto origin = [](uint64_t b) -> uint64_t { return %s; };", g.c_str());
-    }
+    E.line("auto origin = [](uint64_t b) -> uint64_t { return %s; };", origin_expr(P, "b").c_str());
     int r = 0;
     while (r < HIGH_SLOTS && P.slot_qubit[r] == LANE_BITS + r) ++r;
     const int nrun = 64 >> r;

@@ -203,6 +203,10 @@ __device__ __forceinline__ void bulk_load(void* dst_smem, const void* src, uint3
         "l"(src), "r"(bytes), "r"(smem_u32(mb))
         : "memory");
 }
+// `bytes` (a multiple of 16, 16-byte aligned) of this GPU's own memory into L2
+__device__ __forceinline__ void prefetch_l2(const void* src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory");
+}
 // orders this thread's generic shared-memory accesses before later bulk
 // copies into the same memory
 __device__ __forceinline__ void proxy_fence_async() {
