@@ -1416,6 +1416,7 @@ int build_pass(const std::vector<Gate>& G, const Step& st, uint32_t n, PassParam
         PassOp o;
         memset(&o, 0, sizeof o);
         cond(mask, o);
+        o.k = d.x == -1.0 && d.y == 0.0;
         {
             const int tb = LANE_BITS + WARP_BITS;
             const uint64_t thr = o.tmask & ((1ull << tb) - 1), outer = o.tmask >> tb;

@@ -154,6 +154,48 @@ std::string tcond(uint32_t tm) {
     return b;
 }
 
+// The sign bit where the thread condition holds, else 0.
+std::string tsign(uint32_t tm) {
+    if (!tm) return "0x80000000u";
+    char b[64];
+    snprintf(b, sizeof b, "(((tw & 0x%xu) == 0x%xu) ? 0x80000000u : 0u)", tm, tm);
+    return b;
+}
+
+// A run of phase entries (those of a PC_DIAG_MX with one register mask, or a
+// PC_DIAG_TM) folded into the thread's factor f and sign sg (factors of
+// exactly -1); says which of the two the run has.
+struct RunKinds {
+    bool factors = false, signs = false;
+};
+RunKinds emit_run(Emit& E, const PassParams& P, uint32_t from, uint32_t to, const char* T, const char* mul, const char* cf) {
+    const uint32_t* ow = reinterpret_cast<const uint32_t*>(P.ops);
+    RunKinds k;
+    for (uint32_t e = from; e <= to; ++e) {
+        const PassOp& r = P.ops[e];
+        const uint32_t tm = ow[4 * e + 2];
+        const unsigned c = r.coef;
+        if (r.k & 1) {
+            E.line("%ssg %s %s;", k.signs ? "" : "uint32_t ", k.signs ? "^=" : "=", tsign(tm).c_str());
+            k.signs = true;
+        } else if (!k.factors) {
+            if (tm) E.line("%s f = %s ? %s[%u] : make_%s(1, 0);", T, tcond(tm).c_str(), cf, c, T);
+            else E.line("%s f = %s[%u];", T, cf, c);
+            k.factors = true;
+        } else {
+            if (tm) E.line("if (%s) f = %s(f, %s[%u]);", tcond(tm).c_str(), mul, cf, c);
+            else E.line("f = %s(f, %s[%u]);", mul, cf, c);
+        }
+    }
+    return k;
+}
+// The entries of the run that starts at e (the last carries the flag, or ends
+// the group at `end`).
+uint32_t run_end(const PassParams& P, uint32_t e, uint32_t end) {
+    while (e < end && !((P.ops[e].has_tp >> 1) & 1u)) ++e;
+    return e;
+}
+
 // Both mappings put the same tile bits on the warp bits: an exchange between
 // them moves data only among the threads of each warp.
 bool same_warps(const TileMap& a, const TileMap& b) {
@@ -477,11 +519,13 @@ const TileMap* emit_ops128(Emit& E, const PassParams& P, bool arena, const char*
         } else {
             switch (code) {
                 case PC_DIAG_T:
-                    if (tm) E.line("if (%s) pend = c_mul(pend, %s[%u]);", tcond(tm).c_str(), cf, c);
+                    if (op.k & 1) E.line("pend = flip(pend, %s);", tsign(tm).c_str());
+                    else if (tm) E.line("if (%s) pend = c_mul(pend, %s[%u]);", tcond(tm).c_str(), cf, c);
                     else E.line("pend = c_mul(pend, %s[%u]);", cf, c);
                     break;
                 case PC_DIAG_M:
-                    E.line("diag_m(a, %s, 0x%xu, %s[%u]);", tcond(tm).c_str(), cr, cf, c);
+                    if (op.k & 1) E.line("flip_m(a, 0x%xu, %s);", cr, tsign(tm).c_str());
+                    else E.line("diag_m(a, %s, 0x%xu, %s[%u]);", tcond(tm).c_str(), cr, cf, c);
                     break;
                 case PC_DIAG_TA:
                     if (tm) E.line("if (%s) pend = c_mul(pend, sang[%u]);", tcond(tm).c_str(), c);
@@ -492,28 +536,26 @@ const TileMap* emit_ops128(Emit& E, const PassParams& P, bool arena, const char*
                     break;
                 case PC_DIAG_MX:
                 case PC_DIAG_TM: {
-                    // the entries' thread-conditioned factors folded into f;
-                    // MX applies f to its register mask at the end of each run
-                    const uint32_t cnt = op.k;
-                    bool one = true;  // f is known to be 1
-                    E.line("{ T f = make_double2(1.0, 0.0);");
-                    for (uint32_t e = 1; e <= cnt; ++e) {
-                        const PassOp& r = P.ops[oi + e];
-                        const uint32_t rtm = ow[4 * (oi + e) + 2];
-                        if (!rtm && one) E.line("f = %s[%u];", cf, (unsigned)r.coef);
-                        else if (one) E.line("f = %s ? %s[%u] : make_double2(1.0, 0.0);", tcond(rtm).c_str(), cf, (unsigned)r.coef);
-                        else if (!rtm) E.line("f = c_mul(f, %s[%u]);", cf, (unsigned)r.coef);
-                        else E.line("if (%s) f = c_mul(f, %s[%u]);", tcond(rtm).c_str(), cf, (unsigned)r.coef);
-                        one = false;
-                        if (code == PC_DIAG_MX && (e == cnt || ((r.has_tp >> 1) & 1u))) {
-                            E.line("diag_m(a, true, 0x%xu, f);", (unsigned)r.cond_reg);
-                            if (e != cnt) E.line("f = make_double2(1.0, 0.0);");
-                            one = true;
+                    // MX: run by run, applied to the run's registers; TM: all to the pending factor
+                    const uint32_t end = oi + op.k;
+                    for (uint32_t e = oi + 1; e <= end;) {
+                        const uint32_t last = code == PC_DIAG_MX ? run_end(P, e, end) : end;
+                        const unsigned rcr = P.ops[last].cond_reg;
+                        E.line("{");
+                        const RunKinds k = emit_run(E, P, e, last, "double2", "c_mul", cf);
+                        if (code == PC_DIAG_TM) {
+                            if (k.factors) E.line("pend = c_mul(pend, f);");
+                            if (k.signs) E.line("pend = flip(pend, sg);");
+                        } else if (!k.factors) {
+                            E.line("flip_m(a, 0x%xu, sg);", rcr);
+                        } else {
+                            if (k.signs) E.line("f = flip(f, sg);");
+                            E.line("diag_m(a, true, 0x%xu, f);", rcr);
                         }
+                        E.line("}");
+                        e = last + 1;
                     }
-                    if (code == PC_DIAG_TM && cnt) E.line("pend = c_mul(pend, f);");
-                    E.line("}");
-                    oi += cnt;
+                    oi = end;
                     break;
                 }
                 case PC_DIAG_TAB:
@@ -834,11 +876,13 @@ const TileMap* emit_ops64(Emit& E, const PassParams& P, bool arena) {
         } else {
             switch (code) {
                 case PC_DIAG_T:
-                    if (tm) E.line("if (%s) pend = cmulf(pend, scoef[%u]);", tcond(tm).c_str(), c);
+                    if (op.k & 1) E.line("pend = flip(pend, %s);", tsign(tm).c_str());
+                    else if (tm) E.line("if (%s) pend = cmulf(pend, scoef[%u]);", tcond(tm).c_str(), c);
                     else E.line("pend = cmulf(pend, scoef[%u]);", c);
                     break;
                 case PC_DIAG_M:
-                    E.line("diag_p(re, im, %s, 0x%xu, scoef[%u]);", tcond(tm).c_str(), cr, c);
+                    if (op.k & 1) E.line("flip_p(re, im, 0x%xu, %s);", cr, tsign(tm).c_str());
+                    else E.line("diag_p(re, im, %s, 0x%xu, scoef[%u]);", tcond(tm).c_str(), cr, c);
                     break;
                 case PC_DIAG_TA:
                     if (tm) E.line("if (%s) pend = cmulf(pend, sang[%u]);", tcond(tm).c_str(), c);
@@ -849,26 +893,25 @@ const TileMap* emit_ops64(Emit& E, const PassParams& P, bool arena) {
                     break;
                 case PC_DIAG_MX:
                 case PC_DIAG_TM: {
-                    const uint32_t cnt = op.k;
-                    bool one = true;
-                    E.line("{ float2 f = make_float2(1.f, 0.f);");
-                    for (uint32_t e = 1; e <= cnt; ++e) {
-                        const PassOp& r = P.ops[oi + e];
-                        const uint32_t rtm = ow[4 * (oi + e) + 2];
-                        if (!rtm && one) E.line("f = scoef[%u];", (unsigned)r.coef);
-                        else if (one) E.line("f = %s ? scoef[%u] : make_float2(1.f, 0.f);", tcond(rtm).c_str(), (unsigned)r.coef);
-                        else if (!rtm) E.line("f = cmulf(f, scoef[%u]);", (unsigned)r.coef);
-                        else E.line("if (%s) f = cmulf(f, scoef[%u]);", tcond(rtm).c_str(), (unsigned)r.coef);
-                        one = false;
-                        if (code == PC_DIAG_MX && (e == cnt || ((r.has_tp >> 1) & 1u))) {
-                            E.line("diag_p(re, im, true, 0x%xu, f);", (unsigned)r.cond_reg);
-                            if (e != cnt) E.line("f = make_float2(1.f, 0.f);");
-                            one = true;
+                    const uint32_t end = oi + op.k;
+                    for (uint32_t e = oi + 1; e <= end;) {
+                        const uint32_t last = code == PC_DIAG_MX ? run_end(P, e, end) : end;
+                        const unsigned rcr = P.ops[last].cond_reg;
+                        E.line("{");
+                        const RunKinds k = emit_run(E, P, e, last, "float2", "cmulf", "scoef");
+                        if (code == PC_DIAG_TM) {
+                            if (k.factors) E.line("pend = cmulf(pend, f);");
+                            if (k.signs) E.line("pend = flip(pend, sg);");
+                        } else if (!k.factors) {
+                            E.line("flip_p(re, im, 0x%xu, sg);", rcr);
+                        } else {
+                            if (k.signs) E.line("f = flip(f, sg);");
+                            E.line("diag_p(re, im, true, 0x%xu, f);", rcr);
                         }
+                        E.line("}");
+                        e = last + 1;
                     }
-                    if (code == PC_DIAG_TM && cnt) E.line("pend = cmulf(pend, f);");
-                    E.line("}");
-                    oi += cnt;
+                    oi = end;
                     break;
                 }
                 case PC_DIAG_TAB:

@@ -94,7 +94,7 @@ enum PassCode : uint8_t {
 // 16-byte aligned: the pass kernels stage the op stream with 16-byte loads.
 struct alignas(16) PassOp {
     uint8_t code;
-    uint8_t k;          // register bit of the op
+    uint8_t k;          // register bit of the op; phases (and entries of a run): 1 where the factor is exactly -1
     uint16_t coef;      // index into PassParams::coef; PC_XCHG: mapping index
     uint8_t cond_reg;   // register-bit mask
     uint8_t cond_lane;  // lane-bit mask

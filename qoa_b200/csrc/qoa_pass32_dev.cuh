@@ -182,6 +182,18 @@ __device__ __forceinline__ void diag_p(u64p (&re)[8], u64p (&im)[8], bool tp, ui
         if (((uint32_t)j & cl) == cl) cmul2(re[j], im[j], cr, ci);
 }
 
+// flip the signs (sgn: 0 or the sign bit) of the registers v with (v & creg) == creg
+__device__ __forceinline__ void flip_p(u64p (&re)[8], u64p (&im)[8], uint32_t creg, uint32_t sgn) {
+    const uint32_t cl = creg & 7u;
+    const u64p m = ((u64p)sgn << 32) | ((creg & 8u) ? 0u : sgn);
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+        if (((uint32_t)j & cl) == cl) {
+            re[j] ^= m;
+            im[j] ^= m;
+        }
+}
+
 // Squared norm of a thread's 16 amplitudes: packed FP32 products summed per
 // half (8 amplitudes each), the two halves added in FP64.
 __device__ __forceinline__ double norm2_p(const u64p (&re)[8], const u64p (&im)[8]) {

@@ -153,6 +153,22 @@ __device__ __forceinline__ void diag_m(T (&a)[REGS], bool tp, uint32_t creg, T d
         if ((v & creg) == creg) a[v] = c_mul(a[v], d);
 }
 
+// Sign flips (sgn: 0 or the sign bit) in place of products with -1: they run
+// on the integer pipe beside the FP64 work that bounds a pass.
+__device__ __forceinline__ double flip(double x, uint32_t sgn) {
+    return __hiloint2double((int)((uint32_t)__double2hiint(x) ^ sgn), __double2loint(x));
+}
+__device__ __forceinline__ double2 flip(double2 a, uint32_t sgn) { return make_double2(flip(a.x, sgn), flip(a.y, sgn)); }
+__device__ __forceinline__ float2 flip(float2 a, uint32_t sgn) {
+    return make_float2(__uint_as_float(__float_as_uint(a.x) ^ sgn), __uint_as_float(__float_as_uint(a.y) ^ sgn));
+}
+template <typename T>
+__device__ __forceinline__ void flip_m(T (&a)[REGS], uint32_t creg, uint32_t sgn) {
+#pragma unroll
+    for (int v = 0; v < REGS; ++v)
+        if ((v & creg) == creg) a[v] = flip(a[v], sgn);
+}
+
 // Shared-memory position of tile index j: the low three bits are XORed with
 // the three-bit folds of the higher bits, so any three tile bits with distinct
 // residues mod 3 spread a quarter-warp's 16-byte accesses over all banks.
