@@ -63,9 +63,11 @@ const char kPrelude[] =
     "#include \"qoa_pass32_dev.cuh\"\n";
 
 // Resident CTAs per SM of a generated pass (128 threads): complex128 the
-// same register budget as k_pass (128), complex64 up to 80 registers.
+// same register budget as k_pass (128), complex64 up to 72 registers (7 against
+// 6 CTAs: 4 passes of 29 qubits 7.90 -> 7.76 ms, 10 of 23 qubits 406 -> 397 us;
+// 8 no better).
 constexpr int JIT_OCC = 4;
-constexpr int JIT_OCC32 = 6;
+constexpr int JIT_OCC32 = 7;
 
 // QOA_JIT_OCC / QOA_JIT_OCC32 override the resident-CTA targets (tuning).
 int occ_target(bool c64) {
