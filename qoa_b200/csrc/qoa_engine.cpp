@@ -2746,9 +2746,11 @@ inline bool shim_bit_ok(size_t b) { return b < 64; }
 enum BatchRoute { R_SMALL = 0, R_ARENA = 1, R_VIEW = 2 };
 constexpr int kRoundStreams = 4;  // extra streams of a round's generated launches
 // What a structure must serve in a batch to be compiled in the default mode.
-// 1024 tiles are 2^21 amplitudes: a generated pass over them saves ~25 us a run.
+// 512 tiles are one pass of a 20-qubit state, the smallest that compiles its
+// passes (192 circuits of 8-20 qubits: 2639 us with 1024 tiles and 21 kernels,
+// 2201 with 512 and 78, 2227 with 256 and 93).
 constexpr uint32_t kJitMinJobs = 8;
-constexpr uint64_t kJitMinTiles = 1024;
+constexpr uint64_t kJitMinTiles = 512;
 
 struct qoa_batch_s {
     int precision = QOA_PREC_F64;
