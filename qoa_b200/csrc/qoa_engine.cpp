@@ -2098,8 +2098,23 @@ struct PassNorm {
     bool per_gate = false;  // set where the pass ran as per-gate kernels instead (norm2 is then valid)
 };
 
-// Every gate of the pass is unitary by its kind (not a caller's matrix) and
-// finite: with the factors of build_pass in P.phase, a normalised input gives
+// A caller's k x k matrix is unitary to 1e-10: the norm it gives can drift by
+// that much, far from the 1e-12 below which a state is reset.
+bool unitary_matrix(const double2* m, int k) {
+    for (int a = 0; a < k; ++a)
+        for (int b = 0; b <= a; ++b) {
+            double re = a == b ? -1.0 : 0.0, im = 0.0;  // <row b, row a> - delta
+            for (int c = 0; c < k; ++c) {
+                const double2 x = m[a * k + c], y = m[b * k + c];
+                re += x.x * y.x + x.y * y.y;
+                im += x.y * y.x - x.x * y.y;
+            }
+            if (!(std::fabs(re) < 1e-10 && std::fabs(im) < 1e-10)) return false;
+        }
+    return true;
+}
+
+// Every gate of the pass is unitary and finite: with the factors of build_pass in P.phase, a normalised input gives
 // a normalised output (to rounding), so its norm need not be measured before
 // the next pass. Measured after the last of such a run, as the scale the run
 // has drifted by (of order 1e-16 a gate) belongs to all amplitudes alike.
@@ -2110,8 +2125,10 @@ bool unitary_pass(const std::vector<Gate>& G, const Step& st) {
         if (g.kind == K_DIAG) {
             if (!g.neg && !(unit(g.m[0]) && (g.t < 0 || unit(g.m[1])))) return false;
         } else if (g.kind == K_G1) {
-            if (g.sub == G1_GEN) return false;
+            if (g.sub == G1_GEN && !unitary_matrix(g.m, 2)) return false;
             if ((g.sub == G1_RX || g.sub == G1_RY) && !unit(g.m[0])) return false;
+        } else if (g.kind == K_U2) {
+            if (!unitary_matrix(g.m, 4)) return false;
         } else if (g.kind != K_SWAP) {
             return false;
         }
