@@ -44,7 +44,7 @@ cudaError_t launch_swapnet(void* a, bool c64, const PermParams& P, cudaStream_t 
 int reduce_blocks(uint64_t len);
 cudaError_t launch_norm(const void* a, bool f32, uint64_t len, double* partials, unsigned int* ticket, double* out,
                         uint32_t* status, cudaStream_t st);
-cudaError_t launch_p01(const double2* a, uint64_t len, uint32_t q, double* partials, unsigned int* ticket, double* out2,
+cudaError_t launch_p01(const double2* a, uint64_t len, uint32_t q, double* partials, unsigned int* ticket, double* out3,
                        const double* norm2, cudaStream_t st);
 uint32_t expz_blocks(uint64_t len);
 cudaError_t launch_expz(const void* a, bool f32, uint64_t len, const ExpzMasks& M, uint32_t k, const double* norm2,
@@ -53,7 +53,7 @@ cudaError_t launch_reduce_partials(const double* partials, uint32_t count, doubl
 cudaError_t launch_collapse(double2* a, uint64_t len, uint32_t q, uint32_t outcome, double f, double* partials,
                             unsigned int* ticket, double* norm2_out, uint32_t* status, cudaStream_t st);
 cudaError_t launch_materialize(void* a, bool f32, uint64_t len, double* norm2, double* partials, unsigned int* ticket,
-                               uint32_t* status, cudaStream_t st);
+                               uint32_t* status, void* copy, cudaStream_t st);
 cudaError_t launch_set_scalar(double* p, double v, cudaStream_t st);
 cudaError_t launch_init_scalars(double* scal, uint32_t* status, cudaStream_t st);
 cudaError_t launch_probs(const double2* a, uint64_t off, uint64_t cnt, const double* norm2, double* out, cudaStream_t st);
@@ -296,6 +296,9 @@ double gate_bytes(const Gate& g, uint32_t n) {
 }  // namespace
 
 // ------------------------------------------------------------------ handle
+constexpr size_t HOST_RESULTS = 512;  // (a state of up to 8 qubits, or EXPZ_MASKS expectation values)
+static_assert(HOST_RESULTS >= EXPZ_MASKS, "results of one expectation sweep");
+
 struct qoa_state_s {
     uint32_t n = 1;
     uint32_t flags = 0;
@@ -317,7 +320,7 @@ struct qoa_state_s {
     size_t partials_cap = 0;
     double* ws = nullptr;         // scratch kept between calls (workspace)
     size_t ws_cap = 0;
-    double* host_scal = nullptr;  // pinned: mirror of scal, then EXPZ_MASKS results
+    double* host_scal = nullptr;  // pinned: mirror of scal, then HOST_RESULTS doubles that kernels write results to
     uint64_t seed = 0;
     uint64_t noise_stream = 0;
     uint64_t noise_event = 0;
@@ -2221,9 +2224,10 @@ int run_small(qoa_state_t s, const SmallList& L, int in) {
 
 // Reads norm2, P0, P1 of qubit q (logical probabilities) to the host.
 int read_p01(qoa_state_t s, uint32_t q, double& p0, double& p1, double& norm2) {
-    CK(launch_p01(s->amps, state_len(s), q, s->partials, ticket(s), s->scal + 1, s->scal, s->stream));
+    // norm2, P0 and P1 go straight to pinned host memory (a copy after the
+    // kernel costs ~4 us more)
+    CK(launch_p01(s->amps, state_len(s), q, s->partials, ticket(s), s->host_scal, s->scal, s->stream));
     s->launches++;
-    CK(cudaMemcpyAsync(s->host_scal, s->scal, 3 * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     norm2 = s->host_scal[0];
     if (!(norm2 > 1e-12)) {  // logical state is |0..0>
@@ -3613,7 +3617,7 @@ int qoa_create(uint32_t n, int precision, uint32_t flags, qoa_state_t* out) {
     if (cudaMalloc(&s->status, 4 * sizeof(uint32_t)) != cudaSuccess) return fail(set_err(s, QOA_E_OOM, "status alloc"));
     if (launch_init_scalars(s->scal, s->status, s->stream) != cudaSuccess)
         return fail(set_err(s, QOA_E_CUDA, "scalar set-up"));
-    if (cudaMallocHost(&s->host_scal, (16 + EXPZ_MASKS) * sizeof(double)) != cudaSuccess) return fail(set_err(s, QOA_E_OOM, "pinned alloc"));
+    if (cudaMallocHost(&s->host_scal, (16 + HOST_RESULTS) * sizeof(double)) != cudaSuccess) return fail(set_err(s, QOA_E_OOM, "pinned alloc"));
     int rc = alloc_state(s, n);
     if (rc) return fail(rc);
     rc = do_reset_all(s);
@@ -3747,14 +3751,13 @@ int qoa_expect_z(qoa_state_t s, const uint64_t* masks, size_t k, double* out) {
         const uint32_t kk = (uint32_t)std::min<size_t>(EXPZ_MASKS, k - i);
         ExpzMasks M;
         std::memcpy(M.m, masks + i, kk * sizeof(uint64_t));
-        double* ws = nullptr;  // results, then partial sums
-        rc = workspace(s, (size_t)kk * (1 + blocks) * sizeof(double), &ws);
+        double* ws = nullptr;  // partial sums
+        rc = workspace(s, (size_t)kk * blocks * sizeof(double), &ws);
         if (rc) return rc;
-        // FP64 sums over either precision
-        CK(launch_expz(s->amps, s->precision == QOA_PREC_F32, state_len(s), M, kk, s->scal, ws + kk, ticket(s), ws,
-                       s->stream));
+        // FP64 sums over either precision, results straight to pinned host memory
+        CK(launch_expz(s->amps, s->precision == QOA_PREC_F32, state_len(s), M, kk, s->scal, ws, ticket(s),
+                       s->host_scal + 16, s->stream));
         s->launches++;
-        CK(cudaMemcpyAsync(s->host_scal + 16, ws, kk * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
         CK(cudaStreamSynchronize(s->stream));
         std::memcpy(out + i, s->host_scal + 16, kk * sizeof(double));
     }
@@ -3767,9 +3770,16 @@ int qoa_get_state(qoa_state_t s, void* host, size_t bytes) {
     const size_t esz = s->precision == QOA_PREC_F32 ? sizeof(float2) : sizeof(double2);
     if (!host || bytes != state_len(s) * esz)
         return set_err(s, QOA_E_ARG, "get_state needs %llu bytes", (unsigned long long)(state_len(s) * esz));
+    // a small state also goes straight to pinned host memory
+    void* direct = bytes <= HOST_RESULTS * sizeof(double) ? s->host_scal + 16 : nullptr;
     CK(launch_materialize(s->amps, s->precision == QOA_PREC_F32, state_len(s), s->scal, s->partials, ticket(s), s->status,
-                          s->stream));
+                          direct, s->stream));
     s->launches++;
+    if (direct) {
+        CK(cudaStreamSynchronize(s->stream));
+        std::memcpy(host, direct, bytes);
+        return QOA_OK;
+    }
     CK(cudaMemcpyAsync(host, s->amps, bytes, cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     return QOA_OK;
@@ -4549,11 +4559,11 @@ int qoa_vec_apply_reset(double* amps, size_t len, size_t bit) {
     if (len) {
         CK(launch_p01(dev, len, (uint32_t)bit, g_shim_scr + 8, shim_ticket(), g_shim_scr, nullptr, g_shim_stream));
         double p[2];
-        CK(cudaMemcpyAsync(p, g_shim_scr, sizeof p, cudaMemcpyDeviceToHost, g_shim_stream));
+        CK(cudaMemcpyAsync(p, g_shim_scr + 1, sizeof p, cudaMemcpyDeviceToHost, g_shim_stream));
         CK(cudaStreamSynchronize(g_shim_stream));
         if (p[0] > 1e-12) {
             CK(launch_collapse(dev, len, (uint32_t)bit, 0, 1.0 / std::sqrt(p[0]), g_shim_scr + 8, shim_ticket(),
-                               g_shim_scr + 2, nullptr, g_shim_stream));
+                               g_shim_scr + 3, nullptr, g_shim_stream));
         } else {
             GGate k;
             memset(&k, 0, sizeof k);

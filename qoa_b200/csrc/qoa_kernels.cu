@@ -637,7 +637,8 @@ __global__ void k_norm(const T* __restrict__ a, uint64_t len, double* __restrict
     finish_norm(partials, ticket, norm2, status);
 }
 
-// P(bit q = 0), P(bit q = 1) of the stored vector, divided by norm2 (null: not divided)
+// norm2, P(bit q = 0), P(bit q = 1) of the stored vector, divided by norm2 (null: 1);
+// out may be pinned host memory
 __global__ void k_p01(const double2* __restrict__ a, uint64_t len, uint32_t q, double* __restrict__ partials,
                       unsigned int* ticket, const double* __restrict__ norm2, double* __restrict__ out) {
     double v[2] = {0.0, 0.0};
@@ -653,8 +654,9 @@ __global__ void k_p01(const double2* __restrict__ a, uint64_t len, uint32_t q, d
 #pragma unroll
     for (int s = 0; s < 2; ++s) {
         const double t = sum_partials(partials + (uint64_t)s * gridDim.x);
-        if (threadIdx.x == 0) out[s] = d > 1e-12 ? t / d : 0.0;
+        if (threadIdx.x == 0) out[1 + s] = d > 1e-12 ? t / d : 0.0;
     }
+    if (threadIdx.x == 0) out[0] = d;
 }
 
 // Final reduction: out[s] = sum_k partials[s*count + k] in a fixed order (one
@@ -717,10 +719,11 @@ __global__ void k_collapse(double2* __restrict__ a, uint64_t len, uint32_t q, ui
 }
 
 // Materialise the pending normalisation in place (or reset to |0..0>). norm2
-// is read by every CTA before the last of them writes it.
+// is read by every CTA before the last of them writes it. copy (may be null):
+// the result once more, in pinned host memory.
 template <typename T>
 __global__ void k_materialize(T* __restrict__ a, uint64_t len, double* norm2, double* __restrict__ partials,
-                              unsigned int* ticket, uint32_t* __restrict__ status) {
+                              unsigned int* ticket, uint32_t* __restrict__ status, T* __restrict__ copy) {
     using R = typename CT<T>::R;
     double v[1] = {0.0};
     const double nrm = *reinterpret_cast<volatile double*>(norm2);
@@ -735,6 +738,7 @@ __global__ void k_materialize(T* __restrict__ a, uint64_t len, double* norm2, do
             x = CT<T>::mk(i == 0 ? (R)1 : (R)0, (R)0);
         }
         a[i] = x;
+        if (copy) copy[i] = x;
         v[0] += c_abs2(x);
     }
     block_store_partials<1>(v, partials, gridDim.x);
@@ -848,9 +852,9 @@ cudaError_t launch_norm(const void* a, bool f32, uint64_t len, double* partials,
     return cudaGetLastError();
 }
 
-cudaError_t launch_p01(const double2* a, uint64_t len, uint32_t q, double* partials, unsigned int* ticket, double* out2,
+cudaError_t launch_p01(const double2* a, uint64_t len, uint32_t q, double* partials, unsigned int* ticket, double* out3,
                        const double* norm2, cudaStream_t st) {
-    k_p01<<<reduce_blocks(len), 256, 0, st>>>(a, len, q, partials, ticket, norm2, out2);
+    k_p01<<<reduce_blocks(len), 256, 0, st>>>(a, len, q, partials, ticket, norm2, out3);
     return cudaGetLastError();
 }
 
@@ -872,10 +876,10 @@ cudaError_t launch_collapse(double2* a, uint64_t len, uint32_t q, uint32_t outco
 }
 
 cudaError_t launch_materialize(void* a, bool f32, uint64_t len, double* norm2, double* partials, unsigned int* ticket,
-                               uint32_t* status, cudaStream_t st) {
+                               uint32_t* status, void* copy, cudaStream_t st) {
     const int nb = reduce_blocks(len);
-    if (f32) k_materialize<<<nb, 256, 0, st>>>((float2*)a, len, norm2, partials, ticket, status);
-    else k_materialize<<<nb, 256, 0, st>>>((double2*)a, len, norm2, partials, ticket, status);
+    if (f32) k_materialize<<<nb, 256, 0, st>>>((float2*)a, len, norm2, partials, ticket, status, (float2*)copy);
+    else k_materialize<<<nb, 256, 0, st>>>((double2*)a, len, norm2, partials, ticket, status, (double2*)copy);
     return cudaGetLastError();
 }
 
