@@ -296,9 +296,6 @@ double gate_bytes(const Gate& g, uint32_t n) {
 }  // namespace
 
 // ------------------------------------------------------------------ handle
-constexpr size_t HOST_RESULTS = 512;  // (a state of up to 8 qubits, or EXPZ_MASKS expectation values)
-static_assert(HOST_RESULTS >= EXPZ_MASKS, "results of one expectation sweep");
-
 struct qoa_state_s {
     uint32_t n = 1;
     uint32_t flags = 0;
@@ -320,7 +317,7 @@ struct qoa_state_s {
     size_t partials_cap = 0;
     double* ws = nullptr;         // scratch kept between calls (workspace)
     size_t ws_cap = 0;
-    double* host_scal = nullptr;  // pinned: mirror of scal, then HOST_RESULTS doubles that kernels write results to
+    double* host_scal = nullptr;  // pinned: mirror of scal, then EXPZ_MASKS results (kernels write them there)
     uint64_t seed = 0;
     uint64_t noise_stream = 0;
     uint64_t noise_event = 0;
@@ -446,6 +443,59 @@ int alloc_state(qoa_state_t s, uint32_t n) {
     CK(device_alloc((void**)&s->partials, s->partials_cap * sizeof(double)));
     return QOA_OK;
 }
+
+// Pinned host buffers for the results (and uniforms) of synchronous calls, one
+// for the length of a call: a copy between device and pageable memory is
+// staged by the driver piece by piece, and small results need no copy at all
+// when the kernel writes them here. Shared by all handles and threads; at most
+// kStagingKept stay allocated between calls.
+constexpr size_t kStagingBytes = size_t(1) << 20;
+constexpr size_t kStagingKept = 8;
+std::mutex g_staging_mu;
+std::vector<void*> g_staging;
+class Staging {
+public:
+    // null where the call needs more than a buffer holds, or none can be had
+    Staging(size_t bytes, cudaStream_t st) : st_(st) {
+        if (!bytes || bytes > kStagingBytes) return;
+        {
+            std::lock_guard<std::mutex> lk(g_staging_mu);
+            if (!g_staging.empty()) {
+                p_ = g_staging.back();
+                g_staging.pop_back();
+                return;
+            }
+        }
+        if (cudaHostAlloc(&p_, kStagingBytes, cudaHostAllocPortable) != cudaSuccess) {
+            cudaGetLastError();
+            p_ = nullptr;
+        }
+    }
+    ~Staging() {
+        if (!p_) return;
+        if (!done_) cudaStreamSynchronize(st_);  // an error on the way: work may still use the buffer
+        {
+            std::lock_guard<std::mutex> lk(g_staging_mu);
+            if (g_staging.size() < kStagingKept) {
+                g_staging.push_back(p_);
+                return;
+            }
+        }
+        cudaFreeHost(p_);
+    }
+    Staging(const Staging&) = delete;
+    Staging& operator=(const Staging&) = delete;
+    double* get() const { return static_cast<double*>(p_); }
+    void done() { done_ = true; }  // the stream has been waited for
+
+private:
+    cudaStream_t st_;
+    void* p_ = nullptr;
+    bool done_ = false;
+};
+// Kernels write (or read) pinned host memory themselves up to this many bytes;
+// above it a copy is faster than their stores over the bus.
+constexpr size_t kDirectBytes = 64 << 10;
 
 // Scratch of a synchronous call (sampling, probabilities) on the handle's
 // stream, kept by the handle up to kWorkspaceKept bytes: a buffer allocated
@@ -3617,7 +3667,7 @@ int qoa_create(uint32_t n, int precision, uint32_t flags, qoa_state_t* out) {
     if (cudaMalloc(&s->status, 4 * sizeof(uint32_t)) != cudaSuccess) return fail(set_err(s, QOA_E_OOM, "status alloc"));
     if (launch_init_scalars(s->scal, s->status, s->stream) != cudaSuccess)
         return fail(set_err(s, QOA_E_CUDA, "scalar set-up"));
-    if (cudaMallocHost(&s->host_scal, (16 + HOST_RESULTS) * sizeof(double)) != cudaSuccess) return fail(set_err(s, QOA_E_OOM, "pinned alloc"));
+    if (cudaMallocHost(&s->host_scal, (16 + EXPZ_MASKS) * sizeof(double)) != cudaSuccess) return fail(set_err(s, QOA_E_OOM, "pinned alloc"));
     int rc = alloc_state(s, n);
     if (rc) return fail(rc);
     rc = do_reset_all(s);
@@ -3703,20 +3753,28 @@ int qoa_sample(qoa_state_t s, const double* u, size_t shots, int mode, uint64_t*
     const uint32_t n = s->n;
     const size_t nu = mode == 0 ? shots * n : shots;
     const SampleLevels L = sample_levels(n);
-    // uniforms, then the outcomes, then the tree levels: one workspace
+    // uniforms, then the outcomes, then the tree levels: one workspace.
+    // Shots read each uniform and write each outcome once, so both may also
+    // stay in pinned host memory.
+    const size_t io = (nu + shots) * sizeof(double);
+    Staging host(io, s->stream);
+    const bool direct = host.get() && io <= 4 * kDirectBytes;
     double* ws = nullptr;
-    rc = workspace(s, (nu + shots + (size_t)L.total) * sizeof(double), &ws);
+    rc = workspace(s, ((direct ? 0 : nu + shots) + (size_t)L.total) * sizeof(double) + sizeof(double), &ws);
     if (rc) return rc;
-    double* d_u = ws;
-    unsigned long long* d_out = reinterpret_cast<unsigned long long*>(ws + nu);
-    double* d_tree = ws + nu + shots;
-    CK(cudaMemcpyAsync(d_u, u, nu * sizeof(double), cudaMemcpyHostToDevice, s->stream));
+    double* d_u = direct ? host.get() : ws;
+    unsigned long long* d_out = reinterpret_cast<unsigned long long*>(d_u + nu);
+    double* d_tree = direct ? ws : ws + nu + shots;
     const bool f32 = s->precision == QOA_PREC_F32;
     CK(launch_sample_tree(s->amps, f32, n, s->scal, L, d_tree, s->stream));
+    if (direct) std::memcpy(host.get(), u, nu * sizeof(double));  // while the tree is made
+    else CK(cudaMemcpyAsync(d_u, u, nu * sizeof(double), cudaMemcpyHostToDevice, s->stream));
     CK(launch_shots(s->amps, f32, n, s->scal, d_tree, L, d_u, shots, mode, d_out, s->stream));
     s->launches += L.count + 1;
-    CK(cudaMemcpyAsync(out, d_out, shots * sizeof(uint64_t), cudaMemcpyDeviceToHost, s->stream));
+    if (!direct) CK(cudaMemcpyAsync(out, d_out, shots * sizeof(uint64_t), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
+    host.done();
+    if (direct) std::memcpy(out, d_out, shots * sizeof(uint64_t));
     return workspace_done(s);
 }
 
@@ -3726,6 +3784,23 @@ int qoa_probabilities(qoa_state_t s, double* out) {
     if (!out) return set_err(s, QOA_E_ARG, "null out");
     const uint64_t len = state_len(s);
     const uint64_t chunk = std::min<uint64_t>(len, 1ull << 24);
+    Staging host(len * sizeof(double), s->stream);
+    if (host.get()) {
+        const bool direct = len * sizeof(double) <= kDirectBytes;
+        double* d = host.get();
+        if (!direct) {
+            rc = workspace(s, len * sizeof(double), &d);
+            if (rc) return rc;
+        }
+        if (s->precision == QOA_PREC_F32) CK(launch_f32_probs((const float2*)s->amps, 0, len, s->scal, d, s->stream));
+        else CK(launch_probs(s->amps, 0, len, s->scal, d, s->stream));
+        s->launches++;
+        if (!direct) CK(cudaMemcpyAsync(host.get(), d, len * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
+        CK(cudaStreamSynchronize(s->stream));
+        host.done();
+        std::memcpy(out, host.get(), len * sizeof(double));
+        return QOA_OK;
+    }
     double* d = nullptr;
     rc = workspace(s, chunk * sizeof(double), &d);
     if (rc) return rc;
@@ -3770,18 +3845,15 @@ int qoa_get_state(qoa_state_t s, void* host, size_t bytes) {
     const size_t esz = s->precision == QOA_PREC_F32 ? sizeof(float2) : sizeof(double2);
     if (!host || bytes != state_len(s) * esz)
         return set_err(s, QOA_E_ARG, "get_state needs %llu bytes", (unsigned long long)(state_len(s) * esz));
-    // a small state also goes straight to pinned host memory
-    void* direct = bytes <= HOST_RESULTS * sizeof(double) ? s->host_scal + 16 : nullptr;
+    Staging pin(bytes, s->stream);
+    void* direct = bytes <= kDirectBytes ? pin.get() : nullptr;  // the kernel's second copy
     CK(launch_materialize(s->amps, s->precision == QOA_PREC_F32, state_len(s), s->scal, s->partials, ticket(s), s->status,
                           direct, s->stream));
     s->launches++;
-    if (direct) {
-        CK(cudaStreamSynchronize(s->stream));
-        std::memcpy(host, direct, bytes);
-        return QOA_OK;
-    }
-    CK(cudaMemcpyAsync(host, s->amps, bytes, cudaMemcpyDeviceToHost, s->stream));
+    if (!direct) CK(cudaMemcpyAsync(pin.get() ? pin.get() : host, s->amps, bytes, cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
+    pin.done();
+    if (pin.get()) std::memcpy(host, pin.get(), bytes);
     return QOA_OK;
 }
 
