@@ -19,6 +19,7 @@
 #include <stdint.h>
 
 #include "qoa_kernels.cuh"
+#include "qoa_launch.cuh"
 #include "qoa_pass_dev.cuh"
 
 namespace qoa {
@@ -91,6 +92,8 @@ __global__ void __launch_bounds__(THREADS, MI <= 4 ? 4 : 2)
 k_expz(const T* __restrict__ a, uint64_t len, const __grid_constant__ ExpzMasks M, uint32_t k,
        const double* __restrict__ norm2, double* __restrict__ partials, unsigned int* __restrict__ ticket,
        double* __restrict__ out) {
+    grid_go();
+    grid_wait();
     __shared__ double sm[TILE];
     __shared__ bool last;
     const uint32_t t = threadIdx.x, g = t >> 4;
@@ -176,11 +179,11 @@ __global__ void __launch_bounds__(256) k_arena_expz_final(const ExpzJob* __restr
 }
 
 template <typename T>
-void expz(const T* a, uint64_t len, const ExpzMasks& M, uint32_t k, const double* norm2, double* partials,
+cudaError_t expz(const T* a, uint64_t len, const ExpzMasks& M, uint32_t k, const double* norm2, double* partials,
           unsigned int* ticket, double* out, uint32_t blocks, cudaStream_t st) {
-    if (k <= 16) k_expz<T, 1><<<blocks, THREADS, 0, st>>>(a, len, M, k, norm2, partials, ticket, out);
-    else if (k <= 64) k_expz<T, 4><<<blocks, THREADS, 0, st>>>(a, len, M, k, norm2, partials, ticket, out);
-    else k_expz<T, 16><<<blocks, THREADS, 0, st>>>(a, len, M, k, norm2, partials, ticket, out);
+    if (k <= 16) return launch_overlapped(k_expz<T, 1>, blocks, THREADS, 0, st, a, len, M, k, norm2, partials, ticket, out);
+    if (k <= 64) return launch_overlapped(k_expz<T, 4>, blocks, THREADS, 0, st, a, len, M, k, norm2, partials, ticket, out);
+    return launch_overlapped(k_expz<T, 16>, blocks, THREADS, 0, st, a, len, M, k, norm2, partials, ticket, out);
 }
 
 template <typename T>
@@ -204,9 +207,8 @@ cudaError_t launch_expz(const void* a, bool f32, uint64_t len, const ExpzMasks& 
                         double* partials, unsigned int* ticket, double* out, cudaStream_t st) {
     if (k > EXPZ_MASKS) return cudaErrorInvalidValue;
     const uint32_t blocks = expz_blocks(len);
-    if (f32) expz((const float2*)a, len, M, k, norm2, partials, ticket, out, blocks, st);
-    else expz((const double2*)a, len, M, k, norm2, partials, ticket, out, blocks, st);
-    return cudaGetLastError();
+    return f32 ? expz((const float2*)a, len, M, k, norm2, partials, ticket, out, blocks, st)
+               : expz((const double2*)a, len, M, k, norm2, partials, ticket, out, blocks, st);
 }
 
 cudaError_t launch_arena_expz(bool f32, const ExpzJob* jobs, uint32_t njobs, uint32_t chunks, uint32_t max_masks,

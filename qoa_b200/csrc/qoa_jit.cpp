@@ -455,8 +455,8 @@ void emit_head(Emit& E, const PassParams& P, bool c64, bool arena) {
         E.line("const PassParams& P = *reinterpret_cast<const PassParams*>(J.params);");
         E.line("const double nrm = J.fresh ? 0.0 : 1.0;");
     } else {
+        E.line("grid_go();");
         E.line("const uint64_t blk = blockIdx.x;");
-        E.line("const double nrm = *norm2_in;");
     }
     E.line("const uint32_t tw = (uint32_t)lane | ((uint32_t)wid << %d) | ((uint32_t)blk << %d);", LANE_BITS,
            LANE_BITS + WARP_BITS);
@@ -466,6 +466,8 @@ void emit_head(Emit& E, const PassParams& P, bool c64, bool arena) {
     else if (arena)
         E.line("for (uint32_t i = threadIdx.x; i < %uu; i += PASS_THREADS) scoef[i] = P.coef[i];", P.ncoef);
     if (P.nang) E.line("pass_angles(P, blk, sang);");
+    // what the kernel before wrote is read from here on
+    if (!arena) E.line("grid_wait();\nconst double nrm = *norm2_in;");
 }
 
 // The op stream of a complex128 pass (gates, diagonal factors, exchanges
@@ -1234,7 +1236,20 @@ cudaError_t JitKernel::launch(void* amps, const PassParams& P, const double* nor
                                 dim3(PASS_THREADS), args, e_->smem, st);
     }
     void* args[] = {&amps, const_cast<PassParams*>(&P), &norm2_in, &partials};
-    return cudaLaunchKernel(reinterpret_cast<const void*>(e_->kernel), dim3(tiles), dim3(PASS_THREADS), args, 0, st);
+    // overlapped with the end of the kernel before (qoa_launch.cuh), except in a capture
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(tiles);
+    c.blockDim = dim3(PASS_THREADS);
+    c.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone) {
+        c.attrs = at;
+        c.numAttrs = 1;
+    }
+    return cudaLaunchKernelExC(&c, reinterpret_cast<const void*>(e_->kernel), args);
 }
 
 cudaError_t JitKernel::launch_arena(const ArenaJob* jobs, uint32_t njobs, uint32_t lt, cudaStream_t st) const {

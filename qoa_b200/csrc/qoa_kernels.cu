@@ -19,6 +19,7 @@
 #include <string.h>
 
 #include "qoa_kernels.cuh"
+#include "qoa_launch.cuh"
 #include "qoa_pass_dev.cuh"
 
 namespace qoa {
@@ -30,7 +31,8 @@ __device__ __forceinline__ uint64_t tstride(const PassParams& P, uint32_t t) {
 
 // ------------------------------------------------------------ the pass kernel
 // One CTA's tile of one pass. `blk` numbers the tile (its bits go to the
-// qubits outside the tile); `nrm` is the input's squared norm (<= 1e-12: the
+// qubits outside the tile); the input's squared norm is at norm2_in (read after
+// the kernel before has finished) or, where that is null, `nrm` (<= 1e-12: the
 // input is |0..0>, synthesised without reading); `partial_out`, when not
 // null, receives the tile's squared norm after the pass. The pass's
 // coefficients are built in FP64 on the host; a complex64 pass rounds them
@@ -39,7 +41,7 @@ __device__ __forceinline__ uint64_t tstride(const PassParams& P, uint32_t t) {
 // kernel of their own because they spill: in the one kernel they cost every
 // pass 13 % (arena rounds of a batch 3350 against 3794 us).
 template <bool U2, typename T>
-__device__ __forceinline__ void pass_tile(T* __restrict__ amps, const PassParams& P, const double nrm,
+__device__ __forceinline__ void pass_tile(T* __restrict__ amps, const PassParams& P, const double* norm2_in, double nrm,
                                           const uint64_t blk, double* __restrict__ partial_out) {
     using R = typename CT<T>::R;
     extern __shared__ __align__(16) unsigned char pass_smem[];
@@ -73,6 +75,10 @@ __device__ __forceinline__ void pass_tile(T* __restrict__ amps, const PassParams
     __shared__ T sang[MAX_ANG_OPS];
     pass_angles(P, blk, sang);
 
+    if (norm2_in) {
+        grid_wait();
+        nrm = *norm2_in;
+    }
     const bool valid = nrm > 1e-12;
     // The input's 1/||psi|| and the pass's factored global phase are applied
     // once, at the end, as part of the per-thread pending factor.
@@ -297,7 +303,8 @@ template <typename T, bool U2>
 __global__ void __launch_bounds__(PASS_THREADS, PassOcc<T>::value)
 k_pass(T* __restrict__ amps, const __grid_constant__ PassParams P, const double* __restrict__ norm2_in,
        double* __restrict__ partials) {
-    pass_tile<U2, T>(amps, P, *norm2_in, blockIdx.x, partials ? partials + blockIdx.x : nullptr);
+    grid_go();
+    pass_tile<U2, T>(amps, P, norm2_in, 0.0, blockIdx.x, partials ? partials + blockIdx.x : nullptr);
 }
 
 // Arena pass: one launch runs one pass of each of many circuits, whose states
@@ -316,7 +323,7 @@ k_pass_arena(const ArenaJob* __restrict__ jobs, uint32_t njobs, const uint32_t* 
         else hi = mid - 1;
     }
     const ArenaJob J = jobs[lo];
-    pass_tile<U2, T>(reinterpret_cast<T*>(J.amps), *reinterpret_cast<const PassParams*>(J.params),
+    pass_tile<U2, T>(reinterpret_cast<T*>(J.amps), *reinterpret_cast<const PassParams*>(J.params), nullptr,
                  J.fresh ? 0.0 : 1.0, b - tile_start[lo], nullptr);
 }
 
@@ -631,6 +638,8 @@ __device__ __forceinline__ void finish_norm(const double* partials, unsigned int
 template <typename T>
 __global__ void k_norm(const T* __restrict__ a, uint64_t len, double* __restrict__ partials, unsigned int* ticket,
                        double* __restrict__ norm2, uint32_t* __restrict__ status) {
+    grid_go();
+    grid_wait();
     double v[1] = {0.0};
     for (uint64_t i = gtid(); i < len; i += gstride()) v[0] += c_abs2(a[i]);
     block_store_partials<1>(v, partials, gridDim.x);
@@ -641,6 +650,8 @@ __global__ void k_norm(const T* __restrict__ a, uint64_t len, double* __restrict
 // out may be pinned host memory
 __global__ void k_p01(const double2* __restrict__ a, uint64_t len, uint32_t q, double* __restrict__ partials,
                       unsigned int* ticket, const double* __restrict__ norm2, double* __restrict__ out) {
+    grid_go();
+    grid_wait();
     double v[2] = {0.0, 0.0};
     const uint64_t m = 1ull << q;
     for (uint64_t i = gtid(); i < len; i += gstride()) {
@@ -663,6 +674,8 @@ __global__ void k_p01(const double2* __restrict__ a, uint64_t len, uint32_t q, d
 // block per set), then optional scaling by 1/norm2 and status bookkeeping.
 __global__ void k_reduce(const double* __restrict__ partials, uint32_t count, double* __restrict__ out,
                          const double* __restrict__ divide_by, uint32_t* __restrict__ status) {
+    grid_go();
+    grid_wait();
     __shared__ double sh[32];
     const double* p = partials + (uint64_t)blockIdx.x * count;
     // eight independent accumulators per thread keep eight loads in flight
@@ -701,6 +714,8 @@ __global__ void k_reduce(const double* __restrict__ partials, uint32_t count, do
 __global__ void k_collapse(double2* __restrict__ a, uint64_t len, uint32_t q, uint32_t outcome, double f,
                            double* __restrict__ partials, unsigned int* ticket, double* __restrict__ norm2,
                            uint32_t* __restrict__ status) {
+    grid_go();
+    grid_wait();
     double v[1] = {0.0};
     const uint64_t m = 1ull << q;
     for (uint64_t i = gtid(); i < len; i += gstride()) {
@@ -724,6 +739,8 @@ __global__ void k_collapse(double2* __restrict__ a, uint64_t len, uint32_t q, ui
 template <typename T>
 __global__ void k_materialize(T* __restrict__ a, uint64_t len, double* norm2, double* __restrict__ partials,
                               unsigned int* ticket, uint32_t* __restrict__ status, T* __restrict__ copy) {
+    grid_go();
+    grid_wait();
     using R = typename CT<T>::R;
     double v[1] = {0.0};
     const double nrm = *reinterpret_cast<volatile double*>(norm2);
@@ -757,6 +774,8 @@ __global__ void k_init_scalars(double* scal, uint32_t* status) {
 // Probabilities of [off, off+cnt) scaled by 1/norm2 (|0..0> when invalid).
 __global__ void k_probs(const double2* __restrict__ a, uint64_t off, uint64_t cnt, const double* __restrict__ norm2_in,
                         double* __restrict__ out) {
+    grid_go();
+    grid_wait();
     const double nrm = *norm2_in;
     const bool valid = nrm > 1e-12;
     const double inv = valid ? 1.0 / nrm : 0.0;
@@ -783,8 +802,7 @@ static cudaError_t launch_pass_u(double2* amps, const PassParams& P, const doubl
                                          tile_bytes + MAX_PASS_OPS * 16 + MAX_PASS_COEF * (int)sizeof(double2));
     if (e != cudaSuccess) return e;
     const unsigned blocks = 1u << (P.n - TILE_BITS);
-    k_pass<double2, U2><<<blocks, PASS_THREADS, smem, st>>>(amps, P, norm2_in, partials);
-    return cudaGetLastError();
+    return launch_overlapped(k_pass<double2, U2>, blocks, PASS_THREADS, smem, st, amps, P, norm2_in, partials);
 }
 cudaError_t launch_pass(double2* amps, const PassParams& P, const double* norm2_in, double* partials,
                         cudaStream_t st) {
@@ -847,40 +865,38 @@ int reduce_blocks(uint64_t len) { return grid_for(len, 256, 148 * 8); }
 cudaError_t launch_norm(const void* a, bool f32, uint64_t len, double* partials, unsigned int* ticket, double* out,
                         uint32_t* status, cudaStream_t st) {
     const int nb = reduce_blocks(len);
-    if (f32) k_norm<<<nb, 256, 0, st>>>((const float2*)a, len, partials, ticket, out, status);
-    else k_norm<<<nb, 256, 0, st>>>((const double2*)a, len, partials, ticket, out, status);
-    return cudaGetLastError();
+    if (f32) return launch_overlapped(k_norm<float2>, nb, 256, 0, st, (const float2*)a, len, partials, ticket, out, status);
+    return launch_overlapped(k_norm<double2>, nb, 256, 0, st, (const double2*)a, len, partials, ticket, out, status);
 }
 
 cudaError_t launch_p01(const double2* a, uint64_t len, uint32_t q, double* partials, unsigned int* ticket, double* out3,
                        const double* norm2, cudaStream_t st) {
-    k_p01<<<reduce_blocks(len), 256, 0, st>>>(a, len, q, partials, ticket, norm2, out3);
-    return cudaGetLastError();
+    return launch_overlapped(k_p01, reduce_blocks(len), 256, 0, st, a, len, q, partials, ticket, norm2, out3);
 }
 
 cudaError_t launch_reduce_sets(const double* partials, uint32_t count, uint32_t sets, double* out, cudaStream_t st) {
-    k_reduce<<<sets, 1024, 0, st>>>(partials, count, out, nullptr, nullptr);
-    return cudaGetLastError();
+    return launch_overlapped(k_reduce, sets, 1024, 0, st, partials, count, out, nullptr, nullptr);
 }
 
 cudaError_t launch_reduce_partials(const double* partials, uint32_t count, double* out, uint32_t* status,
                                    cudaStream_t st) {
-    k_reduce<<<1, 1024, 0, st>>>(partials, count, out, nullptr, status);
-    return cudaGetLastError();
+    return launch_overlapped(k_reduce, 1, 1024, 0, st, partials, count, out, nullptr, status);
 }
 
 cudaError_t launch_collapse(double2* a, uint64_t len, uint32_t q, uint32_t outcome, double f, double* partials,
                             unsigned int* ticket, double* norm2_out, uint32_t* status, cudaStream_t st) {
-    k_collapse<<<reduce_blocks(len), 256, 0, st>>>(a, len, q, outcome, f, partials, ticket, norm2_out, status);
-    return cudaGetLastError();
+    return launch_overlapped(k_collapse, reduce_blocks(len), 256, 0, st, a, len, q, outcome, f, partials, ticket, norm2_out,
+                             status);
 }
 
 cudaError_t launch_materialize(void* a, bool f32, uint64_t len, double* norm2, double* partials, unsigned int* ticket,
                                uint32_t* status, void* copy, cudaStream_t st) {
     const int nb = reduce_blocks(len);
-    if (f32) k_materialize<<<nb, 256, 0, st>>>((float2*)a, len, norm2, partials, ticket, status, (float2*)copy);
-    else k_materialize<<<nb, 256, 0, st>>>((double2*)a, len, norm2, partials, ticket, status, (double2*)copy);
-    return cudaGetLastError();
+    if (f32)
+        return launch_overlapped(k_materialize<float2>, nb, 256, 0, st, (float2*)a, len, norm2, partials, ticket, status,
+                                 (float2*)copy);
+    return launch_overlapped(k_materialize<double2>, nb, 256, 0, st, (double2*)a, len, norm2, partials, ticket, status,
+                             (double2*)copy);
 }
 
 cudaError_t launch_set_scalar(double* p, double v, cudaStream_t st) {
@@ -895,8 +911,7 @@ cudaError_t launch_init_scalars(double* scal, uint32_t* status, cudaStream_t st)
 
 cudaError_t launch_probs(const double2* a, uint64_t off, uint64_t cnt, const double* norm2, double* out,
                          cudaStream_t st) {
-    k_probs<<<grid_for(cnt, 256, 148 * 16), 256, 0, st>>>(a, off, cnt, norm2, out);
-    return cudaGetLastError();
+    return launch_overlapped(k_probs, grid_for(cnt, 256, 148 * 16), 256, 0, st, a, off, cnt, norm2, out);
 }
 
 }  // namespace qoa

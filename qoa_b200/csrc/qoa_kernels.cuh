@@ -350,4 +350,15 @@ struct GGate {
     double2 m[16];
 };
 
+#if defined(__CUDACC__) || defined(__CUDACC_RTC__)
+// ------------------------------------------- overlap with the kernel before
+// Kernels launched with programmatic stream serialisation (launch_overlapped):
+// grid_go() lets the next such kernel of the stream be placed once every CTA
+// of this one has started; grid_wait() holds a kernel until the one before it
+// has finished and its writes are visible (at once where it was launched
+// plainly). Every thread of an overlapped kernel calls grid_wait().
+__device__ __forceinline__ void grid_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+#endif
+
 }  // namespace qoa

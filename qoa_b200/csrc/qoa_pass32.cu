@@ -14,6 +14,7 @@
 #include <stdint.h>
 
 #include "qoa_kernels.cuh"
+#include "qoa_launch.cuh"
 #include "qoa_pass32_dev.cuh"
 
 namespace qoa {
@@ -28,7 +29,7 @@ __device__ __forceinline__ uint64_t tstride(const PassParams& P, uint32_t t) {
     return 1ull << (t < LANE_BITS ? t : P.slot_qubit[t - LANE_BITS]);
 }
 
-__device__ __forceinline__ void pass_tile_p32(float2* __restrict__ amps, const PassParams& P, const double nrm,
+__device__ __forceinline__ void pass_tile_p32(float2* __restrict__ amps, const PassParams& P, const double* norm2_in, double nrm,
                                               const uint64_t blk, double* __restrict__ partial_out) {
     extern __shared__ __align__(16) unsigned char p32_smem[];
     float2* tile = reinterpret_cast<float2*>(p32_smem);
@@ -61,6 +62,10 @@ __device__ __forceinline__ void pass_tile_p32(float2* __restrict__ amps, const P
         double sn, cs;
         sincos(th, &sn, &cs);
         sang[ai] = make_float2((float)cs, (float)sn);
+    }
+    if (norm2_in) {
+        grid_wait();
+        nrm = *norm2_in;
     }
     const bool valid = nrm > 1e-12;
     float2 pend = valid ? make_float2((float)(P.phase.x / sqrt(nrm)), (float)(P.phase.y / sqrt(nrm)))
@@ -289,7 +294,7 @@ __device__ __forceinline__ void pass_tile_p32(float2* __restrict__ amps, const P
 // every dispatch, condition word and coefficient load serves 32 amplitudes
 // per thread instead of 16. Conditions, angle phases and pending factors are
 // kept per tile.
-__device__ __forceinline__ void pass_tile_p32x2(float2* __restrict__ amps, const PassParams& P, const double nrm,
+__device__ __forceinline__ void pass_tile_p32x2(float2* __restrict__ amps, const PassParams& P, const double* norm2_in,
                                                 const uint64_t blk0, double* __restrict__ partials) {
     extern __shared__ __align__(16) unsigned char p32x2_smem[];
     float2* tile0 = reinterpret_cast<float2*>(p32x2_smem);
@@ -331,6 +336,8 @@ __device__ __forceinline__ void pass_tile_p32x2(float2* __restrict__ amps, const
         sincos(th, &sn, &cs);
         sang[h][ai] = make_float2((float)cs, (float)sn);
     }
+    grid_wait();
+    const double nrm = *norm2_in;
     const bool valid = nrm > 1e-12;
     const float2 pend0 = valid ? make_float2((float)(P.phase.x / sqrt(nrm)), (float)(P.phase.y / sqrt(nrm)))
                                : make_float2((float)P.phase.x, (float)P.phase.y);
@@ -582,7 +589,8 @@ __device__ __forceinline__ void pass_tile_p32x2(float2* __restrict__ amps, const
 __global__ void __launch_bounds__(PASS_THREADS, QOA_PASS_OCC32X2)
 k_pass_p32x2(float2* __restrict__ amps, const __grid_constant__ PassParams P, const double* __restrict__ norm2_in,
              double* __restrict__ partials) {
-    pass_tile_p32x2(amps, P, *norm2_in, blockIdx.x, partials);
+    grid_go();
+    pass_tile_p32x2(amps, P, norm2_in, blockIdx.x, partials);
 }
 
 #ifndef QOA_PASS_OCC32
@@ -592,7 +600,8 @@ k_pass_p32x2(float2* __restrict__ amps, const __grid_constant__ PassParams P, co
 __global__ void __launch_bounds__(PASS_THREADS, QOA_PASS_OCC32)
 k_pass_p32(float2* __restrict__ amps, const __grid_constant__ PassParams P, const double* __restrict__ norm2_in,
            double* __restrict__ partials) {
-    pass_tile_p32(amps, P, *norm2_in, blockIdx.x, partials ? partials + blockIdx.x : nullptr);
+    grid_go();
+    pass_tile_p32(amps, P, norm2_in, 0.0, blockIdx.x, partials ? partials + blockIdx.x : nullptr);
 }
 
 __global__ void __launch_bounds__(PASS_THREADS, QOA_PASS_OCC32)
@@ -605,7 +614,7 @@ k_pass_p32_arena(const ArenaJob* __restrict__ jobs, uint32_t njobs, const uint32
         else h = mid - 1;
     }
     const ArenaJob J = jobs[l];
-    pass_tile_p32(reinterpret_cast<float2*>(J.amps), *reinterpret_cast<const PassParams*>(J.params),
+    pass_tile_p32(reinterpret_cast<float2*>(J.amps), *reinterpret_cast<const PassParams*>(J.params), nullptr,
                   J.fresh ? 0.0 : 1.0, b - tile_start[l], nullptr);
 }
 
@@ -619,16 +628,14 @@ cudaError_t launch_pass_p32(float2* amps, const PassParams& P, const double* nor
         cudaError_t e = cudaFuncSetAttribute(k_pass_p32x2, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              tiles_bytes + MAX_PASS_OPS * 16 + MAX_PASS_COEF * (int)sizeof(float2));
         if (e != cudaSuccess) return e;
-        k_pass_p32x2<<<1u << (P.n - TILE_BITS - 1), PASS_THREADS, smem, st>>>(amps, P, norm2_in, partials);
-        return cudaGetLastError();
+        return launch_overlapped(k_pass_p32x2, 1u << (P.n - TILE_BITS - 1), PASS_THREADS, smem, st, amps, P, norm2_in, partials);
     }
     const int tile_bytes = (1 << TILE_BITS) * (int)sizeof(float2);
     const int smem = tile_bytes + (int)P.nops * 16 + (int)P.ncoef * (int)sizeof(float2);
     cudaError_t e = cudaFuncSetAttribute(k_pass_p32, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          tile_bytes + MAX_PASS_OPS * 16 + MAX_PASS_COEF * (int)sizeof(float2));
     if (e != cudaSuccess) return e;
-    k_pass_p32<<<1u << (P.n - TILE_BITS), PASS_THREADS, smem, st>>>(amps, P, norm2_in, partials);
-    return cudaGetLastError();
+    return launch_overlapped(k_pass_p32, 1u << (P.n - TILE_BITS), PASS_THREADS, smem, st, amps, P, norm2_in, partials);
 }
 
 cudaError_t launch_pass_p32_arena(const ArenaJob* jobs, uint32_t njobs, const uint32_t* tile_start, uint32_t tiles,

@@ -21,6 +21,7 @@
 #include <stdint.h>
 
 #include "qoa_kernels.cuh"
+#include "qoa_launch.cuh"
 #include "qoa_pass_dev.cuh"
 
 namespace qoa {
@@ -65,6 +66,8 @@ __device__ __forceinline__ double fold(const S& s, uint64_t p, uint32_t lo, uint
 template <int B, typename T>
 __global__ void __launch_bounds__(128) k_fold_amps(const T* __restrict__ a, const double* __restrict__ norm2, uint32_t lo,
                                                    double* __restrict__ out) {
+    grid_go();
+    grid_wait();
     const AmpSrc<T> s = amp_src(a, norm2);
     const uint64_t cnt = 1ull << lo;
     for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < cnt; p += (uint64_t)gridDim.x * blockDim.x)
@@ -73,6 +76,8 @@ __global__ void __launch_bounds__(128) k_fold_amps(const T* __restrict__ a, cons
 
 template <int B>
 __global__ void __launch_bounds__(128) k_fold_level(const double* __restrict__ in, uint32_t lo, double* __restrict__ out) {
+    grid_go();
+    grid_wait();
     const uint64_t cnt = 1ull << lo;
     for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < cnt; p += (uint64_t)gridDim.x * blockDim.x)
         out[p] = fold<B, 0, false>(in, p, lo, 0);
@@ -169,6 +174,8 @@ __global__ void __launch_bounds__(128) k_shots(const T* __restrict__ a, uint32_t
                                                const double* __restrict__ tree, const SampleLevels L,
                                                const double* __restrict__ u, uint64_t shots, int mode,
                                                unsigned long long* __restrict__ out) {
+    grid_go();
+    grid_wait();
     const AmpSrc<T> src = amp_src(a, norm2);
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t nw = ((uint64_t)gridDim.x * blockDim.x) >> 5;
@@ -261,49 +268,51 @@ SampleLevels sample_levels(uint32_t n) {
 }
 
 template <typename T>
-static void fold_amps(const T* a, const double* norm2, uint32_t b, uint32_t lo, double* out, cudaStream_t st) {
+static cudaError_t fold_amps(const T* a, const double* norm2, uint32_t b, uint32_t lo, double* out, cudaStream_t st) {
     const int g = fold_grid(lo);
     switch (b) {
-        case 1: k_fold_amps<1, T><<<g, 128, 0, st>>>(a, norm2, lo, out); break;
-        case 2: k_fold_amps<2, T><<<g, 128, 0, st>>>(a, norm2, lo, out); break;
-        case 3: k_fold_amps<3, T><<<g, 128, 0, st>>>(a, norm2, lo, out); break;
-        case 4: k_fold_amps<4, T><<<g, 128, 0, st>>>(a, norm2, lo, out); break;
-        case 5: k_fold_amps<5, T><<<g, 128, 0, st>>>(a, norm2, lo, out); break;
-        default: k_fold_amps<6, T><<<g, 128, 0, st>>>(a, norm2, lo, out); break;
+        case 1: return launch_overlapped(k_fold_amps<1, T>, g, 128, 0, st, a, norm2, lo, out);
+        case 2: return launch_overlapped(k_fold_amps<2, T>, g, 128, 0, st, a, norm2, lo, out);
+        case 3: return launch_overlapped(k_fold_amps<3, T>, g, 128, 0, st, a, norm2, lo, out);
+        case 4: return launch_overlapped(k_fold_amps<4, T>, g, 128, 0, st, a, norm2, lo, out);
+        case 5: return launch_overlapped(k_fold_amps<5, T>, g, 128, 0, st, a, norm2, lo, out);
+        default: return launch_overlapped(k_fold_amps<6, T>, g, 128, 0, st, a, norm2, lo, out);
     }
 }
 
 cudaError_t launch_sample_tree(const void* a, bool f32, uint32_t n, const double* norm2, const SampleLevels& L, double* tree,
                                cudaStream_t st) {
+    cudaError_t e = cudaSuccess;
     for (uint32_t k = 0; k < L.count; ++k) {
         const uint32_t lo = L.bits[k];
         double* out = tree + L.off[k];
         if (k == 0) {
-            if (f32) fold_amps((const float2*)a, norm2, n - lo, lo, out, st);
-            else fold_amps((const double2*)a, norm2, n - lo, lo, out, st);
+            e = f32 ? fold_amps((const float2*)a, norm2, n - lo, lo, out, st)
+                    : fold_amps((const double2*)a, norm2, n - lo, lo, out, st);
+            if (e != cudaSuccess) return e;
             continue;
         }
         const double* in = tree + L.off[k - 1];
         const int g = fold_grid(lo);
         switch (L.bits[k - 1] - lo) {
-            case 1: k_fold_level<1><<<g, 128, 0, st>>>(in, lo, out); break;
-            case 2: k_fold_level<2><<<g, 128, 0, st>>>(in, lo, out); break;
-            case 3: k_fold_level<3><<<g, 128, 0, st>>>(in, lo, out); break;
-            case 4: k_fold_level<4><<<g, 128, 0, st>>>(in, lo, out); break;
-            case 5: k_fold_level<5><<<g, 128, 0, st>>>(in, lo, out); break;
-            default: k_fold_level<6><<<g, 128, 0, st>>>(in, lo, out); break;
+            case 1: e = launch_overlapped(k_fold_level<1>, g, 128, 0, st, in, lo, out); break;
+            case 2: e = launch_overlapped(k_fold_level<2>, g, 128, 0, st, in, lo, out); break;
+            case 3: e = launch_overlapped(k_fold_level<3>, g, 128, 0, st, in, lo, out); break;
+            case 4: e = launch_overlapped(k_fold_level<4>, g, 128, 0, st, in, lo, out); break;
+            case 5: e = launch_overlapped(k_fold_level<5>, g, 128, 0, st, in, lo, out); break;
+            default: e = launch_overlapped(k_fold_level<6>, g, 128, 0, st, in, lo, out); break;
         }
+        if (e != cudaSuccess) return e;
     }
-    return cudaGetLastError();
+    return cudaSuccess;
 }
 
 cudaError_t launch_shots(const void* a, bool f32, uint32_t n, const double* norm2, const double* tree, const SampleLevels& L,
                          const double* u, uint64_t shots, int mode, unsigned long long* out, cudaStream_t st) {
     const uint64_t blocks = (shots + 3) / 4;
     const int g = (int)(blocks < 148 * 16 ? blocks : 148 * 16);
-    if (f32) k_shots<float2><<<g, 128, 0, st>>>((const float2*)a, n, norm2, tree, L, u, shots, mode, out);
-    else k_shots<double2><<<g, 128, 0, st>>>((const double2*)a, n, norm2, tree, L, u, shots, mode, out);
-    return cudaGetLastError();
+    if (f32) return launch_overlapped(k_shots<float2>, g, 128, 0, st, (const float2*)a, n, norm2, tree, L, u, shots, mode, out);
+    return launch_overlapped(k_shots<double2>, g, 128, 0, st, (const double2*)a, n, norm2, tree, L, u, shots, mode, out);
 }
 
 }  // namespace qoa

@@ -25,6 +25,7 @@
 #include <stdint.h>
 
 #include "qoa_kernels.cuh"
+#include "qoa_launch.cuh"
 #include "qoa_pass_dev.cuh"
 
 namespace qoa {
@@ -192,6 +193,8 @@ __global__ void __launch_bounds__(512) k_small_state(T* __restrict__ amps, uint3
     T* s = reinterpret_cast<T*>(small_smem + sizeof(SmallChunk));
     using R = typename CT<T>::R;
     const uint32_t len = 1u << n, slots = len < 8 ? 8 : len;
+    grid_go();
+    grid_wait();
     const double nrm = *norm2_in;
     const bool valid = nrm > 1e-12;
     const R scale = valid ? (R)(1.0 / sqrt(nrm)) : (R)0;
@@ -300,8 +303,7 @@ cudaError_t small_state(T* amps, uint32_t n, const double* norm2_in, const Small
     if (e != cudaSuccess) return e;
     const uint32_t groups = n > 3 ? 1u << (n - 3) : 1u;
     const uint32_t threads = std::min(512u, std::max(32u, groups));
-    k_small_state<T, NC><<<1, threads, small_smem_bytes<T>(n), st>>>(amps, n, norm2_in, P, norm2, status);
-    return cudaGetLastError();
+    return launch_overlapped(k_small_state<T, NC>, 1, threads, small_smem_bytes<T>(n), st, amps, n, norm2_in, P, norm2, status);
 }
 
 }  // namespace
