@@ -1026,25 +1026,39 @@ std::vector<Step> schedule(const std::vector<Gate>& G, uint32_t n, bool per_gate
 // at 20 qubits and 8 % more FP64 work. tb: tile bit of each qubit; pin: the tile bit that is
 // always in a register (complex64 passes), or -1.
 void order_gates(const std::vector<Gate>& G, std::vector<int>& gates, const int* tb_of, int pin) {
-    int tb[64];
-    std::memcpy(tb, tb_of, sizeof tb);
+    // what the scans read of a gate (a Gate is ~350 bytes)
+    struct Scan {
+        uint64_t nmask, dmask;
+        int gate;
+        int8_t t, t2;  // qubits that must be in registers (-1: none)
+        bool swap;
+    };
+    static thread_local std::vector<Scan> scan;
+    static thread_local std::vector<uint16_t> rem, left;
+    int8_t tb[64];
+    for (int q = 0; q < 64; ++q) tb[q] = (int8_t)tb_of[q];
     const size_t ng = gates.size();
-    std::vector<int> out, rem = gates, left;
-    out.reserve(ng);
-    left.reserve(ng);
+    scan.resize(ng);
+    rem.resize(ng);
+    for (size_t i = 0; i < ng; ++i) {
+        const Gate& g = G[gates[i]];
+        const bool two = g.kind == K_U2 || g.kind == K_SWAP;
+        scan[i] = Scan{g.nmask, g.dmask, gates[i], (int8_t)(g.kind == K_G1 || two ? g.t : -1), (int8_t)(two ? g.t2 : -1),
+                       g.kind == K_SWAP};
+        rem[i] = (uint16_t)i;
+    }
     const uint32_t always = pin >= 0 ? 1u << pin : 0u;
-    auto need = [&](const Gate& g) -> uint32_t {
-        if (g.kind == K_G1) return 1u << tb[g.t];
-        if (g.kind == K_U2) return (1u << tb[g.t]) | (1u << tb[g.t2]);
-        return 0u;
+    auto need = [&](const Scan& g) -> uint32_t {
+        if (g.swap || g.t < 0) return 0u;
+        return (1u << tb[g.t]) | (g.t2 >= 0 ? 1u << tb[g.t2] : 0u);
     };
     // the next registers: what the first unblocked gates need (at load, high
     // tile bits only: the lanes hold the low ones)
     auto choose = [&](bool load) {
         uint32_t set = always;
         uint64_t bN = 0, bD = 0;
-        for (int gi : rem) {
-            const Gate& g = G[gi];
+        for (uint16_t i : rem) {
+            const Scan& g = scan[i];
             bool ready = !(g.nmask & (bN | bD)) && !(g.dmask & bN);
             if (ready) {
                 const uint32_t r = set | need(g);
@@ -1058,17 +1072,18 @@ void order_gates(const std::vector<Gate>& G, std::vector<int>& gates, const int*
         }
         return set;
     };
+    size_t done = 0;
     uint32_t regs = choose(true);
     while (true) {
         uint64_t bN = 0, bD = 0;
         left.clear();
-        for (int gi : rem) {
-            const Gate& g = G[gi];
+        for (uint16_t i : rem) {
+            const Scan& g = scan[i];
             if (!(g.nmask & (bN | bD)) && !(g.dmask & bN) && !(need(g) & ~regs)) {
-                out.push_back(gi);
-                if (g.kind == K_SWAP) std::swap(tb[g.t], tb[g.t2]);
+                gates[done++] = g.gate;
+                if (g.swap) std::swap(tb[g.t], tb[g.t2]);
             } else {
-                left.push_back(gi);
+                left.push_back(i);
                 bN |= g.nmask;
                 bD |= g.dmask;
             }
@@ -1077,7 +1092,6 @@ void order_gates(const std::vector<Gate>& G, std::vector<int>& gates, const int*
         if (rem.empty()) break;
         regs = choose(false);
     }
-    gates.swap(out);
 }
 
 // A complex64 pass's coefficients as its kernels read them (coef32).
