@@ -887,6 +887,19 @@ std::vector<Step> schedule_pass_order(const std::vector<Gate>& G, uint32_t n, bo
     std::vector<char> done(N, 0);
     size_t first = 0;
     const bool tiles = !per_gate && n >= (uint32_t)TILE_BITS;
+    // what the scans read of a gate (a Gate is ~350 bytes, and each is looked at in every pass)
+    struct Scan {
+        uint64_t nmask, dmask, need;
+        uint8_t ok, barrier, ncoef, u2;
+    };
+    std::vector<Scan> scan(tiles ? N : 0);
+    for (size_t i = 0; i < scan.size(); ++i) {
+        const Gate& g = G[i];
+        scan[i] = Scan{g.nmask, g.dmask, tile_need(g, f32), (uint8_t)(f32 ? is_pass_gate_f32(g) : is_pass_gate(g, u2)),
+                       (uint8_t)is_barrier(g),
+                       (uint8_t)(g.kind == K_U2 ? 16 : g.kind == K_G1 ? 4 : 2),  // a selector diagonal becomes two phase ops
+                       (uint8_t)(g.kind == K_U2 && !f32)};
+    }
     while (true) {
         while (first < N && done[first]) ++first;
         if (first >= N) break;
@@ -912,21 +925,19 @@ std::vector<Step> schedule_pass_order(const std::vector<Gate>& G, uint32_t n, bo
             int budget_u2 = MAX_XCHG / 2;  // a 4x4 may need an exchange of its own
             for (size_t i = first; i < N; ++i) {
                 if (done[i]) continue;
-                const Gate& g = G[i];
-                if (is_barrier(g)) break;
-                bool ok = (f32 ? is_pass_gate_f32(g) : is_pass_gate(g, u2)) && !(g.nmask & (bN | bD)) && !(g.dmask & bN);
+                const Scan& g = scan[i];
+                if (g.barrier) break;
+                bool ok = g.ok && !(g.nmask & (bN | bD)) && !(g.dmask & bN);
                 if (ok) {
-                    const uint64_t need = tile_need(g, f32) & ~tile;
+                    const uint64_t need = g.need & ~tile;
                     const int k = __builtin_popcountll(need);
-                    const int nc = g.kind == K_U2 ? 16 : g.kind == K_G1 ? 4 : 2;  // a selector diagonal becomes two phase ops
-                    const int u = g.kind == K_U2 && !f32 ? 1 : 0;
-                    if (nslots + k > HIGH_SLOTS || budget_ops < 1 || budget_coef < nc || budget_u2 < u) ok = false;
+                    if (nslots + k > HIGH_SLOTS || budget_ops < 1 || budget_coef < g.ncoef || budget_u2 < g.u2) ok = false;
                     else {
-                        budget_u2 -= u;
                         tile |= need;
                         nslots += k;
                         budget_ops -= 1;
-                        budget_coef -= nc;
+                        budget_coef -= g.ncoef;
+                        budget_u2 -= g.u2;
                     }
                 }
                 if (ok) {
@@ -1448,7 +1459,8 @@ int build_pass(const std::vector<Gate>& G, const Step& st, uint32_t n, PassParam
         // tile bit needed last (the complex64 pass pairs amplitudes along it)
         auto key = [&](uint8_t x) { return x == pin ? (1 << 30) + 1 : (x == must || x == must2 ? -1 : next_use(i, x)); };
         std::stable_sort(nm.reg, nm.reg + REG_BITS, [&](uint8_t x, uint8_t y) { return key(x) < key(y); });
-        if (!getenv("QOA_NO_ORDER_LANES")) order_lanes(nm);
+        static const bool ordered = !getenv("QOA_NO_ORDER_LANES");
+        if (ordered) order_lanes(nm);
         return exchange_to(nm);
     };
     int outer_k[64];  // position of each outer qubit among outer_qubits (-1: in the tile)
@@ -2051,18 +2063,21 @@ void small_program(const std::vector<Gate>& G, size_t begin, size_t end, uint32_
         // gate on one of their qubits, those on none in the thread's factor.
         double2 tab[8];
         uint64_t tab_on = 0;   // register qubits the table depends on
-        const Gate* one = nullptr;  // its only gate
-        auto local = [&](uint64_t mask) {
-            int l = 0;
+        const Gate* one = nullptr;  // its only gate (tab not made yet)
+        auto into_tab = [&](const Gate& g) {
+            int cl = 0;
             for (int j = 0; j < 3; ++j)
-                if ((mask >> qs[j]) & 1) l |= 1 << j;
-            return l;
-        };
-        auto factor = [&](const Gate& g, int v) -> double2 {  // of register index v (conditions and selector in regs)
-            const int cl = local(g.cmask);
-            if ((v & cl) != cl) return d2(1, 0);
-            if (g.neg) return d2(-1, 0);
-            return g.t >= 0 && ((v >> bit_of[g.t]) & 1) ? g.m[1] : g.m[0];
+                if ((g.cmask >> qs[j]) & 1) cl |= 1 << j;
+            const int k = g.t >= 0 ? bit_of[g.t] : 0;
+            for (int v = 0; v < 8; ++v) {
+                if ((v & cl) != cl) continue;
+                const double2 x = tab[v];
+                if (g.neg) tab[v] = d2(-x.x, -x.y);
+                else {
+                    const double2 f = g.t >= 0 && ((v >> k) & 1) ? g.m[1] : g.m[0];
+                    tab[v] = d2(x.x * f.x - x.y * f.y, x.x * f.y + x.y * f.x);
+                }
+            }
         };
         auto flush_tab = [&] {
             if (!tab_on) return;
@@ -2088,11 +2103,16 @@ void small_program(const std::vector<Gate>& G, size_t begin, size_t end, uint32_
             } else if (g.kind == K_DIAG) {
                 const uint64_t on = g.cmask | (g.t >= 0 ? 1ull << g.t : 0);
                 if (!(on & ~regs)) {
-                    for (int v = 0; v < 8; ++v) {
-                        const double2 f = factor(g, v);
-                        tab[v] = tab_on ? d2(tab[v].x * f.x - tab[v].y * f.y, tab[v].x * f.y + tab[v].y * f.x) : f;
+                    if (!tab_on) {
+                        one = &g;
+                    } else {
+                        if (one) {
+                            for (double2& x : tab) x = d2(1, 0);
+                            into_tab(*one);
+                            one = nullptr;
+                        }
+                        into_tab(g);
                     }
-                    one = tab_on ? nullptr : &g;
                     tab_on |= on;
                 } else if (!(on & regs)) {
                     if (g.neg) emit(SO_PNEG, 0, g.cmask, nullptr, 0);

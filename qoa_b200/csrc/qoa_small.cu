@@ -194,6 +194,7 @@ __global__ void __launch_bounds__(512) k_small_state(T* __restrict__ amps, uint3
     using R = typename CT<T>::R;
     const uint32_t len = 1u << n, slots = len < 8 ? 8 : len;
     grid_go();
+    small_stage(c, P.ref[0], P.ops, P.coef);  // while the kernel before finishes
     grid_wait();
     const double nrm = *norm2_in;
     const bool valid = nrm > 1e-12;
@@ -206,8 +207,9 @@ __global__ void __launch_bounds__(512) k_small_state(T* __restrict__ amps, uint3
         }
         s[small_pos(i)] = x;
     }
+    __syncthreads();
     for (uint32_t k = 0; k < P.nchunks; ++k) {
-        small_stage(c, P.ref[k], P.ops, P.coef);
+        if (k) small_stage(c, P.ref[k], P.ops, P.coef);
         small_sweeps(s, n, c, P.ref[k].nops);
     }
     double ss = 0.0;
