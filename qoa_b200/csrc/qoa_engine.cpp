@@ -444,6 +444,14 @@ int alloc_state(qoa_state_t s, uint32_t n) {
     return QOA_OK;
 }
 
+// Allocations of a synchronous call while it lives: they stay allowed while
+// another thread captures a graph in the global mode, as pool allocations are.
+struct AllocWhileCapturing {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    AllocWhileCapturing() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~AllocWhileCapturing() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
 // Pinned host buffers for the results (and uniforms) of synchronous calls, one
 // for the length of a call: a copy between device and pageable memory is
 // staged by the driver piece by piece, and small results need no copy at all
@@ -452,7 +460,8 @@ int alloc_state(qoa_state_t s, uint32_t n) {
 constexpr size_t kStagingBytes = size_t(1) << 20;
 constexpr size_t kStagingKept = 8;
 std::mutex g_staging_mu;
-std::vector<void*> g_staging;
+void* g_staging[kStagingKept];  // the first g_staging_n are free buffers
+size_t g_staging_n = 0;
 class Staging {
 public:
     // null where the call needs more than a buffer holds, or none can be had
@@ -460,12 +469,12 @@ public:
         if (!bytes || bytes > kStagingBytes) return;
         {
             std::lock_guard<std::mutex> lk(g_staging_mu);
-            if (!g_staging.empty()) {
-                p_ = g_staging.back();
-                g_staging.pop_back();
+            if (g_staging_n) {
+                p_ = g_staging[--g_staging_n];
                 return;
             }
         }
+        AllocWhileCapturing relaxed;
         if (cudaHostAlloc(&p_, kStagingBytes, cudaHostAllocPortable) != cudaSuccess) {
             cudaGetLastError();
             p_ = nullptr;
@@ -476,11 +485,12 @@ public:
         if (!done_) cudaStreamSynchronize(st_);  // an error on the way: work may still use the buffer
         {
             std::lock_guard<std::mutex> lk(g_staging_mu);
-            if (g_staging.size() < kStagingKept) {
-                g_staging.push_back(p_);
+            if (g_staging_n < kStagingKept) {
+                g_staging[g_staging_n++] = p_;
                 return;
             }
         }
+        AllocWhileCapturing relaxed;
         cudaFreeHost(p_);
     }
     Staging(const Staging&) = delete;
@@ -504,6 +514,7 @@ constexpr size_t kDirectBytes = 64 << 10;
 constexpr size_t kWorkspaceKept = size_t(256) << 20;
 int workspace(qoa_state_t s, size_t bytes, double** out) {
     if (bytes > s->ws_cap) {
+        AllocWhileCapturing relaxed;
         if (s->ws) cudaFree(s->ws);
         s->ws = nullptr;
         s->ws_cap = 0;
@@ -515,6 +526,7 @@ int workspace(qoa_state_t s, size_t bytes, double** out) {
 }
 int workspace_done(qoa_state_t s) {
     if (s->ws_cap > kWorkspaceKept) {
+        AllocWhileCapturing relaxed;
         cudaFree(s->ws);
         s->ws = nullptr;
         s->ws_cap = 0;

@@ -89,8 +89,8 @@ __device__ __forceinline__ double sum16(double x) {
 // finishes last (ticket returns to 0 by itself), divided by norm2.
 template <typename T, int MI>
 __global__ void __launch_bounds__(THREADS, MI <= 4 ? 4 : 2)
-k_expz(const T* __restrict__ a, uint64_t len, const __grid_constant__ ExpzMasks M, uint32_t k,
-       const double* __restrict__ norm2, double* __restrict__ partials, unsigned int* __restrict__ ticket,
+k_expz(const T* a, uint64_t len, const __grid_constant__ ExpzMasks M, uint32_t k,
+       const double* norm2, double* __restrict__ partials, unsigned int* __restrict__ ticket,
        double* __restrict__ out) {
     grid_go();
     grid_wait();

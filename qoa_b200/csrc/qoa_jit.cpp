@@ -467,7 +467,7 @@ void emit_head(Emit& E, const PassParams& P, bool c64, bool arena) {
         E.line("for (uint32_t i = threadIdx.x; i < %uu; i += PASS_THREADS) scoef[i] = P.coef[i];", P.ncoef);
     if (P.nang) E.line("pass_angles(P, blk, sang);");
     // what the kernel before wrote is read from here on
-    if (!arena) E.line("grid_wait();\nconst double nrm = *norm2_in;");
+    if (!arena) E.line("grid_wait();\nconst double nrm = read_after_wait(norm2_in);");
 }
 
 // The op stream of a complex128 pass (gates, diagonal factors, exchanges

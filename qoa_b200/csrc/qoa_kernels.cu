@@ -77,7 +77,7 @@ __device__ __forceinline__ void pass_tile(T* __restrict__ amps, const PassParams
 
     if (norm2_in) {
         grid_wait();
-        nrm = *norm2_in;
+        nrm = read_after_wait(norm2_in);
     }
     const bool valid = nrm > 1e-12;
     // The input's 1/||psi|| and the pass's factored global phase are applied
@@ -636,7 +636,7 @@ __device__ __forceinline__ void finish_norm(const double* partials, unsigned int
 
 // sum |a|^2: partial sums per CTA, added by the last one
 template <typename T>
-__global__ void k_norm(const T* __restrict__ a, uint64_t len, double* __restrict__ partials, unsigned int* ticket,
+__global__ void k_norm(const T* a, uint64_t len, double* __restrict__ partials, unsigned int* ticket,
                        double* __restrict__ norm2, uint32_t* __restrict__ status) {
     grid_go();
     grid_wait();
@@ -648,8 +648,8 @@ __global__ void k_norm(const T* __restrict__ a, uint64_t len, double* __restrict
 
 // norm2, P(bit q = 0), P(bit q = 1) of the stored vector, divided by norm2 (null: 1);
 // out may be pinned host memory
-__global__ void k_p01(const double2* __restrict__ a, uint64_t len, uint32_t q, double* __restrict__ partials,
-                      unsigned int* ticket, const double* __restrict__ norm2, double* __restrict__ out) {
+__global__ void k_p01(const double2* a, uint64_t len, uint32_t q, double* __restrict__ partials,
+                      unsigned int* ticket, const double* norm2, double* __restrict__ out) {
     grid_go();
     grid_wait();
     double v[2] = {0.0, 0.0};
@@ -672,8 +672,8 @@ __global__ void k_p01(const double2* __restrict__ a, uint64_t len, uint32_t q, d
 
 // Final reduction: out[s] = sum_k partials[s*count + k] in a fixed order (one
 // block per set), then optional scaling by 1/norm2 and status bookkeeping.
-__global__ void k_reduce(const double* __restrict__ partials, uint32_t count, double* __restrict__ out,
-                         const double* __restrict__ divide_by, uint32_t* __restrict__ status) {
+__global__ void k_reduce(const double* partials, uint32_t count, double* __restrict__ out,
+                         const double* divide_by, uint32_t* __restrict__ status) {
     grid_go();
     grid_wait();
     __shared__ double sh[32];
@@ -772,11 +772,11 @@ __global__ void k_init_scalars(double* scal, uint32_t* status) {
 }
 
 // Probabilities of [off, off+cnt) scaled by 1/norm2 (|0..0> when invalid).
-__global__ void k_probs(const double2* __restrict__ a, uint64_t off, uint64_t cnt, const double* __restrict__ norm2_in,
+__global__ void k_probs(const double2* a, uint64_t off, uint64_t cnt, const double* norm2_in,
                         double* __restrict__ out) {
     grid_go();
     grid_wait();
-    const double nrm = *norm2_in;
+    const double nrm = read_after_wait(norm2_in);
     const bool valid = nrm > 1e-12;
     const double inv = valid ? 1.0 / nrm : 0.0;
     for (uint64_t i = gtid(); i < cnt; i += gstride()) {

@@ -356,9 +356,13 @@ struct GGate {
 // grid_go() lets the next such kernel of the stream be placed once every CTA
 // of this one has started; grid_wait() holds a kernel until the one before it
 // has finished and its writes are visible (at once where it was launched
-// plainly). Every thread of an overlapped kernel calls grid_wait().
+// plainly). Every thread of an overlapped kernel calls grid_wait(). A scalar that
+// the kernel before wrote is read by read_after_wait(), and arrays through
+// pointers that are not `const __restrict__`: a load that the compiler takes for
+// a read-only one may be moved above the wait.
 __device__ __forceinline__ void grid_go() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ double read_after_wait(const double* p) { return *(const volatile double*)p; }
 #endif
 
 }  // namespace qoa

@@ -65,7 +65,7 @@ __device__ __forceinline__ void pass_tile_p32(float2* __restrict__ amps, const P
     }
     if (norm2_in) {
         grid_wait();
-        nrm = *norm2_in;
+        nrm = read_after_wait(norm2_in);
     }
     const bool valid = nrm > 1e-12;
     float2 pend = valid ? make_float2((float)(P.phase.x / sqrt(nrm)), (float)(P.phase.y / sqrt(nrm)))
@@ -337,7 +337,7 @@ __device__ __forceinline__ void pass_tile_p32x2(float2* __restrict__ amps, const
         sang[h][ai] = make_float2((float)cs, (float)sn);
     }
     grid_wait();
-    const double nrm = *norm2_in;
+    const double nrm = read_after_wait(norm2_in);
     const bool valid = nrm > 1e-12;
     const float2 pend0 = valid ? make_float2((float)(P.phase.x / sqrt(nrm)), (float)(P.phase.y / sqrt(nrm)))
                                : make_float2((float)P.phase.x, (float)P.phase.y);

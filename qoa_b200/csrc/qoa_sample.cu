@@ -43,7 +43,7 @@ struct AmpSrc {
 
 template <typename T>
 __device__ __forceinline__ AmpSrc<T> amp_src(const T* a, const double* norm2) {
-    const double nrm = *norm2;
+    const double nrm = read_after_wait(norm2);
     const bool valid = nrm > 1e-12;
     return AmpSrc<T>{a, valid ? 1.0 / nrm : 1.0, valid};
 }
@@ -64,7 +64,7 @@ __device__ __forceinline__ double fold(const S& s, uint64_t p, uint32_t lo, uint
 }
 
 template <int B, typename T>
-__global__ void __launch_bounds__(128) k_fold_amps(const T* __restrict__ a, const double* __restrict__ norm2, uint32_t lo,
+__global__ void __launch_bounds__(128) k_fold_amps(const T* a, const double* norm2, uint32_t lo,
                                                    double* __restrict__ out) {
     grid_go();
     grid_wait();
@@ -75,7 +75,7 @@ __global__ void __launch_bounds__(128) k_fold_amps(const T* __restrict__ a, cons
 }
 
 template <int B>
-__global__ void __launch_bounds__(128) k_fold_level(const double* __restrict__ in, uint32_t lo, double* __restrict__ out) {
+__global__ void __launch_bounds__(128) k_fold_level(const double* in, uint32_t lo, double* __restrict__ out) {
     grid_go();
     grid_wait();
     const uint64_t cnt = 1ull << lo;
@@ -170,8 +170,8 @@ struct WarpTree {
 // |0..0>, so every later outcome is 0 (quantum_state.rs:424-455, 888-907).
 // mode 1: inverse CDF with one uniform per shot, walking the same tree.
 template <typename T>
-__global__ void __launch_bounds__(128) k_shots(const T* __restrict__ a, uint32_t n, const double* __restrict__ norm2,
-                                               const double* __restrict__ tree, const SampleLevels L,
+__global__ void __launch_bounds__(128) k_shots(const T* a, uint32_t n, const double* norm2,
+                                               const double* tree, const SampleLevels L,
                                                const double* __restrict__ u, uint64_t shots, int mode,
                                                unsigned long long* __restrict__ out) {
     grid_go();

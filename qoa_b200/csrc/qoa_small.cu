@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(512) k_small_state(T* __restrict__ amps, uint3
     grid_go();
     small_stage(c, P.ref[0], P.ops, P.coef);  // while the kernel before finishes
     grid_wait();
-    const double nrm = *norm2_in;
+    const double nrm = read_after_wait(norm2_in);
     const bool valid = nrm > 1e-12;
     const R scale = valid ? (R)(1.0 / sqrt(nrm)) : (R)0;
     for (uint32_t i = threadIdx.x; i < slots; i += blockDim.x) {
