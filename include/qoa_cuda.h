@@ -234,8 +234,9 @@ typedef struct qoa_batch_tuning {
     uint32_t pass_gate_budget;  /* max gates per tile pass (fusion width); 0 = default */
     uint32_t f32_tensor;        /* complex64 batches: 1 = dense tensor-core blocks, 0 = tile passes */
     uint32_t jit;               /* tile passes as generated kernels, one per pass structure:
-                                   QOA_JIT_OFF, QOA_JIT_ASYNC (default: compiled in the background,
-                                   the graph is captured again once they are loaded), QOA_JIT_SYNC */
+                                   QOA_JIT_OFF, QOA_JIT_ASYNC (default: structures of >= 8 passes or
+                                   >= 512 tiles compiled in the background, the graph is captured
+                                   again once they are loaded), QOA_JIT_SYNC (all, before the run) */
 } qoa_batch_tuning;
 int qoa_batch_create(int precision, uint32_t flags, qoa_batch_t* out);
 int qoa_batch_add(qoa_batch_t b, uint32_t n, const qoa_op* ops, size_t nops, const uint64_t* zmasks, size_t nmasks,
