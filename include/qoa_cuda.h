@@ -228,7 +228,8 @@ const char* qoa_strerror(int code);
 typedef struct qoa_batch_s* qoa_batch_t;
 typedef struct qoa_batch_tuning {
     uint32_t small_max_n;       /* shared-memory kernel up to this many qubits */
-    uint32_t small_threads;     /* threads per CTA of that kernel (multiple of 32) */
+    uint32_t small_threads;     /* threads per CTA of that kernel (multiple of 32 up to 1024; as many
+                                   of them run as the kernel's registers allow) */
     uint32_t small_ctas_per_sm; /* its persistent grid = SMs x this */
     uint32_t streams;           /* streams the larger circuits spread over */
     uint32_t pass_gate_budget;  /* max gates per tile pass (fusion width); 0 = default */

@@ -332,7 +332,14 @@ cudaError_t launch_small_batch(bool f32, const SmallCircuit* circs, uint32_t cou
     // setting made between another thread's set-up and launch fails that launch
     const size_t smem_cap = f32 ? small_smem_bytes<float2>(SMALL_MAX_F32) : small_smem_bytes<double2>(SMALL_MAX_F64);
     if (smem > smem_cap) return cudaErrorInvalidValue;
-    cudaError_t e;
+    // The tuning takes blocks of up to 1024 threads, the registers of a sweep
+    // fewer (100 a thread in complex128: 640 do not fit); the loops stride by the block.
+    // A launch bound instead would change the code for every block (512: 79 ->
+    // 107 registers in complex64).
+    cudaFuncAttributes fa;
+    cudaError_t e = f32 ? cudaFuncGetAttributes(&fa, k_small_batch<float2>) : cudaFuncGetAttributes(&fa, k_small_batch<double2>);
+    if (e != cudaSuccess) return e;
+    threads = std::min(threads, fa.maxThreadsPerBlock & ~31);
     if (f32) e = cudaFuncSetAttribute(k_small_batch<float2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cap);
     else e = cudaFuncSetAttribute(k_small_batch<double2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cap);
     if (e != cudaSuccess) return e;
