@@ -403,8 +403,12 @@ int qoa_get_precision(qoa_state_t s, int* precision);
 /* ---- plan introspection (host only, no GPU needed) ---------------------- */
 /* Runs the pass scheduler on an op list for an n-qubit state and writes, for
  * each expanded gate in submission order, the index of the pass that applies
- * it (pass_of[i]) and the order within the pass (order[i]); *npasses receives
- * the pass count and *ngates the expanded gate count (<= cap). */
+ * it (pass_of[i]) and an order within the pass that gives the same result
+ * (order[i]; the pass's kernel may order commuting gates differently);
+ * *npasses receives the pass count and *ngates the expanded gate count (<=
+ * cap). The plan is that of a complex128 handle, except that a block of SWAPs
+ * stays separate gates. From 11 qubits on (without QOA_FLAG_PER_GATE) a
+ * controlled SWAP is three gates: CNOT, Toffoli, CNOT. */
 /* Plans with the scheduler's slot search at any size (states of 26 or more
  * qubits always plan with it); for tests of the plans. */
 #define QOA_PLAN_SLOT_SEARCH 0x100u

@@ -813,8 +813,8 @@ struct Expander {
 };
 
 // -------------------------------------------------------------- scheduler
-// A step is either a tile pass (a set of K_G1 / K_DIAG gates) or a single
-// gate that runs on its own kernel (SWAP, U2, barriers).
+// A step is either a tile pass (a set of the gates is_pass_gate takes) or a single
+// gate that runs on its own kernel (in complex64 a 4x4; a SWAP block; barriers).
 struct Step {
     bool pass = false;
     std::vector<int> gates;        // indices into the gate list, in application order
@@ -2541,6 +2541,17 @@ void split_controlled_swaps(std::vector<Gate>& G) {
     G.swap(out);
 }
 
+// An op list as a handle runs it in tile passes: its gates put into the forms
+// that passes take, and its steps. qoa_plan and qoa_jit_translate report, and
+// batches run, the same.
+void prepare_gates(std::vector<Gate>& G, bool swap_blocks) {
+    if (swap_blocks) merge_swap_blocks(G);
+    split_controlled_swaps(G);
+}
+std::vector<Step> plan_steps(const std::vector<Gate>& G, uint32_t n, bool per_gate, bool c64, int gate_budget, bool search) {
+    return schedule(G, n, per_gate, false, gate_budget, search, !c64);
+}
+
 int run_perm(qoa_state_t s, const Gate& g) {
     const uint32_t n = s->n;
     PermParams P;
@@ -2647,10 +2658,7 @@ int run_small_list(qoa_state_t s, const std::vector<Gate>& seg, bool& reset_owed
 int run_planned(qoa_state_t s, std::vector<Gate>& seg, bool& reset_owed) {
     const bool c64 = s->precision == QOA_PREC_F32;
     const bool per_gate = (s->flags & QOA_FLAG_PER_GATE) != 0;
-    if (!per_gate) {
-        merge_swap_blocks(seg);
-        split_controlled_swaps(seg);
-    }
+    if (!per_gate) prepare_gates(seg, true);
     const bool jit = !per_gate && s->jit_mode != QOA_JIT_OFF && s->n >= s->jit_min_qubits;
     // a repeated op list reuses its plan
     PlanEntry local;
@@ -2673,8 +2681,8 @@ int run_planned(qoa_state_t s, std::vector<Gate>& seg, bool& reset_owed) {
     if (fresh) {
         // the plan depends on the op list and the size only, so a list
         // executed again gives bit-identical results
-        pe->steps = schedule(seg, s->n, per_gate, false, state_pass_budget(s),
-                             slot_search_pays(s->n) || (s->flags & QOA_FLAG_SLOT_SEARCH), !c64);
+        pe->steps = plan_steps(seg, s->n, per_gate, c64, state_pass_budget(s),
+                               slot_search_pays(s->n) || (s->flags & QOA_FLAG_SLOT_SEARCH));
         pe->built_of.assign(pe->steps.size(), -1);
         // passes built ahead: for generated kernels, whose text is
         // requested from the compile cache, and for a plan that is kept
@@ -3193,8 +3201,8 @@ int batch_prepare(qoa_batch_t b) {
         parallel_for(cands.size(), [&](size_t x) {
             const size_t i = cands[x];
             auto& c = b->circs[i];
-            split_controlled_swaps(c.gates);
-            steps_of[i] = schedule(c.gates, c.n, false, false, budget, false, !f32);
+            prepare_gates(c.gates, false);
+            steps_of[i] = plan_steps(c.gates, c.n, false, f32, budget, false);
             bool ok = true;
             for (const Step& st : steps_of[i]) ok = ok && st.pass;
             all_pass[i] = ok;
@@ -4044,11 +4052,12 @@ int qoa_plan(uint32_t n, uint32_t flags, const qoa_op* ops, size_t nops, size_t 
         ex.cur = (int)i;
         ex.op(ops[i]);
     }
-    const std::vector<Gate>& G = ex.out;
+    std::vector<Gate>& G = ex.out;
     for (const Gate& g : G)
         if (g.kind == K_QINIT) return set_err(nullptr, QOA_E_ARG, "qoa_plan does not take QINIT");
-    std::vector<Step> steps = schedule(G, ex.n, (flags & QOA_FLAG_PER_GATE) != 0, false, 0,
-                                       slot_search_pays(ex.n) || (flags & QOA_PLAN_SLOT_SEARCH));
+    const bool per_gate = (flags & QOA_FLAG_PER_GATE) != 0;
+    if (!per_gate && ex.n >= (uint32_t)TILE_BITS) prepare_gates(G, false);
+    std::vector<Step> steps = plan_steps(G, ex.n, per_gate, false, 0, slot_search_pays(ex.n) || (flags & QOA_PLAN_SLOT_SEARCH));
     *ngates = G.size();
     *npasses = steps.size();
     if (G.size() > cap) return set_err(nullptr, QOA_E_ARG, "cap too small: %zu gates", G.size());
@@ -4589,8 +4598,8 @@ int qoa_jit_translate(uint32_t n, int precision, uint32_t flags, const qoa_op* o
     std::vector<Gate>& G = ex.out;
     for (const Gate& g : G)
         if (g.kind == K_QINIT) return set_err(nullptr, QOA_E_ARG, "qoa_jit_translate does not take QINIT");
-    merge_swap_blocks(G);
-    std::vector<Step> steps = schedule(G, n, false, false, 0, slot_search_pays(n));
+    prepare_gates(G, true);
+    std::vector<Step> steps = plan_steps(G, n, false, precision == QOA_PREC_F32, 0, slot_search_pays(n));
     std::vector<std::string> bodies;
     static thread_local PassParams P;
     for (const Step& st : steps) {
