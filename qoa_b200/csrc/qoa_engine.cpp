@@ -315,8 +315,9 @@ struct qoa_state_s {
     uint32_t* status = nullptr;   // device status words
     double* partials = nullptr;
     size_t partials_cap = 0;
-    double* ws = nullptr;         // scratch kept between calls (workspace)
+    double* ws = nullptr;         // scratch kept between calls (Workspace)
     size_t ws_cap = 0;
+    bool ws_busy = false;         // a call uses it (g_ws_mu)
     double* host_scal = nullptr;  // pinned: mirror of scal, then EXPZ_MASKS results (kernels write them there)
     uint64_t seed = 0;
     uint64_t noise_stream = 0;
@@ -423,12 +424,53 @@ void trim_batch_pools() {
         if (p) cudaMemPoolTrimTo(p, 0);
 }
 
-// cudaMalloc, retried once after trimming the batch pools
+// Allocations of a synchronous call while it lives: they stay allowed while
+// another thread captures a graph in the global mode, as pool allocations are.
+struct AllocWhileCapturing {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    AllocWhileCapturing() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~AllocWhileCapturing() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// The handles that keep scratch (Workspace), and the bytes of all of it.
+// (never destroyed: a handle may be closed while the process exits)
+std::mutex g_ws_mu;
+std::vector<qoa_state_t>& g_ws_owners = *new std::vector<qoa_state_t>;
+size_t g_ws_total = 0;
+
+// Takes a handle's kept scratch out of the books (g_ws_mu held); the caller frees it.
+double* forget(qoa_state_t s) {
+    double* p = s->ws;
+    if (!p) return nullptr;
+    s->ws = nullptr;
+    g_ws_total -= s->ws_cap;
+    s->ws_cap = 0;
+    g_ws_owners.erase(std::find(g_ws_owners.begin(), g_ws_owners.end(), s));
+    return p;
+}
+
+// Frees the scratch that handles on the current device keep and no call uses.
+void drop_idle_workspaces() {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    std::vector<double*> drop;
+    {
+        std::lock_guard<std::mutex> lk(g_ws_mu);
+        const std::vector<qoa_state_t> owners = g_ws_owners;
+        for (qoa_state_t s : owners)
+            if (s->device == dev && !s->ws_busy) drop.push_back(forget(s));
+    }
+    AllocWhileCapturing relaxed;
+    for (double* p : drop) cudaFree(p);
+}
+
+// cudaMalloc, retried once after giving back what batches and handles keep
 cudaError_t device_alloc(void** p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes);
     if (e == cudaErrorMemoryAllocation) {
         cudaGetLastError();
         trim_batch_pools();
+        drop_idle_workspaces();
         e = cudaMalloc(p, bytes);
     }
     return e;
@@ -443,14 +485,6 @@ int alloc_state(qoa_state_t s, uint32_t n) {
     CK(device_alloc((void**)&s->partials, s->partials_cap * sizeof(double)));
     return QOA_OK;
 }
-
-// Allocations of a synchronous call while it lives: they stay allowed while
-// another thread captures a graph in the global mode, as pool allocations are.
-struct AllocWhileCapturing {
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    AllocWhileCapturing() { cudaThreadExchangeStreamCaptureMode(&mode); }
-    ~AllocWhileCapturing() { cudaThreadExchangeStreamCaptureMode(&mode); }
-};
 
 // Pinned host buffers for the results (and uniforms) of synchronous calls, one
 // for the length of a call: a copy between device and pageable memory is
@@ -507,32 +541,55 @@ private:
 // above it a copy is faster than their stores over the bus.
 constexpr size_t kDirectBytes = 64 << 10;
 
-// Scratch of a synchronous call (sampling, probabilities) on the handle's
-// stream, kept by the handle up to kWorkspaceKept bytes: a buffer allocated
-// per call is mapped and unmapped each time (0.9 to 3 ms per GB). Larger
-// ones are freed by workspace_done.
+// Scratch of a synchronous call (sampling, probabilities, expectation values)
+// on the handle's stream, for the call's length. The handle keeps the buffer
+// up to kWorkspaceKept bytes, and all handles together up to
+// kWorkspaceKeptTotal: one allocated per call is mapped and unmapped each time
+// (0.9 to 3 ms per GB). An allocation that finds the device full takes back
+// the buffers that no call uses (drop_idle_workspaces).
 constexpr size_t kWorkspaceKept = size_t(256) << 20;
-int workspace(qoa_state_t s, size_t bytes, double** out) {
-    if (bytes > s->ws_cap) {
+constexpr size_t kWorkspaceKeptTotal = size_t(1) << 30;
+class Workspace {
+public:
+    Workspace(qoa_state_t s, size_t bytes) : s_(s) {
+        double* old = nullptr;
+        {
+            std::lock_guard<std::mutex> lk(g_ws_mu);
+            s->ws_busy = true;
+            if (bytes <= s->ws_cap) return;
+            old = forget(s);
+        }
         AllocWhileCapturing relaxed;
-        if (s->ws) cudaFree(s->ws);
-        s->ws = nullptr;
-        s->ws_cap = 0;
-        CK(device_alloc((void**)&s->ws, bytes));
+        if (old) cudaFree(old);
+        double* p = nullptr;
+        e_ = device_alloc((void**)&p, bytes);
+        if (e_ != cudaSuccess) return;
+        std::lock_guard<std::mutex> lk(g_ws_mu);
+        s->ws = p;
         s->ws_cap = bytes;
+        g_ws_total += bytes;
+        g_ws_owners.push_back(s);
     }
-    *out = s->ws;
-    return QOA_OK;
-}
-int workspace_done(qoa_state_t s) {
-    if (s->ws_cap > kWorkspaceKept) {
+    ~Workspace() {
+        double* drop = nullptr;
+        {
+            std::lock_guard<std::mutex> lk(g_ws_mu);
+            s_->ws_busy = false;
+            if (s_->ws_cap > kWorkspaceKept || (s_->ws && g_ws_total > kWorkspaceKeptTotal)) drop = forget(s_);
+        }
+        if (!drop) return;
         AllocWhileCapturing relaxed;
-        cudaFree(s->ws);
-        s->ws = nullptr;
-        s->ws_cap = 0;
+        cudaFree(drop);
     }
-    return QOA_OK;
-}
+    Workspace(const Workspace&) = delete;
+    Workspace& operator=(const Workspace&) = delete;
+    cudaError_t error() const { return e_; }
+    double* get() const { return s_->ws; }
+
+private:
+    qoa_state_t s_;
+    cudaError_t e_ = cudaSuccess;
+};
 
 struct Timer {
     qoa_state_t s;
@@ -2437,7 +2494,7 @@ int f32_prepare(qoa_state_t s, std::vector<Gate>& G) {
     if (total > s->f32_mats_cap) {
         if (s->f32_mats) cudaFree(s->f32_mats);
         s->f32_mats = nullptr;
-        CK(cudaMalloc(&s->f32_mats, total));
+        CK(device_alloc(&s->f32_mats, total));
         s->f32_mats_cap = total;
     }
     CK(cudaMemcpy(s->f32_mats, host.data(), total, cudaMemcpyHostToDevice));
@@ -2810,9 +2867,9 @@ int shim_begin(double* amps, size_t len, double2** dev) {
         if (g_shim_buf) cudaFree(g_shim_buf);
         if (g_shim_scr) cudaFree(g_shim_scr);
         g_shim_buf = nullptr; g_shim_scr = nullptr; g_shim_cap = 0;
-        CK(cudaMalloc(&g_shim_buf, len * sizeof(double2)));
+        CK(device_alloc((void**)&g_shim_buf, len * sizeof(double2)));
         // results, the ticket word (0 between launches), then partial sums
-        CK(cudaMalloc(&g_shim_scr, (size_t)(2 * reduce_blocks(len) + 8) * sizeof(double)));
+        CK(device_alloc((void**)&g_shim_scr, (size_t)(2 * reduce_blocks(len) + 8) * sizeof(double)));
         CK(cudaMemsetAsync(g_shim_scr, 0, 8 * sizeof(double), g_shim_stream));
         g_shim_cap = len;
     }
@@ -3041,6 +3098,7 @@ cudaError_t dalloc(qoa_batch_t b, T*& dst, size_t bytes) {
     if (e == cudaErrorMemoryAllocation && pool) {  // memory held elsewhere: retry once after a trim
         cudaGetLastError();
         trim_batch_pools();
+        drop_idle_workspaces();
         e = cudaMallocFromPoolAsync(&p, bytes, pool, b->streams[0]);
     }
     dst = static_cast<T*>(p);
@@ -3717,8 +3775,8 @@ int qoa_create(uint32_t n, int precision, uint32_t flags, qoa_state_t* out) {
     };
     if (cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking) != cudaSuccess)
         return fail(set_err(s, QOA_E_CUDA, "stream create failed"));
-    if (cudaMalloc(&s->scal, SCAL_DOUBLES * sizeof(double)) != cudaSuccess) return fail(set_err(s, QOA_E_OOM, "scalar alloc"));
-    if (cudaMalloc(&s->status, 4 * sizeof(uint32_t)) != cudaSuccess) return fail(set_err(s, QOA_E_OOM, "status alloc"));
+    if (device_alloc((void**)&s->scal, SCAL_DOUBLES * sizeof(double)) != cudaSuccess) return fail(set_err(s, QOA_E_OOM, "scalar alloc"));
+    if (device_alloc((void**)&s->status, 4 * sizeof(uint32_t)) != cudaSuccess) return fail(set_err(s, QOA_E_OOM, "status alloc"));
     if (launch_init_scalars(s->scal, s->status, s->stream) != cudaSuccess)
         return fail(set_err(s, QOA_E_CUDA, "scalar set-up"));
     if (cudaMallocHost(&s->host_scal, (16 + EXPZ_MASKS) * sizeof(double)) != cudaSuccess) return fail(set_err(s, QOA_E_OOM, "pinned alloc"));
@@ -3744,7 +3802,12 @@ int qoa_destroy(qoa_state_t s) {
     if (s->f32_mats) cudaFree(s->f32_mats);
     if (s->f32_phases) cudaFree(s->f32_phases);
     if (s->partials) cudaFree(s->partials);
-    if (s->ws) cudaFree(s->ws);
+    double* ws = nullptr;
+    {
+        std::lock_guard<std::mutex> lk(g_ws_mu);
+        ws = forget(s);
+    }
+    if (ws) cudaFree(ws);
     if (s->scal) cudaFree(s->scal);
     if (s->status) cudaFree(s->status);
     if (s->host_scal) cudaFreeHost(s->host_scal);
@@ -3807,15 +3870,15 @@ int qoa_sample(qoa_state_t s, const double* u, size_t shots, int mode, uint64_t*
     const uint32_t n = s->n;
     const size_t nu = mode == 0 ? shots * n : shots;
     const SampleLevels L = sample_levels(n);
-    // uniforms, then the outcomes, then the tree levels: one workspace.
+    // uniforms, then the outcomes, then the tree levels: one buffer.
     // Shots read each uniform and write each outcome once, so both may also
     // stay in pinned host memory.
     const size_t io = (nu + shots) * sizeof(double);
     Staging host(io, s->stream);
     const bool direct = host.get() && io <= 4 * kDirectBytes;
-    double* ws = nullptr;
-    rc = workspace(s, ((direct ? 0 : nu + shots) + (size_t)L.total) * sizeof(double) + sizeof(double), &ws);
-    if (rc) return rc;
+    Workspace scratch(s, ((direct ? 0 : nu + shots) + (size_t)L.total) * sizeof(double) + sizeof(double));
+    CK(scratch.error());
+    double* ws = scratch.get();
     double* d_u = direct ? host.get() : ws;
     unsigned long long* d_out = reinterpret_cast<unsigned long long*>(d_u + nu);
     double* d_tree = direct ? ws : ws + nu + shots;
@@ -3829,7 +3892,7 @@ int qoa_sample(qoa_state_t s, const double* u, size_t shots, int mode, uint64_t*
     CK(cudaStreamSynchronize(s->stream));
     host.done();
     if (direct) std::memcpy(out, d_out, shots * sizeof(uint64_t));
-    return workspace_done(s);
+    return QOA_OK;
 }
 
 int qoa_probabilities(qoa_state_t s, double* out) {
@@ -3841,11 +3904,9 @@ int qoa_probabilities(qoa_state_t s, double* out) {
     Staging host(len * sizeof(double), s->stream);
     if (host.get()) {
         const bool direct = len * sizeof(double) <= kDirectBytes;
-        double* d = host.get();
-        if (!direct) {
-            rc = workspace(s, len * sizeof(double), &d);
-            if (rc) return rc;
-        }
+        Workspace scratch(s, direct ? 0 : len * sizeof(double));
+        CK(scratch.error());
+        double* d = direct ? host.get() : scratch.get();
         if (s->precision == QOA_PREC_F32) CK(launch_f32_probs((const float2*)s->amps, 0, len, s->scal, d, s->stream));
         else CK(launch_probs(s->amps, 0, len, s->scal, d, s->stream));
         s->launches++;
@@ -3855,9 +3916,9 @@ int qoa_probabilities(qoa_state_t s, double* out) {
         std::memcpy(out, host.get(), len * sizeof(double));
         return QOA_OK;
     }
-    double* d = nullptr;
-    rc = workspace(s, chunk * sizeof(double), &d);
-    if (rc) return rc;
+    Workspace scratch(s, chunk * sizeof(double));
+    CK(scratch.error());
+    double* d = scratch.get();
     for (uint64_t off = 0; off < len; off += chunk) {
         const uint64_t cnt = std::min(chunk, len - off);
         if (s->precision == QOA_PREC_F32)
@@ -3868,29 +3929,29 @@ int qoa_probabilities(qoa_state_t s, double* out) {
         CK(cudaMemcpyAsync(out + off, d, cnt * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
     }
     CK(cudaStreamSynchronize(s->stream));
-    return workspace_done(s);
+    return QOA_OK;
 }
 
 int qoa_expect_z(qoa_state_t s, const uint64_t* masks, size_t k, double* out) {
     int rc = check_handle(s);
     if (rc) return rc;
     if ((!masks || !out) && k) return set_err(s, QOA_E_ARG, "null argument");
+    if (!k) return QOA_OK;
     const uint32_t blocks = expz_blocks(state_len(s));
+    Workspace scratch(s, std::min<size_t>(EXPZ_MASKS, k) * blocks * sizeof(double));  // partial sums
+    CK(scratch.error());
     for (size_t i = 0; i < k; i += EXPZ_MASKS) {
         const uint32_t kk = (uint32_t)std::min<size_t>(EXPZ_MASKS, k - i);
         ExpzMasks M;
         std::memcpy(M.m, masks + i, kk * sizeof(uint64_t));
-        double* ws = nullptr;  // partial sums
-        rc = workspace(s, (size_t)kk * blocks * sizeof(double), &ws);
-        if (rc) return rc;
         // FP64 sums over either precision, results straight to pinned host memory
-        CK(launch_expz(s->amps, s->precision == QOA_PREC_F32, state_len(s), M, kk, s->scal, ws, ticket(s),
+        CK(launch_expz(s->amps, s->precision == QOA_PREC_F32, state_len(s), M, kk, s->scal, scratch.get(), ticket(s),
                        s->host_scal + 16, s->stream));
         s->launches++;
         CK(cudaStreamSynchronize(s->stream));
         std::memcpy(out + i, s->host_scal + 16, kk * sizeof(double));
     }
-    return workspace_done(s);
+    return QOA_OK;
 }
 
 int qoa_get_state(qoa_state_t s, void* host, size_t bytes) {
