@@ -15,6 +15,7 @@
 
 #include <algorithm>
 #include <memory>
+#include <optional>
 #include <deque>
 #include <thread>
 #include <functional>
@@ -59,10 +60,12 @@ cudaError_t launch_set_scalar(double* p, double v, cudaStream_t st);
 cudaError_t launch_init_scalars(double* scal, uint32_t* status, cudaStream_t st);
 cudaError_t launch_probs(const double2* a, uint64_t off, uint64_t cnt, const double* norm2, double* out, cudaStream_t st);
 SampleLevels sample_levels(uint32_t n);
-cudaError_t launch_sample_tree(const void* a, bool f32, uint32_t n, const double* norm2, const SampleLevels& L, double* tree,
-                               cudaStream_t st);
+bool sample_all_levels(uint32_t n, uint64_t shots);
+uint64_t sample_all_doubles(uint32_t n);
+cudaError_t launch_sample_tree(const void* a, bool f32, uint32_t n, const double* norm2, const SampleLevels& L, bool all,
+                               double* tree, cudaStream_t st);
 cudaError_t launch_shots(const void* a, bool f32, uint32_t n, const double* norm2, const double* tree, const SampleLevels& L,
-                         const double* u, uint64_t shots, int mode, unsigned long long* out, cudaStream_t st);
+                         bool all, const double* u, uint64_t shots, int mode, unsigned long long* out, cudaStream_t st);
 cudaError_t launch_f32_pass(float2* amps, const F32PassParams& P, const float* mats, const F32PhaseOp* pops,
                             const F32Angle* angles, const F32Phase* phases, const float2* tables,
                             const double* norm2_in, double* partials, uint32_t* status, cudaStream_t st);
@@ -3874,18 +3877,26 @@ int qoa_sample(qoa_state_t s, const double* u, size_t shots, int mode, uint64_t*
     const size_t io = (nu + shots) * sizeof(double);
     Staging host(io, s->stream);
     const bool direct = host.get() && io <= 4 * kDirectBytes;
-    Workspace scratch(s, ((direct ? 0 : nu + shots) + (size_t)L.total) * sizeof(double) + sizeof(double));
-    CK(scratch.error());
-    double* ws = scratch.get();
+    const size_t io_ws = direct ? 0 : nu + shots;
+    bool all = sample_all_levels(n, shots);
+    std::optional<Workspace> scratch;
+    scratch.emplace(s, (io_ws + (size_t)(all ? sample_all_doubles(n) : L.total)) * sizeof(double) + sizeof(double));
+    if (all && scratch->error() == cudaErrorMemoryAllocation) {  // no room for all levels
+        cudaGetLastError();
+        all = false;
+        scratch.emplace(s, (io_ws + (size_t)L.total) * sizeof(double) + sizeof(double));
+    }
+    CK(scratch->error());
+    double* ws = scratch->get();
     double* d_u = direct ? host.get() : ws;
     unsigned long long* d_out = reinterpret_cast<unsigned long long*>(d_u + nu);
     double* d_tree = direct ? ws : ws + nu + shots;
     const bool f32 = s->precision == QOA_PREC_F32;
-    CK(launch_sample_tree(s->amps, f32, n, s->scal, L, d_tree, s->stream));
+    CK(launch_sample_tree(s->amps, f32, n, s->scal, L, all, d_tree, s->stream));
     if (direct) std::memcpy(host.get(), u, nu * sizeof(double));  // while the tree is made
     else CK(cudaMemcpyAsync(d_u, u, nu * sizeof(double), cudaMemcpyHostToDevice, s->stream));
-    CK(launch_shots(s->amps, f32, n, s->scal, d_tree, L, d_u, shots, mode, d_out, s->stream));
-    s->launches += L.count + 1;
+    CK(launch_shots(s->amps, f32, n, s->scal, d_tree, L, all, d_u, shots, mode, d_out, s->stream));
+    s->launches += L.count + 1 + (all && n >= 2 ? 1 : 0);
     if (!direct) CK(cudaMemcpyAsync(out, d_out, shots * sizeof(uint64_t), cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
     host.done();

@@ -7,7 +7,9 @@
 // shot is one warp: at each stored level it gathers the up to 2^8 values
 // below its prefix, folds them into the levels in between and walks those.
 // Every sum pairs the top bit of its index first, at every level, whichever
-// levels are stored, so a shot does not depend on the split.
+// levels are stored, so a shot does not depend on the split. Where shots are
+// many (sample_all_levels) the same folds store every level they pass, and a
+// thread walks a shot.
 //
 // What bounds it: reading the state once (the fold of the amplitudes), and
 // for small states the launches: 1 + ceil((n - 8) / 6) of them, where a
@@ -18,6 +20,7 @@
 // 78.5 -> 19.9 ms.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <stdint.h>
 
 #include "qoa_kernels.cuh"
@@ -48,39 +51,69 @@ __device__ __forceinline__ AmpSrc<T> amp_src(const T* a, const double* norm2) {
     return AmpSrc<T>{a, valid ? 1.0 / nrm : 1.0, valid};
 }
 
+// Offset of level k (1 <= k < n) in a tree of all levels.
+__host__ __device__ __forceinline__ uint64_t level_at(uint32_t k) { return (1ull << k) - 2; }
+
 // Sum over j < 2^B of the values p + (j << lo), top bit of j paired first.
-// From amplitudes, 1/norm2 is applied to the sums of two (level n - 1).
-template <int B, int K, bool AMPS, typename S>
-__device__ __forceinline__ double fold(const S& s, uint64_t p, uint32_t lo, uint32_t j) {
+// From amplitudes, 1/norm2 is applied to the sums of two (level n - 1). ALL:
+// every sum on the way is a value of a level in between and goes to the tree
+// of all levels at `out`; else the sum goes to out[p].
+template <int B, int K, bool AMPS, bool ALL, typename S>
+__device__ __forceinline__ double fold(const S& s, uint64_t p, uint32_t lo, uint32_t j, double* out) {
     if constexpr (K == B) {
         const uint64_t i = p + ((uint64_t)j << lo);
         if constexpr (AMPS) return s.raw(i);
         else return s[i];
     } else {
-        const double x = fold<B, K + 1, AMPS>(s, p, lo, j) + fold<B, K + 1, AMPS>(s, p, lo, j + (1u << K));
-        if constexpr (AMPS && K == B - 1) return x * s.inv;
+        double x = fold<B, K + 1, AMPS, ALL>(s, p, lo, j, out) + fold<B, K + 1, AMPS, ALL>(s, p, lo, j + (1u << K), out);
+        if constexpr (AMPS && K == B - 1) x = x * s.inv;
+        if constexpr (ALL) out[level_at(lo + K) + p + ((uint64_t)j << lo)] = x;
+        else if constexpr (K == 0) out[p] = x;
         return x;
     }
 }
 
-template <int B, typename T>
-__global__ void __launch_bounds__(128) k_fold_amps(const T* a, const double* norm2, uint32_t lo,
-                                                   double* __restrict__ out) {
+template <int B, bool ALL, typename T>
+__global__ void __launch_bounds__(128) k_fold_amps(const T* a, const double* norm2, uint32_t lo, double* out) {
     grid_go();
     grid_wait();
     const AmpSrc<T> s = amp_src(a, norm2);
     const uint64_t cnt = 1ull << lo;
     for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < cnt; p += (uint64_t)gridDim.x * blockDim.x)
-        out[p] = fold<B, 0, true>(s, p, lo, 0);
+        fold<B, 0, true, ALL>(s, p, lo, 0, out);
 }
 
-template <int B>
-__global__ void __launch_bounds__(128) k_fold_level(const double* in, uint32_t lo, double* __restrict__ out) {
+template <int B, bool ALL>
+__global__ void __launch_bounds__(128) k_fold_level(const double* in, uint32_t lo, double* out) {
     grid_go();
     grid_wait();
     const uint64_t cnt = 1ull << lo;
     for (uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; p < cnt; p += (uint64_t)gridDim.x * blockDim.x)
-        out[p] = fold<B, 0, false>(in, p, lo, 0);
+        fold<B, 0, false, ALL>(in, p, lo, 0, out);
+}
+
+// The lowest levels of a tree of all levels: from level ROOT_BITS (n above
+// it), or from the amplitudes, down to level 1.
+template <typename T>
+__global__ void __launch_bounds__(128) k_tree_root(const T* a, uint32_t n, const double* norm2, double* tree) {
+    grid_go();
+    grid_wait();
+    __shared__ double s[1 << ROOT_BITS];
+    uint32_t k;
+    if (n > ROOT_BITS) {
+        k = ROOT_BITS;
+        for (uint32_t p = threadIdx.x; p < (1u << k); p += blockDim.x) s[p] = tree[level_at(k) + p];
+    } else {
+        const AmpSrc<T> src = amp_src(a, norm2);
+        k = n - 1;
+        for (uint32_t p = threadIdx.x; p < (1u << k); p += blockDim.x)
+            tree[level_at(k) + p] = s[p] = (src.raw(p) + src.raw(p + (1u << k))) * src.inv;
+    }
+    while (--k >= 1) {
+        __syncthreads();
+        const uint32_t p = threadIdx.x, h = 1u << k;
+        if (p < h) tree[level_at(k) + p] = s[p] = s[p] + s[p + h];
+    }
 }
 
 // The levels between a prefix and the 2^b values below it, in one warp:
@@ -238,6 +271,48 @@ __global__ void __launch_bounds__(128) k_shots(const T* a, uint32_t n, const dou
     }
 }
 
+// One thread per shot on a tree of all levels: n dependent loads, and shots
+// beside one another hide them. The same sums and the same walk as k_shots.
+template <typename T>
+__global__ void __launch_bounds__(128) k_shots_tree(const T* a, uint32_t n, const double* norm2, const double* tree,
+                                                    const double* __restrict__ u, uint64_t shots, int mode,
+                                                    unsigned long long* __restrict__ out) {
+    grid_go();
+    grid_wait();
+    const AmpSrc<T> src = amp_src(a, norm2);
+    auto h = [&](uint32_t k, uint64_t p) -> double {
+        if (k == n) return src.raw(p) * src.inv;
+        if (k == 0) return n == 1 ? (src.raw(0) + src.raw(1)) * src.inv : tree[0] + tree[1];
+        return tree[level_at(k) + p];
+    };
+    for (uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; s < shots; s += (uint64_t)gridDim.x * blockDim.x) {
+        uint64_t pre = 0;
+        if (mode == 0) {
+            double tot = h(0, 0);
+            for (uint32_t q = 0; q < n; ++q) {
+                const double left = h(q + 1, pre), p0 = left / tot;
+                double kept = left, pb = p0;
+                if (!(u[s * n + q] < p0)) {
+                    pre |= 1ull << q;
+                    kept = h(q + 1, pre);
+                    pb = kept / tot;
+                }
+                if (!(pb > 1e-12)) break;
+                tot = kept;
+            }
+        } else {
+            double t = u[s] * h(0, 0);
+            for (uint32_t q = 0; q < n; ++q) {
+                const double left = h(q + 1, pre);
+                if (t < left) continue;
+                t -= left;
+                pre |= 1ull << q;
+            }
+        }
+        out[s] = pre;
+    }
+}
+
 int fold_grid(uint32_t lo) {
     const uint64_t b = ((1ull << lo) + 127) / 128;
     return (int)(b < 148 * 16 ? b : 148 * 16);
@@ -267,52 +342,83 @@ SampleLevels sample_levels(uint32_t n) {
     return L;
 }
 
-template <typename T>
+// Shots from which a tree of all levels and a thread per shot beat the stored
+// levels and a warp per shot (2.5 ns a shot at 20 qubits, against 0.1 ns and
+// the tree's writes and launches). Whole calls in us, inverse CDF, warp against
+// all levels: 20 qubits 2^14 shots 91 / 48, 2^20 4075 / 936; 24 qubits 2^14 150
+// / 161, 2^16 398 / 210; 26 qubits (a tree too large to keep is mapped per
+// call) 2^18 1501 / 1610, 2^20 5407 / 2391; 28 qubits 2^18 2219 / 3779, 2^20
+// 6566 / 4532. Below 2^14 shots they differ by less than 20 % up to 22 qubits.
+bool sample_all_levels(uint32_t n, uint64_t shots) {
+    return shots >= std::max<uint64_t>(1ull << 14, (1ull << n) >> 8);
+}
+uint64_t sample_all_doubles(uint32_t n) { return n >= 2 ? level_at(n) : 1; }
+
+template <bool ALL, typename T>
 static cudaError_t fold_amps(const T* a, const double* norm2, uint32_t b, uint32_t lo, double* out, cudaStream_t st) {
     const int g = fold_grid(lo);
     switch (b) {
-        case 1: return launch_overlapped(k_fold_amps<1, T>, g, 128, 0, st, a, norm2, lo, out);
-        case 2: return launch_overlapped(k_fold_amps<2, T>, g, 128, 0, st, a, norm2, lo, out);
-        case 3: return launch_overlapped(k_fold_amps<3, T>, g, 128, 0, st, a, norm2, lo, out);
-        case 4: return launch_overlapped(k_fold_amps<4, T>, g, 128, 0, st, a, norm2, lo, out);
-        case 5: return launch_overlapped(k_fold_amps<5, T>, g, 128, 0, st, a, norm2, lo, out);
-        default: return launch_overlapped(k_fold_amps<6, T>, g, 128, 0, st, a, norm2, lo, out);
+        case 1: return launch_overlapped(k_fold_amps<1, ALL, T>, g, 128, 0, st, a, norm2, lo, out);
+        case 2: return launch_overlapped(k_fold_amps<2, ALL, T>, g, 128, 0, st, a, norm2, lo, out);
+        case 3: return launch_overlapped(k_fold_amps<3, ALL, T>, g, 128, 0, st, a, norm2, lo, out);
+        case 4: return launch_overlapped(k_fold_amps<4, ALL, T>, g, 128, 0, st, a, norm2, lo, out);
+        case 5: return launch_overlapped(k_fold_amps<5, ALL, T>, g, 128, 0, st, a, norm2, lo, out);
+        default: return launch_overlapped(k_fold_amps<6, ALL, T>, g, 128, 0, st, a, norm2, lo, out);
+    }
+}
+template <bool ALL>
+static cudaError_t fold_level(const double* in, uint32_t b, uint32_t lo, double* out, cudaStream_t st) {
+    const int g = fold_grid(lo);
+    switch (b) {
+        case 1: return launch_overlapped(k_fold_level<1, ALL>, g, 128, 0, st, in, lo, out);
+        case 2: return launch_overlapped(k_fold_level<2, ALL>, g, 128, 0, st, in, lo, out);
+        case 3: return launch_overlapped(k_fold_level<3, ALL>, g, 128, 0, st, in, lo, out);
+        case 4: return launch_overlapped(k_fold_level<4, ALL>, g, 128, 0, st, in, lo, out);
+        case 5: return launch_overlapped(k_fold_level<5, ALL>, g, 128, 0, st, in, lo, out);
+        default: return launch_overlapped(k_fold_level<6, ALL>, g, 128, 0, st, in, lo, out);
     }
 }
 
-cudaError_t launch_sample_tree(const void* a, bool f32, uint32_t n, const double* norm2, const SampleLevels& L, double* tree,
+// tree: L.total doubles (the stored levels at L.off), or with ALL
+// sample_all_doubles(n) (level k at 2^k - 2).
+template <bool ALL, typename T>
+static cudaError_t sample_tree(const T* a, uint32_t n, const double* norm2, const SampleLevels& L, double* tree,
                                cudaStream_t st) {
     cudaError_t e = cudaSuccess;
-    for (uint32_t k = 0; k < L.count; ++k) {
+    for (uint32_t k = 0; k < L.count && e == cudaSuccess; ++k) {
         const uint32_t lo = L.bits[k];
-        double* out = tree + L.off[k];
+        double* out = ALL ? tree : tree + L.off[k];
         if (k == 0) {
-            e = f32 ? fold_amps((const float2*)a, norm2, n - lo, lo, out, st)
-                    : fold_amps((const double2*)a, norm2, n - lo, lo, out, st);
-            if (e != cudaSuccess) return e;
+            e = fold_amps<ALL>(a, norm2, n - lo, lo, out, st);
             continue;
         }
-        const double* in = tree + L.off[k - 1];
-        const int g = fold_grid(lo);
-        switch (L.bits[k - 1] - lo) {
-            case 1: e = launch_overlapped(k_fold_level<1>, g, 128, 0, st, in, lo, out); break;
-            case 2: e = launch_overlapped(k_fold_level<2>, g, 128, 0, st, in, lo, out); break;
-            case 3: e = launch_overlapped(k_fold_level<3>, g, 128, 0, st, in, lo, out); break;
-            case 4: e = launch_overlapped(k_fold_level<4>, g, 128, 0, st, in, lo, out); break;
-            case 5: e = launch_overlapped(k_fold_level<5>, g, 128, 0, st, in, lo, out); break;
-            default: e = launch_overlapped(k_fold_level<6>, g, 128, 0, st, in, lo, out); break;
-        }
-        if (e != cudaSuccess) return e;
+        const double* in = ALL ? tree + level_at(L.bits[k - 1]) : tree + L.off[k - 1];
+        e = fold_level<ALL>(in, L.bits[k - 1] - lo, lo, out, st);
     }
-    return cudaSuccess;
+    if (ALL && e == cudaSuccess && n >= 2) e = launch_overlapped(k_tree_root<T>, 1, 128, 0, st, a, n, norm2, tree);
+    return e;
 }
 
-cudaError_t launch_shots(const void* a, bool f32, uint32_t n, const double* norm2, const double* tree, const SampleLevels& L,
-                         const double* u, uint64_t shots, int mode, unsigned long long* out, cudaStream_t st) {
-    const uint64_t blocks = (shots + 3) / 4;
+cudaError_t launch_sample_tree(const void* a, bool f32, uint32_t n, const double* norm2, const SampleLevels& L, bool all,
+                               double* tree, cudaStream_t st) {
+    if (f32) return all ? sample_tree<true>((const float2*)a, n, norm2, L, tree, st)
+                        : sample_tree<false>((const float2*)a, n, norm2, L, tree, st);
+    return all ? sample_tree<true>((const double2*)a, n, norm2, L, tree, st)
+               : sample_tree<false>((const double2*)a, n, norm2, L, tree, st);
+}
+
+template <typename T>
+static cudaError_t shots_on(const T* a, uint32_t n, const double* norm2, const double* tree, const SampleLevels& L, bool all,
+                            const double* u, uint64_t shots, int mode, unsigned long long* out, cudaStream_t st) {
+    const uint64_t blocks = all ? (shots + 127) / 128 : (shots + 3) / 4;
     const int g = (int)(blocks < 148 * 16 ? blocks : 148 * 16);
-    if (f32) return launch_overlapped(k_shots<float2>, g, 128, 0, st, (const float2*)a, n, norm2, tree, L, u, shots, mode, out);
-    return launch_overlapped(k_shots<double2>, g, 128, 0, st, (const double2*)a, n, norm2, tree, L, u, shots, mode, out);
+    if (all) return launch_overlapped(k_shots_tree<T>, g, 128, 0, st, a, n, norm2, tree, u, shots, mode, out);
+    return launch_overlapped(k_shots<T>, g, 128, 0, st, a, n, norm2, tree, L, u, shots, mode, out);
+}
+cudaError_t launch_shots(const void* a, bool f32, uint32_t n, const double* norm2, const double* tree, const SampleLevels& L,
+                         bool all, const double* u, uint64_t shots, int mode, unsigned long long* out, cudaStream_t st) {
+    return f32 ? shots_on((const float2*)a, n, norm2, tree, L, all, u, shots, mode, out, st)
+               : shots_on((const double2*)a, n, norm2, tree, L, all, u, shots, mode, out, st);
 }
 
 }  // namespace qoa
