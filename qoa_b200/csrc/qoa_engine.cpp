@@ -266,6 +266,7 @@ struct Gate {
     uint64_t nmask = 0;     // qubits acted on non-diagonally
     uint64_t dmask = 0;     // qubits acted on diagonally (controls, phase masks, selector)
     int src = -1;           // source op index
+    int part = -1;          // one of the three gates of a controlled SWAP: which of the list's (split_controlled_swaps)
     double u = -1.0;        // K_MEASURE: uniform
     uint8_t pi[64];         // K_PERM: partner of each qubit (itself if unpaired)
 };
@@ -873,6 +874,8 @@ struct Expander {
 // gate that runs on its own kernel (in complex64 a 4x4; a SWAP block; barriers).
 struct Step {
     bool pass = false;
+    bool own = false;              // a handle's: its few gates run on their own kernels (mark_own_kernels)
+    bool few = false;              // a handle's pass of few gates: never on a generated kernel
     std::vector<int> gates;        // indices into the gate list, in application order
     std::vector<int> slots;        // pass: high qubits of the tile (HIGH_SLOTS)
 };
@@ -888,6 +891,7 @@ struct PlanEntry {
     bool prebuilt = false;
     std::vector<PassParams> built;
     std::vector<int> built_of;
+    std::vector<int> body_of;        // per built pass: its text in bodies (-1: interpreted)
     std::vector<std::string> bodies;
     std::vector<JitKernel> kernels;  // of bodies, as the last request gave them
 };
@@ -916,7 +920,7 @@ void plan_hash(const std::vector<Gate>& G, uint64_t key, uint64_t& h1, uint64_t&
         }
     };
     for (const Gate& g : G) {
-        mix((uint64_t)(uint8_t)g.kind | ((uint64_t)(uint8_t)g.sub << 8) | ((uint64_t)g.neg << 16) |
+        mix((uint64_t)(uint8_t)g.kind | ((uint64_t)(uint8_t)g.sub << 8) | ((uint64_t)g.neg << 16) | ((uint64_t)(g.part >= 0) << 24) |
             ((uint64_t)(uint16_t)g.t << 32) | ((uint64_t)(uint16_t)g.t2 << 48));
         mix(g.cmask);
         mix(g.nmask);
@@ -2572,8 +2576,10 @@ void split_controlled_swaps(std::vector<Gate>& G) {
     if (!extra) return;
     std::vector<Gate> out;
     out.reserve(G.size() + extra);
+    int part = -1;
     auto x = [&](const Gate& g, int t, uint64_t cm) {
         Gate o;
+        o.part = part;
         o.kind = K_G1;
         o.sub = G1_X;
         o.t = t;
@@ -2590,6 +2596,7 @@ void split_controlled_swaps(std::vector<Gate>& G) {
             out.push_back(g);
             continue;
         }
+        ++part;
         x(g, g.t2, 1ull << g.t);
         x(g, g.t, g.cmask | (1ull << g.t2));
         x(g, g.t2, 1ull << g.t);
@@ -2606,6 +2613,92 @@ void prepare_gates(std::vector<Gate>& G, bool swap_blocks) {
 }
 std::vector<Step> plan_steps(const std::vector<Gate>& G, uint32_t n, bool per_gate, bool c64, int gate_budget, bool search) {
     return schedule(G, n, per_gate, false, gate_budget, search, !c64);
+}
+
+// A handle's passes that hold nothing but unitary 4x4 gates and controlled
+// SWAPs, with no other pass before or after them (among other passes the norm
+// is carried and launches overlap): a run of p such passes with few of those
+// gates goes to their own kernels. A pass sweeps the whole state (a controlled SWAP a quarter of it) and takes an
+// interpreter's start. Calls in us, kernels against passes:
+//   up to 18 qubits, any two (p = 1): 9 / 13, any three 12 / 14 (p = 2: 16);
+//   states that L2 holds, controlled SWAPs: one at 20 qubits 9 / 13, three at
+//   22 qubits 27 / 40; beyond, one at 26 198 / 371, two at 24 108 / 98;
+//   one 4x4: at 20 qubits 7 / 13, at 26 359 / 366, two at 22 33 / 29.
+// Passes of up to eight run interpreted: making and looking up a kernel's text
+// costs more than it saves (20 qubits, a list of three 4x4: new 60 against 16,
+// repeated 22 against 14; of fourteen 129 against 36 and 36 against 35; 24
+// qubits alike).
+void mark_own_kernels(const std::vector<Gate>& G, std::vector<Step>& steps, uint32_t n, bool c64) {
+    constexpr size_t kFew = 24;  // gates: eight controlled SWAPs
+    const uint64_t bytes = (c64 ? 8ull : 16ull) << n;
+    for (Step& st : steps) {
+        st.few = st.pass && st.gates.size() <= kFew;
+        for (size_t i = 0; st.few && i < st.gates.size(); ++i) {
+            const Gate& g = G[st.gates[i]];
+            st.few = g.part >= 0 || (g.kind == K_U2 && unitary_matrix(g.m, 4));
+        }
+    }
+    std::vector<Step> out;
+    out.reserve(steps.size());
+    for (size_t k = 0; k < steps.size();) {
+        size_t end = k;
+        std::vector<int> all;  // the run's gates as submitted: an order that its passes keep to
+        for (; end < steps.size() && steps[end].few; ++end)
+            all.insert(all.end(), steps[end].gates.begin(), steps[end].gates.end());
+        std::sort(all.begin(), all.end());
+        size_t u2 = 0, swaps = 0;
+        bool whole = true;
+        for (size_t i = 0; whole && i < all.size();) {
+            const int part = G[all[i]].part;
+            if (part < 0) {
+                ++u2;
+                ++i;
+            } else if (i + 2 < all.size() && G[all[i + 1]].part == part && G[all[i + 2]].part == part) {
+                ++swaps;
+                i += 3;
+            } else {
+                whole = false;  // the rest of it is in a pass with other gates
+            }
+        }
+        const size_t p = end - k;
+        const bool apart = p && (out.empty() || !out.back().pass) && (end == steps.size() || !steps[end].pass);
+        if (!apart)
+            for (size_t i = k; i < end; ++i) steps[i].few = false;
+        const size_t most = bytes <= (4ull << 20) ? p + 1 : !u2 ? (bytes <= (64ull << 20) ? 3 : 2) * p : p == 1 ? 1 : 0;
+        if (apart && whole && u2 + swaps <= most) {
+            Step own;
+            own.own = true;
+            own.gates.swap(all);
+            out.push_back(std::move(own));
+            k = end;
+            continue;
+        }
+        do out.push_back(std::move(steps[k])); while (++k < end);
+    }
+    steps.swap(out);
+}
+
+// Runs a step marked so.
+int run_own(qoa_state_t s, const std::vector<Gate>& G, const Step& st) {
+    for (size_t i = 0; i < st.gates.size();) {
+        const Gate& g = G[st.gates[i]];
+        if (g.kind == K_U2) {
+            const int rc = run_gate(s, g);
+            if (rc) return rc;
+            ++i;
+            continue;
+        }
+        const Gate& y = G[st.gates[i + 1]];  // of x(b; a), x(a; control, b), x(b; a)
+        Gate w;
+        w.kind = K_SWAP;
+        w.t = y.t;
+        w.t2 = g.t;
+        w.cmask = y.cmask & ~(1ull << g.t);
+        const int rc = run_gate(s, w);
+        if (rc) return rc;
+        i += 3;
+    }
+    return QOA_OK;
 }
 
 int run_perm(qoa_state_t s, const Gate& g) {
@@ -2739,6 +2832,7 @@ int run_planned(qoa_state_t s, std::vector<Gate>& seg, bool& reset_owed) {
         // executed again gives bit-identical results
         pe->steps = plan_steps(seg, s->n, per_gate, c64, state_pass_budget(s),
                                slot_search_pays(s->n) || (s->flags & QOA_FLAG_SLOT_SEARCH));
+        mark_own_kernels(seg, pe->steps, s->n, c64);
         pe->built_of.assign(pe->steps.size(), -1);
         // passes built ahead: for generated kernels, whose text is
         // requested from the compile cache, and for a plan that is kept
@@ -2750,7 +2844,9 @@ int run_planned(qoa_state_t s, std::vector<Gate>& seg, bool& reset_owed) {
             for (size_t k = 0; k < pe->steps.size(); ++k) {
                 if (!pe->steps[k].pass || build_pass(seg, pe->steps[k], s->n, pe->built[b], c64) != 0) continue;
                 pe->built_of[k] = (int)b;
-                if (jit) pe->bodies.push_back(c64 ? jit_pass32_body(pe->built[b]) : jit_pass_body(pe->built[b]));
+                const bool text = jit && !pe->steps[k].few;
+                pe->body_of.push_back(text ? (int)pe->bodies.size() : -1);
+                if (text) pe->bodies.push_back(c64 ? jit_pass32_body(pe->built[b]) : jit_pass_body(pe->built[b]));
                 ++b;
             }
             pe->prebuilt = jit;
@@ -2783,11 +2879,16 @@ int run_planned(qoa_state_t s, std::vector<Gate>& seg, bool& reset_owed) {
             // a pass after a unitary pass takes its input as normalised
             nm.out = !(k + 1 < steps.size() && steps[k + 1].pass && unitary_pass(seg, st));
             nm.per_gate = false;
-            if (built_of[k] >= 0)
-                rc = run_pass_built(s, built[built_of[k]], pe->prebuilt ? jk[built_of[k]] : none, nm);
+            const int b = built_of[k], body = b >= 0 ? pe->body_of[b] : -1;
+            if (b >= 0)
+                rc = run_pass_built(s, built[b], pe->prebuilt && body >= 0 ? jk[body] : none, nm);
             else
                 rc = run_pass(s, seg, st, nm);
             nm.in = nm.out || nm.per_gate ? 0 : SCAL_ONE;
+        } else if (st.own) {
+            if (reset_owed) rc = do_reset_all(s);  // the kernels read the state
+            reset_owed = false;
+            if (!rc) rc = run_own(s, seg, st);
         } else {
             const Gate& g = seg[st.gates[0]];
             if (is_barrier(g) && g.kind != K_PERM) {
@@ -4128,6 +4229,7 @@ int qoa_plan(uint32_t n, uint32_t flags, const qoa_op* ops, size_t nops, size_t 
     const bool per_gate = (flags & QOA_FLAG_PER_GATE) != 0;
     if (!per_gate && ex.n >= (uint32_t)TILE_BITS) prepare_gates(G, false);
     std::vector<Step> steps = plan_steps(G, ex.n, per_gate, false, 0, slot_search_pays(ex.n) || (flags & QOA_PLAN_SLOT_SEARCH));
+    mark_own_kernels(G, steps, ex.n, false);
     *ngates = G.size();
     *npasses = steps.size();
     if (G.size() > cap) return set_err(nullptr, QOA_E_ARG, "cap too small: %zu gates", G.size());
@@ -4672,11 +4774,12 @@ int qoa_jit_translate(uint32_t n, int precision, uint32_t flags, const qoa_op* o
     std::vector<Step> steps = plan_steps(G, n, false, precision == QOA_PREC_F32, 0, slot_search_pays(n));
     std::vector<std::string> bodies;
     static thread_local PassParams P;
+    const bool arena = (compile & 2) != 0;
+    if (!arena) mark_own_kernels(G, steps, n, precision == QOA_PREC_F32);
     for (const Step& st : steps) {
         if (!st.pass) continue;
         if (build_pass(G, st, n, P, precision == QOA_PREC_F32) != 0)
             return set_err(nullptr, QOA_E_ARG, "a pass does not fit one launch");
-        const bool arena = (compile & 2) != 0;
         bodies.push_back(precision == QOA_PREC_F32 ? jit_pass32_body(P, arena) : jit_pass_body(P, arena));
     }
     if (npasses) *npasses = bodies.size();
