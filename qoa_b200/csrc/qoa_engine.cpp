@@ -323,6 +323,10 @@ struct qoa_state_s {
     double* ws = nullptr;         // scratch kept between calls (Workspace)
     size_t ws_cap = 0;
     bool ws_busy = false;         // a call uses it (g_ws_mu)
+    // The stored vector's norm2 is known on the host to be above 1e-12, so that
+    // gates may act on the stored amplitudes (otherwise the logical state may
+    // be |0..0>). False after anything that is not unitary, until a reset.
+    bool norm_sure = false;
     double* host_scal = nullptr;  // pinned: mirror of scal, then EXPZ_MASKS results (kernels write them there)
     uint64_t seed = 0;
     uint64_t noise_stream = 0;
@@ -2236,27 +2240,6 @@ GGate to_ggate(const Gate& g) {
     return k;
 }
 
-int run_gate(qoa_state_t s, const Gate& g) {
-    const GGate k = to_ggate(g);
-    Timer tm(s, gate_bytes(g, s->n) * (s->precision == QOA_PREC_F32 ? 0.5 : 1.0), 1);
-    if (s->precision == QOA_PREC_F32) CK(launch_gate_c64((float2*)s->amps, state_len(s), k, s->stream));
-    else CK(launch_gate(s->amps, state_len(s), k, s->stream));
-    s->launches++;
-    return QOA_OK;
-}
-
-int do_reset_all(qoa_state_t s);
-
-// How a pass takes its input's squared norm and whether it leaves its own.
-//   in   SCAL_* index: 0 the handle's norm2, SCAL_ONE a normalised input
-//        (the pass before was unitary), SCAL_ZERO |0..0>, which is not read
-//   out  norm partials and their sum into the handle's norm2
-struct PassNorm {
-    int in = 0;
-    bool out = true;
-    bool per_gate = false;  // set where the pass ran as per-gate kernels instead (norm2 is then valid)
-};
-
 // A caller's k x k matrix is unitary to 1e-10: the norm it gives can drift by
 // that much, far from the 1e-12 below which a state is reset.
 bool unitary_matrix(const double2* m, int k) {
@@ -2273,25 +2256,47 @@ bool unitary_matrix(const double2* m, int k) {
     return true;
 }
 
+bool unitary_gate(const Gate& g) {
+    auto unit = [](double2 d) { return std::fabs(d.x * d.x + d.y * d.y - 1.0) < 1e-12; };
+    switch (g.kind) {
+        case K_DIAG: return g.neg || (unit(g.m[0]) && (g.t < 0 || unit(g.m[1])));
+        case K_G1:
+            if (g.sub == G1_GEN) return unitary_matrix(g.m, 2);
+            return (g.sub != G1_RX && g.sub != G1_RY) || unit(g.m[0]);
+        case K_U2: return unitary_matrix(g.m, 4);
+        default: return g.kind == K_SWAP;
+    }
+}
+
+int run_gate(qoa_state_t s, const Gate& g) {
+    const GGate k = to_ggate(g);
+    Timer tm(s, gate_bytes(g, s->n) * (s->precision == QOA_PREC_F32 ? 0.5 : 1.0), 1);
+    if (s->precision == QOA_PREC_F32) CK(launch_gate_c64((float2*)s->amps, state_len(s), k, s->stream));
+    else CK(launch_gate(s->amps, state_len(s), k, s->stream));
+    s->launches++;
+    if (s->norm_sure && !unitary_gate(g)) s->norm_sure = false;
+    return QOA_OK;
+}
+
+int do_reset_all(qoa_state_t s);
+
+// How a pass takes its input's squared norm and whether it leaves its own.
+//   in   SCAL_* index: 0 the handle's norm2, SCAL_ONE a normalised input
+//        (the pass before was unitary), SCAL_ZERO |0..0>, which is not read
+//   out  norm partials and their sum into the handle's norm2
+struct PassNorm {
+    int in = 0;
+    bool out = true;
+    bool per_gate = false;  // set where the pass ran as per-gate kernels instead (norm2 is then valid)
+};
+
 // Every gate of the pass is unitary and finite: with the factors of build_pass in P.phase, a normalised input gives
 // a normalised output (to rounding), so its norm need not be measured before
 // the next pass. Measured after the last of such a run, as the scale the run
 // has drifted by (of order 1e-16 a gate) belongs to all amplitudes alike.
 bool unitary_pass(const std::vector<Gate>& G, const Step& st) {
-    auto unit = [](double2 d) { return std::fabs(d.x * d.x + d.y * d.y - 1.0) < 1e-12; };
-    for (int gi : st.gates) {
-        const Gate& g = G[gi];
-        if (g.kind == K_DIAG) {
-            if (!g.neg && !(unit(g.m[0]) && (g.t < 0 || unit(g.m[1])))) return false;
-        } else if (g.kind == K_G1) {
-            if (g.sub == G1_GEN && !unitary_matrix(g.m, 2)) return false;
-            if ((g.sub == G1_RX || g.sub == G1_RY) && !unit(g.m[0])) return false;
-        } else if (g.kind == K_U2) {
-            if (!unitary_matrix(g.m, 4)) return false;
-        } else if (g.kind != K_SWAP) {
-            return false;
-        }
-    }
+    for (int gi : st.gates)
+        if (!unitary_gate(G[gi])) return false;
     return true;
 }
 
@@ -2399,6 +2404,7 @@ int do_reset_all(qoa_state_t s) {
         CK(launch_f32_reset((float2*)s->amps, state_len(s), s->stream));
         CK(launch_set_scalar(s->scal, 1.0, s->stream));
         s->launches += 2;
+        s->norm_sure = true;
         return QOA_OK;
     }
     GGate k;
@@ -2407,6 +2413,7 @@ int do_reset_all(qoa_state_t s) {
     CK(launch_gate(s->amps, state_len(s), k, s->stream));
     CK(launch_set_scalar(s->scal, 1.0, s->stream));
     s->launches += 2;
+    s->norm_sure = true;
     return QOA_OK;
 }
 
@@ -2433,6 +2440,7 @@ int do_measure(qoa_state_t s, uint32_t q, double u, uint32_t* outcome) {
     CK(launch_collapse(s->amps, state_len(s), q, res, f / std::sqrt(norm2), s->partials, ticket(s), s->scal,
                        s->status, s->stream));
     s->launches++;
+    s->norm_sure = true;
     return QOA_OK;
 }
 
@@ -2446,6 +2454,7 @@ int do_reset_qubit(qoa_state_t s, uint32_t q) {
         CK(launch_collapse(s->amps, state_len(s), q, 0, (1.0 / std::sqrt(p0)) / std::sqrt(norm2), s->partials,
                            ticket(s), s->scal, s->status, s->stream));
         s->launches++;
+        s->norm_sure = true;
         return QOA_OK;
     }
     return do_reset_all(s);
@@ -2678,8 +2687,15 @@ void mark_own_kernels(const std::vector<Gate>& G, std::vector<Step>& steps, uint
     steps.swap(out);
 }
 
-// Runs a step marked so.
+// Runs a step marked so. Its kernels act on the stored amplitudes, which are
+// made the logical state first where that may be |0..0> instead.
 int run_own(qoa_state_t s, const std::vector<Gate>& G, const Step& st) {
+    if (!s->norm_sure) {
+        CK(launch_materialize(s->amps, s->precision == QOA_PREC_F32, state_len(s), s->scal, s->partials, ticket(s),
+                              s->status, nullptr, s->stream));
+        s->launches++;
+        s->norm_sure = true;
+    }
     for (size_t i = 0; i < st.gates.size();) {
         const Gate& g = G[st.gates[i]];
         if (g.kind == K_U2) {
@@ -2792,6 +2808,8 @@ int run_small_list(qoa_state_t s, const std::vector<Gate>& seg, bool& reset_owed
         if (b > a) {
             SmallList list;
             small_program(seg, a, b, s->n, list);
+            if (reset_owed) s->norm_sure = true;
+            for (size_t i = a; s->norm_sure && i < b; ++i) s->norm_sure = unitary_gate(seg[i]);
             rc = run_small(s, list, reset_owed ? SCAL_ZERO : 0);
             reset_owed = false;
         } else {
@@ -2874,10 +2892,16 @@ int run_planned(qoa_state_t s, std::vector<Gate>& seg, bool& reset_owed) {
         const Step& st = steps[k];
         int rc = QOA_OK;
         if (st.pass) {
-            if (reset_owed) nm.in = SCAL_ZERO;
+            if (reset_owed) {
+                nm.in = SCAL_ZERO;
+                s->norm_sure = true;
+            }
             reset_owed = false;
             // a pass after a unitary pass takes its input as normalised
-            nm.out = !(k + 1 < steps.size() && steps[k + 1].pass && unitary_pass(seg, st));
+            const bool next = k + 1 < steps.size() && steps[k + 1].pass;
+            const bool unitary = (next || s->norm_sure) && unitary_pass(seg, st);
+            s->norm_sure = s->norm_sure && unitary;
+            nm.out = !(next && unitary);
             nm.per_gate = false;
             const int b = built_of[k], body = b >= 0 ? pe->body_of[b] : -1;
             if (b >= 0)
@@ -4100,6 +4124,7 @@ int qoa_set_state(qoa_state_t s, const void* host, size_t bytes) {
         s->host_resets++;
         return do_reset_all(s);
     }
+    s->norm_sure = true;
     return QOA_OK;
 }
 
@@ -4110,6 +4135,7 @@ int qoa_set_random_state(qoa_state_t s, uint64_t seed) {
     CK(launch_random_state(s->amps, f32, state_len(s), seed, s->stream));
     CK(launch_norm(s->amps, f32, state_len(s), s->partials, ticket(s), s->scal, nullptr, s->stream));
     s->launches += 2;
+    s->norm_sure = true;
     CK(cudaStreamSynchronize(s->stream));
     return QOA_OK;
 }
@@ -4695,6 +4721,7 @@ int qoa_state_load(const char* path, uint32_t flags, qoa_state_t* out) {
         return set_err(nullptr, QOA_E_ARG, "%s: truncated or corrupt checkpoint", path);
     }
     s->host_scal[0] = norm2;
+    s->norm_sure = norm2 > 1e-12;
     if (cudaMemcpyAsync(s->scal, s->host_scal, sizeof(double), cudaMemcpyHostToDevice, s->stream) != cudaSuccess ||
         cudaMemcpyAsync(s->status, words, 4 * sizeof(uint32_t), cudaMemcpyHostToDevice, s->stream) != cudaSuccess ||
         cudaStreamSynchronize(s->stream) != cudaSuccess) {

@@ -115,3 +115,22 @@ def test_short_lists_of_every_mix(n, precision):
             ops.insert(len(ops) // 2, C.Op(C.CNOT, [0, n - 1]))
         got, want = state_after(n, precision, [start(n), ops, ops])
         assert rel_l2(got, want) < TOL[precision]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("zero", [np.zeros(4, dtype=complex), np.full(4, np.nan, dtype=complex)])
+def test_after_a_gate_that_leaves_no_state(zero):
+    """A zero or NaN vector is |0..0> to the next gate, whatever kernel runs it."""
+    n = 13
+    op = u2(12, 1, 6)
+    with qb.QuantumState(n) as st, qb.QuantumState(n) as ref:
+        st.execute(start(n))
+        st.execute([C.Op(C.U1, [3], 0.0, zero)])
+        st.execute([op])
+        ref.execute([op])
+        assert np.max(np.abs(st.get_state_vector() - ref.get_state_vector())) < 1e-15
+        st.execute([C.Op(C.U1, [3], 0.0, zero)])
+        st.execute([C.Op(C.CSWAP, [1, 2, 12]), C.Op(C.CSWAP, [4, 2, 11])])
+        assert st.get_probabilities()[0] == 1.0
+        st.execute([op])
+        assert np.max(np.abs(st.get_state_vector() - ref.get_state_vector())) < 1e-15
