@@ -2805,7 +2805,10 @@ int run_small_list(qoa_state_t s, const std::vector<Gate>& seg, bool& reset_owed
         size_t b = a;
         while (b < seg.size() && seg[b].kind <= K_U2) ++b;
         int rc;
-        if (b > a) {
+        if (b - a == 1 && !reset_owed && s->norm_sure && unitary_gate(seg[a])) {
+            // one gate: its own kernel (a call in a row of them 9.3 against 10.4 us)
+            rc = run_gate(s, seg[b - 1]);
+        } else if (b > a) {
             SmallList list;
             small_program(seg, a, b, s->n, list);
             if (reset_owed) s->norm_sure = true;
