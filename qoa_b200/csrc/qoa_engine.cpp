@@ -485,6 +485,9 @@ cudaError_t device_alloc(void** p, size_t bytes) {
     return e;
 }
 
+constexpr uint32_t kMaxQubits = 40;
+
+// On an error the handle has no state (amps or partials null).
 int alloc_state(qoa_state_t s, uint32_t n) {
     if (s->amps) { cudaFree(s->amps); s->amps = nullptr; }
     if (s->partials) { cudaFree(s->partials); s->partials = nullptr; }
@@ -2931,6 +2934,19 @@ int run_planned(qoa_state_t s, std::vector<Gate>& seg, bool& reset_owed) {
     return QOA_OK;
 }
 
+// QINIT to another size. Where the new state cannot be had, the handle is left
+// with |0..0> of its size before (or of one qubit).
+int resize_state(qoa_state_t s, uint32_t n) {
+    if (n > kMaxQubits) return set_err(s, QOA_E_OOM, "n=%u qubits exceeds the engine limit", n);
+    CK(cudaStreamSynchronize(s->stream));
+    const uint32_t before = s->n;
+    const int rc = alloc_state(s, n);
+    if (!rc) return QOA_OK;
+    const std::string why = s->err;
+    if (!alloc_state(s, before) || !alloc_state(s, 1)) do_reset_all(s);
+    return set_err(s, rc, "%s", why.c_str());
+}
+
 int execute(qoa_state_t s, std::vector<Gate>& G) {
     const bool c64 = s->precision == QOA_PREC_F32;
     if (c64 && (s->flags & QOA_FLAG_F32_TENSOR)) return execute_f32(s, G);
@@ -2948,15 +2964,13 @@ int execute(qoa_state_t s, std::vector<Gate>& G) {
         size_t j = i;
         while (j < G.size() && G[j].kind != K_QINIT) ++j;
         std::vector<Gate> seg(G.begin() + i, G.begin() + j);
-        const int src = seg.empty() ? QOA_OK : small_route(s) ? run_small_list(s, seg, reset_owed) : run_planned(s, seg, reset_owed);
-        if (src) return src;
+        int rc = seg.empty() ? QOA_OK : small_route(s) ? run_small_list(s, seg, reset_owed) : run_planned(s, seg, reset_owed);
+        if (!rc && j < G.size() && (uint32_t)G[j].t != s->n) rc = resize_state(s, (uint32_t)G[j].t);
+        if (rc) {
+            if (reset_owed && s->amps) do_reset_all(s);
+            return rc;
+        }
         if (j < G.size()) {  // QINIT
-            const uint32_t nn = (uint32_t)G[j].t;
-            if (nn != s->n) {
-                CK(cudaStreamSynchronize(s->stream));
-                int rc = alloc_state(s, nn);
-                if (rc) return rc;
-            }
             reset_owed = true;
             ++j;
         }
@@ -2968,6 +2982,7 @@ int execute(qoa_state_t s, std::vector<Gate>& G) {
 int check_handle(qoa_state_t s) {
     if (!s) return set_err(nullptr, QOA_E_ARG, "null handle");
     if (cudaSetDevice(s->device) != cudaSuccess) return set_err(s, QOA_E_CUDA, "cudaSetDevice failed");
+    if (!s->amps || !s->partials) return set_err(s, QOA_E_OOM, "the handle has no state: an allocation failed");
     return QOA_OK;
 }
 
@@ -3886,7 +3901,7 @@ int qoa_create(uint32_t n, int precision, uint32_t flags, qoa_state_t* out) {
     if (precision == QOA_PREC_F32 && (flags & QOA_FLAG_F32_TENSOR) && n < (uint32_t)TILE_BITS)
         return set_err(nullptr, QOA_E_ARG, "the tensor-core block form needs n >= %d", TILE_BITS);
     if (n < 1) n = 1;
-    if (n > 40) return set_err(nullptr, QOA_E_ARG, "n=%u qubits exceeds the engine limit", n);
+    if (n > kMaxQubits) return set_err(nullptr, QOA_E_ARG, "n=%u qubits exceeds the engine limit", n);
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return set_err(nullptr, QOA_E_NOGPU, "no CUDA device");
     s = new qoa_state_s();
@@ -4147,7 +4162,7 @@ int qoa_compare(qoa_state_t a, qoa_state_t b, double* rel_l2, double* infidelity
     qoa_state_t s = a;  // error reporting
     int rc = check_handle(a);
     if (rc) return rc;
-    if (!b || a->n != b->n || a->device != b->device) return set_err(a, QOA_E_ARG, "states differ in size or device");
+    if (!b || !b->amps || a->n != b->n || a->device != b->device) return set_err(a, QOA_E_ARG, "states differ in size or device");
     CK(cudaStreamSynchronize(b->stream));
     CK(launch_compare(a->amps, a->precision == QOA_PREC_F32, b->amps, b->precision == QOA_PREC_F32, state_len(a),
                       a->scal, b->scal, a->partials, a->scal + 8, a->stream));
