@@ -9,9 +9,9 @@ namespace qoa {
 // --------------------------------------------------------------------------
 // Shots of sampled batch circuits: one CTA per circuit builds the marginal
 // tree of its final state in global scratch (level k, 1 <= k < n, holds the
-// 2^k sums over qubits k..n-1 at tree + 2^k - 2, as k_tree_leaf / k_tree_up
-// lay it out), then each thread takes shots and walks the tree from qubit 0:
-// the inverse-CDF rule of k_sample mode 1 (bit q = 0 while the remaining mass
+// 2^k sums over qubits k..n-1 at tree + 2^k - 2, each the sum of two values of
+// level k + 1 that differ in their top bit), then each thread takes shots and
+// walks the tree from qubit 0 by inverse CDF (bit q = 0 while the remaining mass
 // is below the marginal of that prefix). The tree is not divided by the norm:
 // the states of a batch are unit vectors up to rounding, and t = u x total
 // scales with it.

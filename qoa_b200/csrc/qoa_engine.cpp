@@ -2049,7 +2049,9 @@ struct SmallList {
 // as chunks. Greedy like the pass scheduler: a gate joins the open sweep when
 // no waiting gate blocks it and its non-diagonal qubits are among the sweep's
 // three, claiming free ones in the order gates ask for them; the scan looks at
-// most kSmallScan gates ahead.
+// most kSmallScan gates ahead. A 2x2 gate with conditions is X or Y, all that
+// the instruction set makes (is_pass_gate): the other forms' records carry no
+// conditions on register qubits.
 constexpr size_t kSmallScan = 96;
 constexpr int kSmallSweepOps = 96, kSmallSweepCoef = 224;  // a sweep takes at most about half a chunk
 

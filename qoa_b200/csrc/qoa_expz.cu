@@ -196,7 +196,8 @@ void arena_partials(const ExpzJob* jobs, uint32_t njobs, uint32_t tiles, uint32_
 
 }  // namespace
 
-// CTAs of the sweep: the tiles, or four resident CTAs on each of 148 SMs.
+// CTAs of the sweep: the tiles, or four for each of 148 SMs: resident at once
+// up to 64 masks, in two waves above (two CTAs an SM, 128 registers).
 uint32_t expz_blocks(uint64_t len) {
     const uint64_t tiles = (len + TILE - 1) / TILE;
     return (uint32_t)(tiles < 148 * 4 ? tiles : 148 * 4);

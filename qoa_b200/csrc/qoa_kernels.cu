@@ -35,8 +35,7 @@ __device__ __forceinline__ uint64_t tstride(const PassParams& P, uint32_t t) {
 // the kernel before has finished) or, where that is null, `nrm` (<= 1e-12: the
 // input is |0..0>, synthesised without reading); `partial_out`, when not
 // null, receives the tile's squared norm after the pass. The pass's
-// coefficients are built in FP64 on the host; a complex64 pass rounds them
-// once when it stages them.
+// coefficients are built in FP64 on the host. (Complex64 passes: qoa_pass32.cu.)
 // U2: whether the op stream may hold 4x4 gates (PassParams::has_u2). They have a
 // kernel of their own because they spill: in the one kernel they cost every
 // pass 13 % (arena rounds of a batch 3350 against 3794 us).
@@ -671,9 +670,9 @@ __global__ void k_p01(const double2* a, uint64_t len, uint32_t q, double* __rest
 }
 
 // Final reduction: out[s] = sum_k partials[s*count + k] in a fixed order (one
-// block per set), then optional scaling by 1/norm2 and status bookkeeping.
+// block per set), with status bookkeeping where it is a norm.
 __global__ void k_reduce(const double* partials, uint32_t count, double* __restrict__ out,
-                         const double* divide_by, uint32_t* __restrict__ status) {
+                         uint32_t* __restrict__ status) {
     grid_go();
     grid_wait();
     __shared__ double sh[32];
@@ -696,10 +695,6 @@ __global__ void k_reduce(const double* partials, uint32_t count, double* __restr
     if (threadIdx.x == 0) {
         double t = 0.0;
         for (int k = 0; k < (int)(blockDim.x >> 5); ++k) t += sh[k];
-        if (divide_by) {
-            const double d = *divide_by;
-            t = (d > 1e-12) ? t / d : 0.0;
-        }
         out[blockIdx.x] = t;
         if (status) {
             if (t != t) atomicOr(&status[0], 1u);
@@ -875,12 +870,12 @@ cudaError_t launch_p01(const double2* a, uint64_t len, uint32_t q, double* parti
 }
 
 cudaError_t launch_reduce_sets(const double* partials, uint32_t count, uint32_t sets, double* out, cudaStream_t st) {
-    return launch_overlapped(k_reduce, sets, 1024, 0, st, partials, count, out, nullptr, nullptr);
+    return launch_overlapped(k_reduce, sets, 1024, 0, st, partials, count, out, nullptr);
 }
 
 cudaError_t launch_reduce_partials(const double* partials, uint32_t count, double* out, uint32_t* status,
                                    cudaStream_t st) {
-    return launch_overlapped(k_reduce, 1, 1024, 0, st, partials, count, out, nullptr, status);
+    return launch_overlapped(k_reduce, 1, 1024, 0, st, partials, count, out, status);
 }
 
 cudaError_t launch_collapse(double2* a, uint64_t len, uint32_t q, uint32_t outcome, double f, double* partials,

@@ -12,12 +12,13 @@
 // thread walks a shot.
 //
 // What bounds it: reading the state once (the fold of the amplitudes), and
-// for small states the launches: 1 + ceil((n - 8) / 6) of them, where a
-// level-by-level tree takes n. The stored levels take 1/64 (complex128) of
-// the state instead of half of it. Measured on B200, a whole circuit with its
-// shots, against level-by-level trees in scratch mapped on each call: 20
-// qubits 3.3 -> 1.5 ms, 27 qubits 39.8 -> 24.1 ms, 29 qubits (complex64 QFT)
-// 78.5 -> 19.9 ms.
+// for small states the launches: up to 22 qubits 1 + ceil((n - 8) / 4) of them
+// (steps of at most 4 bits), above 1 + ceil((n - 8) / 6), where a
+// level-by-level tree takes n. The stored levels take 8 bytes for every 2^step
+// amplitudes and a little more: 1/128 of a complex128 state with steps of 6
+// bits, 1/32 with steps of 4. Measured on B200, a whole circuit with its shots,
+// against level-by-level trees in scratch mapped on each call: 20 qubits 3.3 ->
+// 1.5 ms, 27 qubits 39.8 -> 24.1 ms, 29 qubits (complex64 QFT) 78.5 -> 19.9 ms.
 #include <cuda_runtime.h>
 
 #include <algorithm>
