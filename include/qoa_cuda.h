@@ -432,7 +432,8 @@ int qoa_plan(uint32_t n, uint32_t flags, const qoa_op* ops, size_t nops, size_t 
  *                  their kernel is ready (one-off structures, such as a
  *                  noisy trajectory's Pauli draws, are never compiled)
  *   QOA_JIT_SYNC   compile before the first launch
- * States below min_qubits (default 20) always interpret. At most 8192
+ * States below min_qubits (default 20) always interpret, and so does a list of
+ * up to eight 4x4 gates and controlled SWAPs alone. At most 8192
  * kernels are loaded per process (environment QOA_JIT_MAX_KERNELS); further
  * structures interpret. */
 #define QOA_JIT_OFF   0
