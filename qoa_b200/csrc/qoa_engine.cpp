@@ -327,6 +327,7 @@ struct qoa_state_s {
     // gates may act on the stored amplitudes (otherwise the logical state may
     // be |0..0>). False after anything that is not unitary, until a reset.
     bool norm_sure = false;
+    bool list_plain = false;        // the list being run is unitary as it stands (Expander::plain)
     double* host_scal = nullptr;  // pinned: mirror of scal, then EXPZ_MASKS results (kernels write them there)
     uint64_t seed = 0;
     uint64_t noise_stream = 0;
@@ -624,6 +625,7 @@ struct Expander {
     uint32_t n;
     uint32_t flags;
     qoa_state_t s;                 // for noise draws (may be null in plan mode)
+    bool plain = true;  // no matrices of the caller's, all angles finite: every gate is unitary
     std::vector<Gate> out;
     int first_err = QOA_OK;
     std::string err;
@@ -704,20 +706,24 @@ struct Expander {
     }
     void phase(uint32_t q, double2 f) {
         if (q >= n) return skip(QOA_E_RANGE, "phase qubit out of range");
+        plain &= f.x - f.x == 0.0;
         Gate g; diag_phase(g, 1ull << q, f); push(g, 1ull << q);
     }
     void rx(uint32_t q, double a) {
         if (q >= n) return skip(QOA_E_RANGE, "RX qubit out of range");
+        plain &= a - a == 0.0;
         const double c = std::cos(a / 2.0), sn = std::sin(a / 2.0);
         Gate g; g1(g, q, G1_RX, d2(c, sn), d2(0, -sn), d2(0, -sn), d2(c, 0), 0); push(g, 1ull << q);
     }
     void ry(uint32_t q, double a) {
         if (q >= n) return skip(QOA_E_RANGE, "RY qubit out of range");
+        plain &= a - a == 0.0;
         const double c = std::cos(a / 2.0), sn = std::sin(a / 2.0);
         Gate g; g1(g, q, G1_RY, d2(c, sn), d2(-sn, 0), d2(sn, 0), d2(c, 0), 0); push(g, 1ull << q);
     }
     void rz(uint32_t q, double a) {
         if (q >= n) return skip(QOA_E_RANGE, "RZ qubit out of range");
+        plain &= a - a == 0.0;
         Gate g;
         g.kind = K_DIAG; g.t = (int)q; g.cmask = 0;
         g.m[0] = from_polar(1.0, -a / 2.0);
@@ -741,6 +747,7 @@ struct Expander {
     void cphase(uint32_t c, uint32_t t, double a) {
         if (c >= n || t >= n) return skip(QOA_E_RANGE, "CPHASE qubit out of range");
         if (c == t) return skip(QOA_E_RANGE, "CPHASE control == target");
+        plain &= a - a == 0.0;
         Gate g; diag_phase(g, cz_mask(c, t), from_polar(1.0, a)); push(g, (1ull << c) | (1ull << t));
     }
     void swap(uint32_t a, uint32_t b, int ctrl) {
@@ -767,6 +774,7 @@ struct Expander {
     void u1(uint32_t q, const double* m) {
         if (q >= n) return skip(QOA_E_RANGE, "U1 qubit out of range");
         if (!m) return skip(QOA_E_ARG, "U1 without matrix");
+        plain = false;
         Gate g; g1(g, q, G1_GEN, d2(m[0], m[1]), d2(m[2], m[3]), d2(m[4], m[5]), d2(m[6], m[7]), 0);
         push(g, 1ull << q);
     }
@@ -774,6 +782,7 @@ struct Expander {
         if (q1 >= n || q2 >= n) return skip(QOA_E_RANGE, "U2 qubit out of range");
         if (q1 == q2) return skip(QOA_E_RANGE, "U2 qubits equal");
         if (!m) return skip(QOA_E_ARG, "U2 without matrix");
+        plain = false;
         Gate g;
         g.kind = K_U2; g.t = (int)std::min(q1, q2); g.t2 = (int)std::max(q1, q2);
         for (int k = 0; k < 16; ++k) g.m[k] = d2(m[2 * k], m[2 * k + 1]);
@@ -2817,7 +2826,8 @@ int run_small_list(qoa_state_t s, const std::vector<Gate>& seg, bool& reset_owed
             SmallList list;
             small_program(seg, a, b, s->n, list);
             if (reset_owed) s->norm_sure = true;
-            for (size_t i = a; s->norm_sure && i < b; ++i) s->norm_sure = unitary_gate(seg[i]);
+            if (!s->list_plain)
+                for (size_t i = a; s->norm_sure && i < b; ++i) s->norm_sure = unitary_gate(seg[i]);
             rc = run_small(s, list, reset_owed ? SCAL_ZERO : 0);
             reset_owed = false;
         } else {
@@ -3987,7 +3997,9 @@ int qoa_apply(qoa_state_t s, const qoa_op* ops, size_t nops) {
         ex.cur = (int)i;
         ex.op(ops[i]);
     }
+    s->list_plain = ex.plain;
     rc = execute(s, ex.out);
+    s->list_plain = false;
     if (rc) return rc;
     if (ex.first_err != QOA_OK) return set_err(s, ex.first_err, "%s", ex.err.c_str());
     return QOA_OK;
